@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 #include <vector>
@@ -457,11 +458,62 @@ extern "C" gd_status gd_complex_free(gd_dcomplex *d) {
 
 extern "C" size_t gd_complex_device_bytes(const gd_dcomplex *d) { return d ? d->bytes : 0; }
 
-// Packs the protein conformations into {x, y, z, ele} and {hpp, meta}.
 // The device order of the points: those whose type forms an H-bond with
-// some ligand type (hdb0 > 0.1) first, each kind in the caller's order.  The
-// energy is a sum over points, so the order changes nothing but the FP32
-// rounding inside a 32-point chunk.
+// some ligand type (hdb0 > 0.1) first, each kind in two zones about the
+// pocket: the points within kNearZone, which a ligand in the pocket is mostly
+// near to (its size plus the distance from which the far form holds, about
+// 16 A), then the others by distance, so that a 32-point chunk's points are
+// mostly all near or all far.  The near zone's points are dealt over its
+// chunks, so that each holds its share of the closest ones, whose close-range
+// terms cost most.  The chunks of both kinds, nearest first, are then dealt
+// over the tiles (and over the chunk positions of a tile), so that every
+// tile, and every tile group's chunks, hold the same mix: a split unit's CTAs
+// and a CTA's tile groups wait for the slowest.  The energy is a sum over
+// points, so the order changes nothing but the FP32 rounding inside a chunk.
+static void order_points(const gd_protein &P, const bool *hb_type, std::vector<int> *out) {
+  const int pnp = P.pnp, chunk = 32, per_tile = TILE_PTS / chunk;
+  const float kNearZone = 24.0f;
+  std::vector<float> key(pnp);  // squared distance from the pocket
+  for (int p = 0; p < pnp; ++p) {
+    const float dx = P.x[p] - P.pocket_center[0], dy = P.y[p] - P.pocket_center[1];
+    const float dz = P.z[p] - P.pocket_center[2];
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    key[p] = d2 < 3.0e38f ? d2 : 3.0e38f;  // also orders NaN
+  }
+  std::vector<int> order, zone;
+  order.reserve(pnp);
+  for (int pass = 0; pass < 2; ++pass) {
+    zone.clear();
+    for (int p = 0; p < pnp; ++p)
+      if (hb_type[P.t[p]] == (pass == 0)) zone.push_back(p);
+    std::stable_sort(zone.begin(), zone.end(), [&](int a, int b) { return key[a] < key[b]; });
+    int near = 0;
+    while (near < (int)zone.size() && key[zone[near]] < kNearZone * kNearZone) ++near;
+    const int nc = (near + chunk - 1) / chunk;
+    for (int c = 0; c < nc; ++c)
+      for (int i = c; i < near; i += nc) order.push_back(zone[i]);
+    order.insert(order.end(), zone.begin() + near, zone.end());
+  }
+  // whole chunks by their middle point; the points past them stay last
+  const int full = pnp / chunk, tiles = (full + per_tile - 1) / per_tile;
+  std::vector<int> rank(full);
+  for (int c = 0; c < full; ++c) rank[c] = c;
+  std::stable_sort(rank.begin(), rank.end(), [&](int a, int b) {
+    return key[order[a * chunk + chunk / 2]] < key[order[b * chunk + chunk / 2]];
+  });
+  out->resize(pnp);
+  int next = 0;
+  for (int q = 0; q < per_tile; ++q)
+    for (int t = 0; t < tiles; ++t) {
+      const int pos = t * per_tile + (q + t) % per_tile;
+      if (pos >= full) continue;
+      std::copy_n(order.begin() + rank[next] * chunk, chunk, out->begin() + pos * chunk);
+      ++next;
+    }
+  std::copy(order.begin() + full * chunk, order.end(), out->begin() + full * chunk);
+}
+
+// Packs the protein conformations into {x, y, z, ele} and {hpp, meta}.
 static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, gd_dcomplex *d) {
   KTables &T = d->T;
   const int pnp = P.pnp;
@@ -472,11 +524,7 @@ static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, gd_dco
     for (int i = 0; i < GD_NLT; ++i) hb_type[j] = hb_type[j] || F.hdb0[i][j] > 0.1f;
   }
   std::vector<int> &order = d->point_order;
-  order.clear();
-  order.reserve(pnp);
-  for (int pass = 0; pass < 2; ++pass)
-    for (int p = 0; p < pnp; ++p)
-      if (hb_type[P.t[p]] == (pass == 0)) order.push_back(p);
+  order_points(P, hb_type, &order);
   std::vector<float4> pa((size_t)P.n_conf * pnp_pad,
                          make_float4(PAD_POINT_COORD, PAD_POINT_COORD, PAD_POINT_COORD, 0.f));
   for (int c = 0; c < P.n_conf; ++c)
@@ -508,6 +556,26 @@ static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, gd_dco
   return GD_OK;
 }
 
+// The distance from which the kernel's far form holds for a ligand type i and
+// a point type j (infinity: never), each bound solved from the term itself:
+// - contact PMF pmf1 / (1 + e), e = exp((6 - d/2)(d - pmf0)): from where
+//   e <= exp(-18) < 2^-25, 1 + e rounds to 1 in FP32 and the term is pmf1;
+// - H-bond hdb1 exp(-h^2/2), h = (d - hdb0) hdb1: below 2^-40 of its peak
+//   from h = 7.46 on (the FP32 sum of the near terms no longer sees it);
+// - near-field electrostatics (el1 d < 1), hydrophobic contact (9 A) and the
+//   contact tests (d <= pmf0) are over.
+static float far_distance(const gd_enepara &F, int i, int j, float max_pmf0) {
+  const double inf = std::numeric_limits<double>::infinity();
+  const double p0 = F.pmf0[i][j];
+  double D = std::max(9.0, (double)max_pmf0);
+  D = std::max(D, F.el1 > 0.f ? 1.0 / (double)F.el1 : inf);
+  D = std::max(D, 0.5 * (12.0 + p0 + std::sqrt((12.0 - p0) * (12.0 - p0) + 144.0)));
+  if (F.hdb0[i][j] > 0.1f)
+    D = std::max(D, F.hdb1[i][j] > 0.f ? (double)F.hdb0[i][j] + 7.46 / (double)F.hdb1[i][j] : inf);
+  D = D * 1.0005 + 0.01;  // rounding of the distances compared with it
+  return std::isfinite(p0) && D < 1e6 ? (float)D : std::numeric_limits<float>::infinity();
+}
+
 // Ligand, pocket template and force-field tables of a complex.
 static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
   const gd_ligand &L = cx->lig;
@@ -525,6 +593,10 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
       tb[i * GD_NPT + j] = make_float2(F.hdb0[i][j], F.hdb1[i][j]);
       max_pmf0 = std::max(max_pmf0, F.pmf0[i][j]);
     }
+  // padding atoms (the last row) bound nothing
+  std::vector<float> tf(TAB_ROWS * GD_NPT, 0.f);
+  for (int i = 0; i < GD_NLT; ++i)
+    for (int j = 0; j < GD_NPT; ++j) tf[i * GD_NPT + j] = far_distance(F, i, j, max_pmf0);
   std::vector<float4> lg((size_t)L.n_conf * lna);
   for (size_t i = 0; i < lg.size(); ++i) lg[i] = make_float4(L.x[i], L.y[i], L.z[i], 0.f);
   std::vector<int> lt(L.t, L.t + lna);
@@ -558,6 +630,7 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
   }
   GD_TRY(upload(d, ta, &T.tab_a));
   GD_TRY(upload(d, tb, &T.tab_b));
+  GD_TRY(upload(d, tf, &T.tab_far));
   GD_TRY(upload(d, lg, &T.lig));
   GD_TRY(upload(d, lt, &T.lig_t));
   GD_TRY(upload(d, lq, &T.lig_q));

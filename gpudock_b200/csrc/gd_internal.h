@@ -48,6 +48,8 @@ struct KTables {
   const float2 *pt_b;   // [pnp_pad] {hpp, meta bits}
   const float4 *tab_a;  // [TAB_ROWS*NPT] {p1a, p2a, pmf0, pmf1}
   const float2 *tab_b;  // [TAB_ROWS*NPT] {hdb0, hdb1}
+  const float *tab_far; // [TAB_ROWS*NPT] distance from which the type pair's
+                        // terms are the far form's (far_distance, gd_api.cu)
   const float4 *lig;    // [n_lig][lna] {x, y, z, 0} relative to the centre
   const int *lig_order; // [lna] atom of each kernel slot: atoms with an H-bond
                         // term first, so they share atom pairs and warps

@@ -41,7 +41,13 @@ namespace gd {
 
 constexpr int STAGE_BYTES = TILE_PTS * (16 + 8);
 constexpr int CHUNK = 32;  // points per FP32 partial before the FP64 flush
-constexpr int kPointUnroll = 2;  // protein points per iteration of the fast path
+// Protein points per iteration of the pair loops: two overlap their chains
+// where a warp holds few atom pairs.  With more, one: a warp alternates
+// between the near and the far loop of every chunk, and bodies of two points
+// no longer fit the instruction caches together (headline interval with NH =
+// 5: 26.2 ms with two points in both loops, 23.4 with one in the far loop,
+// 22.4 with one in both; ncu's no-instruction stall 0.87 / 0.37 / 0.17).
+__host__ __device__ constexpr int point_unroll(int NH) { return NH <= 2 ? 2 : 1; }
 constexpr float LOG2E = 1.4426950408889634f;
 // coordinate of the padding atoms: far from every point, and close enough
 // that d^9 to any point stays finite in FP32
@@ -51,6 +57,9 @@ constexpr float FAR = 1.0e3f;
 // fill a tile past the protein's last point, so they add exactly zero.
 constexpr int PT_ROWS = 32;
 static_assert(PAD_POINT_TYPE >= GD_NPT && PAD_POINT_TYPE < PT_ROWS, "padding type row");
+
+// Points of a chunk plus what the loops read ahead of their last one.
+constexpr int LIST_LEN = CHUNK + 2;
 
 // Per-replica state in shared memory, written by warp 0 only.
 struct LaneState {
@@ -79,9 +88,15 @@ static_assert(sizeof(KItem) % 8 == 0, "KItem must keep the barriers 8-byte align
 //                                               term is defined, else 0)
 // hmask[ag][pt] has bit h set when pair h of group ag has an H-bond term with
 // point type pt.  Slot s = ag + A k holds ligand atom order[s].
+//   far[ag][pt]  = the distance from which every atom of the group takes the
+//                  far form with point type pt
+//   fpmf[ag][pt] = the sum of the group's pmf1 with it (the PMF term there)
+//   list[warp]   = the points of the warp's current chunk, near ones first:
+//                  {byte offset of the point | point type << 16, threshold of
+//                  its close-range vote}
 struct SmemLayout {
-  size_t ptab, htab, hmask, slot_q, slot_t, slot_a, tiles, red, hpc, lane, item, bars, ctl,
-      xch, xch_step, total;
+  size_t ptab, htab, hmask, far, fpmf, list, slot_q, slot_t, slot_a, tiles, red, hpc, lane, item, bars,
+      ctl, xch, xch_step, total;
 };
 
 // Piece bookkeeping of a CTA, in shared memory so that none of it holds a
@@ -119,6 +134,12 @@ __host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, 
   o += (size_t)A * NH * PT_ROWS * 16;
   L.hmask = o;
   o += (size_t)A * PT_ROWS * 4;
+  L.far = o;
+  o += (size_t)A * PT_ROWS * 4;
+  L.fpmf = o;
+  o += (size_t)A * PT_ROWS * 8;
+  L.list = o;
+  o += W * LIST_LEN * sizeof(uint2);
   L.slot_q = o;
   o += MAXA * 4;
   L.slot_t = o;
@@ -477,31 +498,157 @@ __device__ __forceinline__ void pair_block1(const float2 (&nx)[NH], const float2
   }
 }
 
+// The n points of a list (n >= 1); the records are at ta.  Returns the mask of
+// the list positions that some lane has a close-range term with.
 template <int NH, int NHB>
 __device__ __forceinline__ uint32_t chunk_fast(const float2 (&nx)[NH], const float2 (&ny)[NH],
-                                               const float2 (&nz)[NH], const float4 *ta,
-                                               const float2 *tb, int j0, int j1,
-                                               const float4 *my_ptab, const float4 *my_htab,
-                                               const PairConst &K, float thr_l, float2 &fvdw,
-                                               float2 &fpmf, float2 &fhdb, float2 (&fek)[NH]) {
+                                               const float2 (&nz)[NH], const unsigned char *ta,
+                                               const uint2 *list, int n, const float4 *my_ptab,
+                                               const float4 *my_htab, const PairConst &K,
+                                               float2 &fvdw, float2 &fpmf, float2 &fhdb,
+                                               float2 (&fek)[NH]) {
   uint32_t close = 0u;
-  // the next point's record is read one iteration ahead
-  float4 Ap = ta[j0];
-  int pt = (int)(__float_as_uint(tb[j0].y) & META_TYPE_MASK);
-#pragma unroll kPointUnroll
-  for (int j = j0; j < j1; ++j) {
-    const int jn = min(j + 1, j1 - 1);
-    const float4 An = ta[jn];
-    const int ptn = (int)(__float_as_uint(tb[jn].y) & META_TYPE_MASK);
+  // the next point's record is read one iteration ahead, its list entry two
+  uint2 e = list[0], en = list[1];
+  float4 Ap = *reinterpret_cast<const float4 *>(ta + (e.x & 0xffffu));
+#pragma unroll point_unroll(NH)
+  for (int k = 0; k < n; ++k) {
+    const float4 An = *reinterpret_cast<const float4 *>(ta + (en.x & 0xffffu));
+    const uint2 e2 = list[k + 2];
+    const int pt = (int)(e.x >> 16);
     float mn = 3.0e38f;
     pair_block1<NH, NHB>(nx, ny, nz, Ap, my_ptab + pt * 2, my_htab + pt, K, fvdw, fpmf, fhdb,
                          fek, mn);
-    const float thr = __shfl_sync(0xffffffffu, thr_l, j - j0);
-    close |= (__any_sync(0xffffffffu, mn <= thr) ? 1u : 0u) << (j - j0);
+    close |= (__any_sync(0xffffffffu, mn <= __uint_as_float(e.y)) ? 1u : 0u) << k;
     Ap = An;
-    pt = ptn;
+    e = en;
+    en = e2;
   }
   return close;
+}
+
+// The far form: the points of the list (n >= 1) are beyond far[ag][pt] of
+// every atom of the warp in every lane, where the PMF term is pmf1 (added per
+// chunk by the lane that holds the point), the H-bond term and every
+// close-range term are zero, and the soft LJ and the electrostatics are
+// pair_block1's own instructions: 15 packed FMA-pipe and 4 MUFU per atom pair
+// and point against its 22 and 6.
+template <int NH>
+__device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (&ny)[NH],
+                                          const float2 (&nz)[NH], const unsigned char *ta,
+                                          const uint2 *list, int n, const float4 *my_ptab,
+                                          const PairConst &K, float2 &fvdw, float2 (&fek)[NH]) {
+  uint32_t e = list[0].x, en = list[1].x;
+  float4 Ap = *reinterpret_cast<const float4 *>(ta + (e & 0xffffu));
+#pragma unroll point_unroll(NH)
+  for (int k = 0; k < n; ++k) {
+    const float4 An = *reinterpret_cast<const float4 *>(ta + (en & 0xffffu));
+    const uint32_t e2 = list[k + 2].x;
+    const float4 *pp = my_ptab + (e >> 16) * 2;
+    float2 d2[NH], r[NH], den[NH], num[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const float2 dx = add2(dup2(Ap.x), nx[h]);
+      const float2 dy = add2(dup2(Ap.y), ny[h]);
+      const float2 dz = add2(dup2(Ap.z), nz[h]);
+      d2[h] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+      r[h] = make_float2(frsqrt(d2[h].x), frsqrt(d2[h].y));
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const float4 T0 = pp[h * 2 * PT_ROWS];  // p1a, -p2a
+      const float2 d = mul2(d2[h], r[h]);
+      const float2 g = mul2(d2[h], d);
+      const float2 g3 = mul2(mul2(g, g), g);
+      den[h] = fma2(lo2(T0), fma2(K.lj1, d2[h], K.lj0), g3);
+      num[h] = fma2(hi2(T0), g, lo2(T0));
+      fek[h] = fma2(dup2(Ap.w), r[h], fek[h]);
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const float2 inv = make_float2(frcp(den[h].x), frcp(den[h].y));
+      fvdw = fma2(num[h], inv, fvdw);
+    }
+    Ap = An;
+    e = en;
+    en = e2;
+  }
+}
+
+// Where a warp's placed atoms are, over all lanes: the box of their
+// coordinates, its centre, and the largest distance of an atom from that.
+// Atoms without a usable position (not finite, or so far out that d^9
+// overflows) leave an unbounded region, which no point is far from.
+struct Region {
+  float3 lo, hi, mid;
+  float rad;
+};
+template <int NA>
+__device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
+                                              const float2 (&ny)[NA / 2],
+                                              const float2 (&nz)[NA / 2], int n_my) {
+  // n_my: atoms of this lane's replica (0 in a lane without one)
+  const float big = 3.0e38f;
+  float lo[3] = {big, big, big}, hi[3] = {-big, -big, -big};
+  bool usable = true;
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    if (k < n_my) {
+      const float2 ax = nx[k >> 1], ay = ny[k >> 1], az = nz[k >> 1];
+      const float v[3] = {-((k & 1) ? ax.y : ax.x), -((k & 1) ? ay.y : ay.x),
+                          -((k & 1) ? az.y : az.x)};
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        usable = usable && fabsf(v[i]) < 5.0e3f;
+        lo[i] = fminf(lo[i], v[i]);
+        hi[i] = fmaxf(hi[i], v[i]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[i] = fminf(lo[i], __shfl_xor_sync(0xffffffffu, lo[i], o));
+      hi[i] = fmaxf(hi[i], __shfl_xor_sync(0xffffffffu, hi[i], o));
+    }
+  }
+  Region g;
+  g.lo = make_float3(lo[0], lo[1], lo[2]);
+  g.hi = make_float3(hi[0], hi[1], hi[2]);
+  g.mid = make_float3(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]));
+  float r2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    if (k < n_my) {
+      const float2 ax = nx[k >> 1], ay = ny[k >> 1], az = nz[k >> 1];
+      const float dx = g.mid.x + ((k & 1) ? ax.y : ax.x);
+      const float dy = g.mid.y + ((k & 1) ? ay.y : ay.x);
+      const float dz = g.mid.z + ((k & 1) ? az.y : az.x);
+      r2 = fmaxf(r2, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+  g.rad = sqrtf(r2);
+  if (!__all_sync(0xffffffffu, usable)) {
+    g.lo = make_float3(-big, -big, -big);
+    g.hi = make_float3(big, big, big);
+    g.rad = big;
+  }
+  return g;
+}
+
+// Whether the point p is at least D away from the region: outside the box
+// grown by D, or outside the ball grown by D.
+__device__ __forceinline__ bool is_far(const Region &g, const float4 &p, float D) {
+  const float bx = fmaxf(fmaxf(g.lo.x - p.x, p.x - g.hi.x), 0.f);
+  const float by = fmaxf(fmaxf(g.lo.y - p.y, p.y - g.hi.y), 0.f);
+  const float bz = fmaxf(fmaxf(g.lo.z - p.z, p.z - g.hi.z), 0.f);
+  const float cx = g.mid.x - p.x, cy = g.mid.y - p.y, cz = g.mid.z - p.z;
+  const float e = D + g.rad;
+  return fmaf(bz, bz, fmaf(by, by, bx * bx)) > D * D ||
+         fmaf(cz, cz, fmaf(cy, cy, cx * cx)) > e * e;
 }
 
 // Close-range terms of one protein point (calcenergy_d.cu:80-138): the
@@ -611,6 +758,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   float4 *s_ptab = reinterpret_cast<float4 *>(smem + SL.ptab);
   float4 *s_htab = reinterpret_cast<float4 *>(smem + SL.htab);
   uint32_t *s_hmask = reinterpret_cast<uint32_t *>(smem + SL.hmask);
+  float *s_far = reinterpret_cast<float *>(smem + SL.far);
+  double *s_fpmf = reinterpret_cast<double *>(smem + SL.fpmf);
   float *s_q = reinterpret_cast<float *>(smem + SL.slot_q);
   int *s_lt = reinterpret_cast<int *>(smem + SL.slot_t);
   int *s_atom = reinterpret_cast<int *>(smem + SL.slot_a);
@@ -738,6 +887,18 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         if (TG.tab_b[r0].x > 0.1f || TG.tab_b[r1].x > 0.1f) m |= 1u << h;
       }
       s_hmask[i] = m;
+      // far form: the group's largest distance and its PMF sum
+      float fd = 0.f;
+      double fp = 0.0;
+      for (int k = 0; k < NA && pt < GD_NPT; ++k) {
+        const int s = ag + A * k;
+        if (s >= lna) break;
+        const int r = TG.lig_t[TG.lig_order[s]] * GD_NPT + pt;
+        fd = fmaxf(fd, TG.tab_far[r]);
+        fp += (double)TG.tab_a[r].w;
+      }
+      s_far[i] = fd;
+      s_fpmf[i] = fp;
     }
     __syncthreads();  // every thread has read s_ctl->item
     if (threadIdx.x == 0) s_ctl->item = item;
@@ -875,6 +1036,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const float4 *my_ptab = s_ptab + (size_t)ag * NH * PT_ROWS * 2;
   const float4 *my_htab = s_htab + (size_t)ag * NH * PT_ROWS;
   const uint32_t *my_hmask = s_hmask + (size_t)ag * PT_ROWS;
+  const float *my_far = s_far + (size_t)ag * PT_ROWS;
+  const double *my_fpmf = s_fpmf + (size_t)ag * PT_ROWS;
+  uint2 *my_list = reinterpret_cast<uint2 *>(smem + SL.list) + (size_t)warp * LIST_LEN;
+  // entries past a chunk's points are read ahead: point 0 of the tile
+  if (lane < LIST_LEN - CHUNK) my_list[CHUNK + lane] = make_uint2(0u, 0u);
+  my_list[lane] = make_uint2(0u, 0u);
   const bool mcc_on = MODE != KMODE_POSES && (I.flags & GD_MC_MCC) != 0u;
   // atom pairs of this warp with an H-bond term for some point type: the
   // first my_nhb pairs (capable atoms come first in the slot order)
@@ -952,6 +1119,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     }
 #pragma unroll
     for (int h = 0; h < NH; ++h) my_hpc2[h * 32] = make_float2(0.f, 0.f);
+    const Region G = warp_region<NA>(nx, ny, nz, active ? n_my : 0);
+    double far_pmf = 0.0;  // PMF of this lane's far points (every lane's replica)
 
     // ---- pair terms over the protein tiles -----------------------------------
     // FP64 sums of this lane live in the warp's own reduction slots (read by
@@ -990,40 +1159,65 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         // (points are ordered so that chunks rarely mix the two kinds); the
         // close-range votes are collected in a mask and served after the
         // branch-free pass, so consecutive points' chains overlap
+        // lane j looks at point j: the warp lists the points that are not far
+        // of all its atoms in all lanes, then the far ones (the far form)
         const int jl = j0 + lane;
-        const uint32_t meta_l = jl < j1 ? __float_as_uint(tb[jl].y) : (uint32_t)PAD_POINT_TYPE;
-        const bool chunk_hdb = __any_sync(0xffffffffu, my_hmask[meta_l & META_TYPE_MASK] != 0u);
+        const bool valid = jl < j1;
+        const uint32_t meta_l = valid ? __float_as_uint(tb[jl].y) : (uint32_t)PAD_POINT_TYPE;
+        const int pt_l = (int)(meta_l & META_TYPE_MASK);
+        const bool far_l =
+            MODE != KMODE_POSES && valid && is_far(G, ta[valid ? jl : j0], my_far[pt_l]);
+        const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
+        const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
+        const int n_near = __popc(near_m), n_far = __popc(far_m);
         float thr_l = T.near4[((meta_l & META_HPC_BIT) ? 1 : 0) |
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
         if (mcc_on) thr_l = fmaxf(thr_l, T.near_mcc2);
-        // three variants per kernel: no H-bond term, HB - 1 pairs (warps that
-        // need no more) and HB pairs; each is a long unrolled body, so more
-        // of them would cost more in instruction fetch than they save
-        const uint32_t close =
-            (chunk_hdb && my_nhb > 0)
-                ? (my_nhb <= kHB1
-                       ? chunk_fast<NH, kHB1>(nx, ny, nz, ta, tb, j0, j1, my_ptab, my_htab, K,
-                                              thr_l, fvdw, fpmf, fhdb, fek)
-                       : chunk_fast<NH, HB>(nx, ny, nz, ta, tb, j0, j1, my_ptab, my_htab, K,
-                                            thr_l, fvdw, fpmf, fhdb, fek))
-                : chunk_fast<NH, 0>(nx, ny, nz, ta, tb, j0, j1, my_ptab, my_htab, K, thr_l,
-                                    fvdw, fpmf, fhdb, fek);
-        if (close) {
-          // the chunk's hydrophobic sums in registers, added to the per-atom
-          // sums once per chunk
-          float2 hacc[NH];
+        const uint32_t below = (1u << lane) - 1u;
+        __syncwarp();  // the previous chunk's list has been read
+        if (valid)
+          my_list[far_l ? n_near + __popc(far_m & below) : __popc(near_m & below)] =
+              make_uint2((uint32_t)(jl * 16) | ((uint32_t)pt_l << 16), __float_as_uint(thr_l));
+        __syncwarp();
+        const unsigned char *tab = reinterpret_cast<const unsigned char *>(ta);
+        if (n_far) {
+          if (far_l) far_pmf += my_fpmf[pt_l];
+          chunk_far<NH>(nx, ny, nz, tab, my_list + n_near, n_far, my_ptab, K, fvdw, fek);
+        }
+        if (n_near) {
+          const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && my_hmask[pt_l] != 0u);
+          // three variants per kernel: no H-bond term, HB - 1 pairs (warps that
+          // need no more) and HB pairs; each is a long unrolled body, so more
+          // of them would cost more in instruction fetch than they save
+          const uint32_t close =
+              (chunk_hdb && my_nhb > 0)
+                  ? (my_nhb <= kHB1
+                         ? chunk_fast<NH, kHB1>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab,
+                                                K, fvdw, fpmf, fhdb, fek)
+                         : chunk_fast<NH, HB>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab,
+                                              K, fvdw, fpmf, fhdb, fek))
+                  : chunk_fast<NH, 0>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab, K,
+                                      fvdw, fpmf, fhdb, fek);
+          if (close) {
+            // the chunk's hydrophobic sums in registers, added to the per-atom
+            // sums once per chunk
+            float2 hacc[NH];
 #pragma unroll
-          for (int h = 0; h < NH; ++h) hacc[h] = make_float2(0.f, 0.f);
-          for (uint32_t m = close; m != 0u; m &= m - 1u) {
-            const int j = j0 + __ffs(m) - 1;
-            const uint32_t meta = __float_as_uint(tb[j].y);
-            close_range<NA>(nx, ny, nz, ta[j], tb[j].x, meta,
-                            my_ptab + (int)(meta & META_TYPE_MASK) * 2, T, s_q, s_lt, s_atom,
-                            hacc, A, ag, n_my, inv_el1, fnear, fpsp, mcc_on, t * TILE_PTS + j,
-                            my_red);
+            for (int h = 0; h < NH; ++h) hacc[h] = make_float2(0.f, 0.f);
+            for (uint32_t m = close; m != 0u; m &= m - 1u) {
+              const int j = (int)(my_list[__ffs(m) - 1].x & 0xffffu) >> 4;
+              const uint32_t meta = __float_as_uint(tb[j].y);
+              close_range<NA>(nx, ny, nz, ta[j], tb[j].x, meta,
+                              my_ptab + (int)(meta & META_TYPE_MASK) * 2, T, s_q, s_lt, s_atom,
+                              hacc, A, ag, n_my, inv_el1, fnear, fpsp, mcc_on, t * TILE_PTS + j,
+                              my_red);
+            }
+#pragma unroll
+            for (int h = 0; h < NH; ++h) my_hpc2[h * 32] = add2(my_hpc2[h * 32], hacc[h]);
           }
-#pragma unroll
-          for (int h = 0; h < NH; ++h) my_hpc2[h * 32] = add2(my_hpc2[h * 32], hacc[h]);
+          my_red[2 * 32] += (double)fpmf.x + (double)fpmf.y;
+          my_red[3 * 32] += (double)fpsp;
+          my_red[4 * 32] += (double)fhdb.x + (double)fhdb.y;
         }
         float fele = 0.f;
 #pragma unroll
@@ -1033,9 +1227,6 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         }
         my_red[0 * 32] += (double)fvdw.x + (double)fvdw.y;
         my_red[1 * 32] += (double)fele * (double)inv_el1 + (double)fnear;
-        my_red[2 * 32] += (double)fpmf.x + (double)fpmf.y;
-        my_red[3 * 32] += (double)fpsp;
-        my_red[4 * 32] += (double)fhdb.x + (double)fhdb.y;
       }
       if (!resident) {
         // the last of the W warps to finish this stage refills it with the
@@ -1055,6 +1246,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         }
       }
     }
+
+    // the far points' PMF, summed over the lanes that hold them
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) far_pmf += __shfl_xor_sync(0xffffffffu, far_pmf, o);
+    my_red[2 * 32] += far_pmf;
 
     // ---- KDE ------------------------------------------------------------------
     double dkde = 0.0, dlhm = 0.0;
