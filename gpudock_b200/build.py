@@ -23,6 +23,8 @@ OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libgpudock.so")
 SOURCES = ["gd_kernels.cu", "gd_api.cu", "gd_ensemble.cu", "gd_server.cu", "gd_noalloc.cu",
            "gd_similarity.cu", "gd_load.cpp"]
+# the kernel variants of gd_kernels.cu are compiled in parts, in parallel
+PARTS = {"gd_kernels.cu": [f"-DGD_DOCK_PART={k}" for k in range(6)]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -38,8 +40,8 @@ def _flags():
             "-ccbin", shutil.which("g++") or "g++", "-I" + os.path.join(ROOT, "include")]
 
 
-def _compile(src: str, obj: str, verbose: bool):
-    cmd = [nvcc(), *_flags(), "-c", "-o", obj + ".tmp", src]
+def _compile(src: str, obj: str, define: str, verbose: bool):
+    cmd = [nvcc(), *_flags(), *([define] if define else []), "-c", "-o", obj + ".tmp", src]
     if verbose:
         cmd[1:1] = ["-Xptxas", "-v"]
     res = subprocess.run(cmd, capture_output=True, text=True)
@@ -58,16 +60,18 @@ def build(verbose: bool = False, force: bool = False) -> str:
     t_hdr = max(os.path.getmtime(h) for h in headers)
     objs, todo = [], []
     for s in srcs:
-        o = os.path.join(OBJDIR, os.path.basename(s) + ".o")
-        objs.append(o)
-        if force or not os.path.exists(o) or os.path.getmtime(o) < max(t_hdr,
-                                                                        os.path.getmtime(s)):
-            todo.append((s, o))
+        name = os.path.basename(s)
+        for k, define in enumerate(PARTS.get(name, [""])):
+            o = os.path.join(OBJDIR, name + (f".{k}" if define else "") + ".o")
+            objs.append(o)
+            if force or not os.path.exists(o) or os.path.getmtime(o) < max(t_hdr,
+                                                                            os.path.getmtime(s)):
+                todo.append((s, o, define))
     if not todo and os.path.exists(LIB) and all(
             os.path.getmtime(o) <= os.path.getmtime(LIB) for o in objs):
         return LIB
     with ThreadPoolExecutor(max_workers=max(1, min(len(todo), os.cpu_count() or 1))) as ex:
-        for f in [ex.submit(_compile, s, o, verbose) for s, o in todo]:
+        for f in [ex.submit(_compile, s, o, d, verbose) for s, o, d in todo]:
             f.result()
     cmd = [nvcc(), *ARCH, "-shared", "-cudart", "static", "-ccbin",
            shutil.which("g++") or "g++", "-o", LIB + ".tmp", *objs]

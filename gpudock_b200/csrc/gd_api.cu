@@ -103,6 +103,14 @@ int units_of(int n_prt, int n_lig, int n_tmp) {
   return n_prt * ((n_lig * n_tmp + 31) / 32);
 }
 
+bool has_packed_units(int n_prt, int n_lig, int n_tmp) {
+  // every unit but the last of a protein conformation is full
+  const int G = 32 % n_tmp == 0 ? 32 / n_tmp : 0;
+  const int full = G ? G * n_tmp : 32, all = n_lig * n_tmp;
+  const int last = all % full ? all % full : full;
+  return packed_reps(last) < 32 || (all >= full && packed_reps(full) < 32);
+}
+
 Tile tile_for(gd_ctx *ctx, const KTables &T) {
   const int n_tiles = (T.pnp + TILE_PTS - 1) / TILE_PTS;
   const int hi = lna_bucket(T.lna);
@@ -464,8 +472,8 @@ extern "C" size_t gd_complex_device_bytes(const gd_dcomplex *d) { return d ? d->
 // near to (its size plus the distance from which the far form holds, about
 // 16 A), then the others by distance, so that a 32-point chunk's points are
 // mostly all near or all far.  The near zone's points are dealt over its
-// chunks, so that each holds its share of the closest ones, whose close-range
-// terms cost most.  The chunks of both kinds, nearest first, are then dealt
+// half chunks, so that each holds its share of the closest ones, whose
+// close-range terms cost most.  The chunks of both kinds, nearest first, are then dealt
 // over the tiles (and over the chunk positions of a tile), so that every
 // tile, and every tile group's chunks, hold the same mix: a split unit's CTAs
 // and a CTA's tile groups wait for the slowest.  The energy is a sum over
@@ -489,9 +497,13 @@ static void order_points(const gd_protein &P, const bool *hb_type, std::vector<i
     std::stable_sort(zone.begin(), zone.end(), [&](int a, int b) { return key[a] < key[b]; });
     int near = 0;
     while (near < (int)zone.size() && key[zone[near]] < kNearZone * kNearZone) ++near;
-    const int nc = (near + chunk - 1) / chunk;
+    // in runs of two: packed lanes take several points at a time
+    const int half = chunk / 2, run = 2, nr = near / run;
+    const int nc = std::max(1, near / half);
     for (int c = 0; c < nc; ++c)
-      for (int i = c; i < near; i += nc) order.push_back(zone[i]);
+      for (int r = c; r < nr; r += nc)
+        order.insert(order.end(), zone.begin() + r * run, zone.begin() + (r + 1) * run);
+    order.insert(order.end(), zone.begin() + nr * run, zone.begin() + near);
     order.insert(order.end(), zone.begin() + near, zone.end());
   }
   // whole chunks by their middle point; the points past them stay last
@@ -615,7 +627,7 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
   // MCS gathered per ligand atom: field n + 1 (calcenergy_d.cu:240-241)
   const int pos = cx->mcs.pos;
   std::vector<float4> mc((size_t)pos * lna);
-  std::vector<float> tcc(pos), cnt(pos);
+  std::vector<double2> mw(pos);
   for (int m = 0; m < pos; ++m) {
     int c = 0;
     for (int a = 0; a < lna; ++a) {
@@ -625,8 +637,8 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
           make_float4(cx->mcs.x[f], cx->mcs.y[f], cx->mcs.z[f], valid ? 1.f : 0.f);
       c += valid;
     }
-    tcc[m] = cx->mcs.tcc[m];
-    cnt[m] = (float)c;
+    // no valid atom: 0 x inf = NaN, as the reference's 0 / 0
+    mw[m] = make_double2((double)cx->mcs.tcc[m], 1.0 / (double)c);
   }
   GD_TRY(upload(d, ta, &T.tab_a));
   GD_TRY(upload(d, tb, &T.tab_b));
@@ -651,8 +663,7 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
   GD_TRY(upload(d, kd, &T.kde));
   GD_TRY(upload(d, koff, &T.kde_off));
   GD_TRY(upload(d, mc, &T.mcs));
-  GD_TRY(upload(d, tcc, &T.mcs_tcc));
-  GD_TRY(upload(d, cnt, &T.mcs_cnt));
+  GD_TRY(upload(d, mw, &T.mcs_w));
 
   T.lna = lna;
   T.n_lig = L.n_conf;
@@ -667,7 +678,10 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
   T.b1 = F.b1;
   T.kde2 = F.kde2;
   T.kde3 = F.kde3;
-  T.s2pi = sqrtf(2.0f * kPI);
+  T.inv_lna = 1.0 / (double)lna;
+  T.inv_pos = 1.0 / (double)pos;  // no records: 0 x inf = NaN, as 0 / 0
+  T.inv_kde3 = 1.0 / (double)F.kde3;
+  T.inv_s2pi = 1.0 / (double)sqrtf(2.0f * kPI);
   // the close-range terms fire inside these distances: near-field
   // electrostatics el1 d < 1 (every point), hydrophobic d <= 9 (points with
   // the hpc flag), psp d <= pmf0 (class-2 points); thresholds by point kind

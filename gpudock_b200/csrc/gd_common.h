@@ -145,6 +145,8 @@ int split_for(gd_ctx *ctx, const KTables &T, int run_units, double min_cost);
 // 32-replica units of a complex's replicas (n_prt x n_lig x n_tmp): whole
 // exchange groups per unit when n_tmp divides 32.
 int units_of(int n_prt, int n_lig, int n_tmp);
+// Whether some of those units has at most 16 replicas (KRun.packed).
+bool has_packed_units(int n_prt, int n_lig, int n_tmp);
 
 // Launches of different shapes (one per launch plan) are independent; each
 // kernel holds one CTA per SM, so a plan with fewer CTAs than SMs leaves the

@@ -42,6 +42,7 @@ struct Plan {
   int n_stages = 0, resident = 0, group_major = 0, fused = 0, grid = 0;
   int hb_pairs = 0;  // largest hb_pairs_of over its items
   int split = 1;     // CTAs (a cluster) per unit (split_for)
+  int packed = 0;    // some unit has at most 16 replicas (KRun.packed)
   int *d_cta_item = nullptr, *d_cta_rep0 = nullptr, *d_cta_nrep = nullptr;
   // persistent schedules (KRun.pieces) of this plan's units, by launch length
   std::vector<double> unit_cost;  // [grid] cost of one MC step of each unit
@@ -258,7 +259,7 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
   GD_TRY(dcopy(E, &E.d_items, E.items));
 
   // launch plans: one per (shape, staging, layout); CTAs in decreasing cost
-  using Key = std::tuple<int, int, int, int, int, int, int>;
+  using Key = std::tuple<int, int, int, int, int, int, int, int>;
   std::map<Key, std::vector<std::tuple<double, int, int, int>>> ctas;  // cost, item, rep0, n
   std::map<Key, Plan> plans;
   std::vector<KGroup> groups;
@@ -273,10 +274,12 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
     const int nt = I.n_tmp, nl = I.n_lig_conf;
     const bool gm = (32 % nt) == 0;
     const bool exch = (I.flags & GD_MC_EXCHANGE) != 0;
-    const Key key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, split};
+    const int packed = has_packed_units(I.n_prt, nl, nt) ? 1 : 0;
+    const Key key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, split, packed};
     Plan &pl = plans[key];
     pl.tile = t;
     pl.split = split;
+    pl.packed = packed;
     pl.n_stages = ns;
     pl.resident = res;
     pl.group_major = gm ? 1 : 0;
@@ -358,6 +361,7 @@ KRun run_desc(const Ens &E, const Plan &pl, int mode) {
   R.wait_bias = E.ctx->wait_bias;
   R.hb_pairs = pl.hb_pairs;
   R.split = pl.split;
+  R.packed = pl.packed;
   return R;
 }
 

@@ -21,6 +21,7 @@ constexpr int MAX_RESIDENT_TILES = 56; // 7168 points kept in smem for a launch
 constexpr int MAX_WARPS = GD_MAX_WARPS; // warps per CTA (all compute)
 constexpr int MAX_NA = 10;             // ligand atoms per warp (template bound)
 constexpr int MAX_LNA = 128;           // ligand atoms per complex
+constexpr int MAX_SPLIT = 16;          // CTAs that can share a unit (a cluster)
 constexpr int NRED = 10;               // partial sums per replica per warp
 constexpr int MAX_TMP = 64;            // temperatures per exchange group
 constexpr int TAB_ROWS = GD_NLT + 1;   // + one all-zero row for padding atoms
@@ -39,6 +40,15 @@ constexpr int MAX_SEQ3R = (1 << 20) - 1;
 // them and add exactly zero.
 constexpr int PAD_POINT_TYPE = 31;
 constexpr float PAD_POINT_COORD = -3.0e3f;
+
+// Lane packing: a unit of n replicas takes packed_reps(n) lanes of each warp,
+// and 32 / packed_reps groups of lanes (at most MAX_SUBS) share the points.
+constexpr int MAX_SUBS = 8;
+__host__ __device__ inline int packed_reps(int n) {
+  int reps = 32;
+  while (reps > 32 / MAX_SUBS && n <= reps / 2) reps /= 2;
+  return reps;
+}
 
 enum KMode : int { KMODE_POSES = 0, KMODE_REMC = 1, KMODE_INIT = 2 };
 
@@ -61,8 +71,7 @@ struct KTables {
   const float4 *kde;    // [pnk] sorted by type {x, y, z, 0}
   const int *kde_off;   // [NLT + 1]
   const float4 *mcs;    // [pos][lna] {x, y, z, valid}
-  const float *mcs_tcc; // [pos]
-  const float *mcs_cnt; // [pos] number of valid atoms (float)
+  const double2 *mcs_w; // [pos] {tcc, 1 / number of valid atoms}
   const uint32_t *mcc_ref;  // [lna][mcc_words] reference contact map (bits)
   int lna, n_lig, pnp, pnp_pad, n_prt, pos, psp_ncol, mcc_words;
   int n_hb;             // atoms with an H-bond term (the first n_hb slots)
@@ -73,7 +82,8 @@ struct KTables {
   float near_ele2;      // squared distance of the near-field electrostatics
                         // switch (1/el1)^2, with margin
   float lj0, lj0lj1, el0, el1, inv_el1, a1, b1, kde2, kde3;
-  float s2pi;           // sqrtf(2 * 3.1415926535f), the reference's float
+  double inv_lna, inv_pos, inv_kde3;  // reciprocals of the finish
+  double inv_s2pi;      // of sqrtf(2 * 3.1415926535f), the reference's float
   float near4[4];       // squared distance below which a close-range term can
                         // fire, by point kind (hpc flag | class 2 << 1)
   float hpl0[GD_NLT], hpl1[GD_NLT], hpl2[GD_NLT];
@@ -139,6 +149,9 @@ struct KRun {
                          // CTAs (<= 8) share each unit, CTA rank r taking the
                          // protein tiles r, r + split, ... (grid = units x split);
                          // 0 or 1: one CTA per unit
+  int packed;            // REMC / INIT: nonzero when some unit of the launch has at
+                         // most 16 replicas (packed_reps < 32); POSES: poses
+                         // per unit (8 or 16), or 0 for 32
   int hb_pairs;          // most atom pairs with an H-bond term in any warp of
                          // any item (hb_pairs_of); selects the kernel variant
   // Persistent schedule (REMC; nullptr: CTA b runs every step of unit b,

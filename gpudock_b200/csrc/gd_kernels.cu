@@ -58,8 +58,9 @@ constexpr float FAR = 1.0e3f;
 constexpr int PT_ROWS = 32;
 static_assert(PAD_POINT_TYPE >= GD_NPT && PAD_POINT_TYPE < PT_ROWS, "padding type row");
 
-// Points of a chunk plus what the loops read ahead of their last one.
-constexpr int LIST_LEN = CHUNK + 2;
+// A chunk's list: its points, both parts filled up to a multiple of the
+// subsets, and what the loops read ahead of their last entry.
+constexpr int LIST_LEN = CHUNK + 4 * MAX_SUBS;
 
 // Per-replica state in shared memory, written by warp 0 only.
 struct LaneState {
@@ -78,6 +79,12 @@ struct LaneState {
 static_assert(sizeof(LaneState) == 152, "LaneState layout");
 static_assert(sizeof(KItem) % 8 == 0, "KItem must keep the barriers 8-byte aligned");
 
+// KDE points of a slot's ligand type: first, end and 1 / their number.
+struct SlotKde {
+  int begin, end;
+  double inv_n;
+};
+
 // Shared-memory carve-up of one CTA.  The pair tables hold, for every
 // (atom group, atom pair h, point type), the parameters of the warp's two
 // atoms of pair h side by side, so one 16-byte load yields the operand pairs
@@ -92,10 +99,11 @@ static_assert(sizeof(KItem) % 8 == 0, "KItem must keep the barriers 8-byte align
 //                  far form with point type pt
 //   fpmf[ag][pt] = the sum of the group's pmf1 with it (the PMF term there)
 //   list[warp]   = the points of the warp's current chunk, near ones first:
-//                  {byte offset of the point | point type << 16, threshold of
-//                  its close-range vote}
+//                  {offset of its record in shared memory | point type << 23
+//                  (list_entry), threshold of its close-range vote}
+//   pad          = the record of a padding point (fills up the lists)
 struct SmemLayout {
-  size_t ptab, htab, hmask, far, fpmf, list, slot_q, slot_t, slot_a, tiles, red, hpc, lane, item, bars,
+  size_t ptab, htab, hmask, far, fpmf, list, pad, slot_q, slot_t, slot_a, slot_k, tiles, red, hpc, lane, item, bars,
       ctl, xch, xch_step, total;
 };
 
@@ -140,12 +148,18 @@ __host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, 
   o += (size_t)A * PT_ROWS * 8;
   L.list = o;
   o += W * LIST_LEN * sizeof(uint2);
+  o = (o + 15) & ~size_t(15);
+  L.pad = o;
+  o += 16;
   L.slot_q = o;
   o += MAXA * 4;
   L.slot_t = o;
   o += MAXA * 4;
   L.slot_a = o;
   o += MAXA * 4;
+  o = (o + 15) & ~size_t(15);
+  L.slot_k = o;
+  o += MAXA * sizeof(SlotKde);
   o = (o + 127) & ~size_t(127);
   L.tiles = o;
   o += (size_t)NS * STAGE_BYTES;
@@ -169,9 +183,11 @@ __host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, 
   return L;
 }
 
+#if GD_DOCK_PART == 0
 size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split) {
   return smem_layout(A, P, NA, n_stages, split).total;
 }
+#endif
 
 // Hardware approximations (PTX rsqrt / rcp / ex2, flush-to-zero).
 __device__ __forceinline__ float frsqrt(float x) {
@@ -215,6 +231,18 @@ __device__ __forceinline__ void make_rot(float a3, float a4, float a5, float *R)
   R[8] = c2 * c3;
 }
 
+// Lane packing.  A unit with few replicas would leave most lanes idle: its
+// replicas take the first `reps` lanes (packed_reps) of a warp, and the
+// 32 / reps groups of lanes hold the same replicas and share a chunk's points
+// (lane group g takes the list entries g, g + subs, ...).  Their partial sums
+// are added across the groups with the cross-warp sums.
+// Sum over the lanes that hold the same replica (every one gets it).
+template <typename T>
+__device__ __forceinline__ T sum_subs(T v, int reps) {
+  for (int o = reps; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Per-atom hydrophobic sums in shared memory: for tile group g, the float2
 // of atom pair h (slots ag + 2hA, ag + (2h+1)A) of atom group ag and lane
 // `lane` sits at float2 index ((g A + ag) NH + h) 32 + lane (a warp reads
@@ -243,62 +271,58 @@ __device__ __forceinline__ float2 hpc_transform(const KTables &T, const int *s_l
 }
 __device__ __forceinline__ float2 hpc_restraint(const KTables &T, const float2 *s_hpc2,
                                                 const int *s_lt, int P, int A, int NH, int ag,
-                                                int hp, int lane) {
+                                                int hp, int lane, int reps) {
   float2 v = make_float2(0.f, 0.f);
   for (int g = 0; g < P; ++g) {
     const float2 x = s_hpc2[hpc_pair_at(g, ag, hp, lane, A, NH)];
     v.x += x.x;
     v.y += x.y;
   }
+  v = make_float2(sum_subs(v.x, reps), sum_subs(v.y, reps));
   return hpc_transform(T, s_lt, A, ag, hp, v);
 }
 
-// Warp 0 after the step's partial sums: cross-warp reduction in a fixed
-// order, hydrophobic restraint per atom (hpc_done: already transformed by the
-// warps into tile group 0's slots), normalisation and total in the
-// reference's order, then the pose output, or the Metropolis decision (with
-// the trajectory record) and, at the end of an interval, the in-CTA
-// temperature exchange.  Kept out of line so its registers do not burden the
-// pair loop.
+// Warp 0 after the step's sums (slot 0 of s_red, and the hydrophobic
+// restraints in tile group 0's slots, both from all warps): normalisation and
+// total in the reference's order, then the pose output, or the Metropolis
+// decision (with the trajectory record) and, at the end of an interval, the
+// in-CTA temperature exchange.  Every lane of a replica computes the same;
+// the first lane group writes.  Kept out of line so its registers do not
+// burden the pair loop.
 template <int MODE>
 __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneState &me,
-                                         double *s_red, const float *s_hpc, const int *s_lt,
-                                         int W, int P, int A, int NH, int lane, int rep,
-                                         bool active, int prt_conf, int lig_conf, int step,
-                                         bool primary, bool hpc_done) {
+                                         double *s_red, const float *s_hpc, int A, int NH,
+                                         int lane, int reps, int rep, bool active, int prt_conf,
+                                         int lig_conf, int step, bool primary) {
   const KTables &T = I.T;
   const int lna = T.lna;
   const float lcx = T.lig_center[0], lcy = T.lig_center[1], lcz = T.lig_center[2];
+    const int rl = lane & (reps - 1);
     double S[NRED];
 #pragma unroll
-    for (int i = 0; i < NRED; ++i) S[i] = 0.0;
-    for (int w = 0; w < W; ++w) {
-      const double *red = s_red + (size_t)w * NRED * 32;
-#pragma unroll
-      for (int i = 0; i < NRED; ++i) S[i] += red[i * 32 + lane];
-    }
+    for (int i = 0; i < NRED; ++i) S[i] = s_red[i * 32 + rl];
     // hydrophobic restraint per ligand atom, by slot (slot a = ag + A k holds
-    // one atom, s_lt its type), an atom pair's two slots at a time, in slot
-    // order
+    // one atom), an atom pair's two slots at a time, in slot order
     const float2 *s_hpc2 = reinterpret_cast<const float2 *>(s_hpc);
     for (int ag = 0; ag < A; ++ag)
       for (int hp = 0; hp < NH; ++hp) {
         if (ag + 2 * hp * A >= lna) break;
-        const float2 r = hpc_done ? s_hpc2[hpc_pair_at(0, ag, hp, lane, A, NH)]
-                                  : hpc_restraint(T, s_hpc2, s_lt, P, A, NH, ag, hp, lane);
+        const float2 r = s_hpc2[hpc_pair_at(0, ag, hp, rl, A, NH)];
         S[5] += (double)r.x;
         if (ag + A * (2 * hp + 1) < lna) S[5] += (double)r.y;
       }
-    const double n = (double)lna;
+    // multiplied by the host's FP64 reciprocals (an FP64 division takes some
+    // 30 dependent instructions, and here every warp waits for this one)
+    const double inv_n = T.inv_lna;
     double raw[GD_NRAW];
-    raw[0] = S[0] / n;
-    raw[1] = S[1] / n;
-    raw[2] = S[2] / n;
-    raw[3] = S[3] / n;
-    raw[4] = -(S[4] / n / (double)T.s2pi);
-    raw[5] = S[5] / n;
-    raw[6] = S[6] / (double)T.kde3 / n;
-    raw[7] = log(S[7] / (double)T.pos);
+    raw[0] = S[0] * inv_n;
+    raw[1] = S[1] * inv_n;
+    raw[2] = S[2] * inv_n;
+    raw[3] = S[3] * inv_n;
+    raw[4] = -(S[4] * inv_n * T.inv_s2pi);
+    raw[5] = S[5] * inv_n;
+    raw[6] = S[6] * T.inv_kde3 * inv_n;
+    raw[7] = log(S[7] * T.inv_pos);
     {
       // distance to the pocket (calcenergy_d.cu:278-283); centre = c + m
       const float cx = __fadd_rn(lcx, me.m_new[0]);
@@ -330,9 +354,11 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
       const float dividend = __fsqrt_rn(
           __fmul_rn(__fmul_rn(__fmul_rn(__fadd_rn(tp, fp), __fadd_rn(tp, fn)), __fadd_rn(tn, fp)),
                     __fadd_rn(tn, fn)));
-      me.cmcc_new = dividend != 0.0f
-                        ? __fdiv_rn(__fsub_rn(__fmul_rn(tp, tn), __fmul_rn(fp, fn)), dividend)
-                        : GD_CMCC_INVALID;
+      const float cmcc =
+          dividend != 0.0f
+              ? __fdiv_rn(__fsub_rn(__fmul_rn(tp, tn), __fmul_rn(fp, fn)), dividend)
+              : GD_CMCC_INVALID;
+      if (lane < reps) me.cmcc_new = cmcc;
     }
 
     if (MODE == KMODE_POSES) {
@@ -367,7 +393,7 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
           rc->accepted = acc;
         }
       }
-      if (acc) {
+      if (acc && lane < reps) {
         me.acs += 1;
 #pragma unroll
         for (int i = 0; i < GD_NTERM; ++i) me.e_old[i] = e[i];
@@ -383,6 +409,7 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
         const int nt = I.n_tmp;
         int *s_tmp = reinterpret_cast<int *>(s_red);          // 32 ints
         float *s_en = reinterpret_cast<float *>(s_red) + 32;  // 32 floats
+        __syncwarp();  // the accepted state is written
         s_tmp[lane] = me.idx_tmp;
         s_en[lane] = me.e_old[GD_E_TOTAL];
         __syncwarp();
@@ -419,8 +446,10 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
           }
         }
         __syncwarp();
-        me.idx_tmp = s_tmp[lane];
-        me.mbeta = I.minus_beta[me.idx_tmp];
+        if (lane < reps) {
+          me.idx_tmp = s_tmp[lane];
+          me.mbeta = I.minus_beta[me.idx_tmp];
+        }
       }
     }
   }
@@ -498,27 +527,53 @@ __device__ __forceinline__ void pair_block1(const float2 (&nx)[NH], const float2
   }
 }
 
-// The n points of a list (n >= 1); the records are at ta.  Returns the mask of
-// the list positions that some lane has a close-range term with.
-template <int NH, int NHB>
+template <int V>
+struct Int {
+  static constexpr int value = V;
+};
+
+// A list entry's first word: the record's byte offset in shared memory (below
+// 2^18) and the point type from bit 23, so that the word >> 18 is the byte
+// offset of the type's 32-byte entry in the pair table.
+__device__ __forceinline__ uint32_t list_entry(uint32_t at, int pt) {
+  return at | ((uint32_t)pt << 23);
+}
+__device__ __forceinline__ uint32_t entry_at(uint32_t e) { return e & 0x3ffffu; }
+__device__ __forceinline__ float4 entry_point(const unsigned char *smem, uint32_t e) {
+  return *reinterpret_cast<const float4 *>(smem + entry_at(e));
+}
+
+// n points of a list (n >= 1) for each of the `subs` point subsets of the
+// lanes (PACKED; else one): list points at this lane's first entry, its next
+// ones follow at distance subs.  Returns the mask of the iterations in which some lane has a
+// close-range term.
+template <int NH, int NHB, bool PACKED>
 __device__ __forceinline__ uint32_t chunk_fast(const float2 (&nx)[NH], const float2 (&ny)[NH],
-                                               const float2 (&nz)[NH], const unsigned char *ta,
-                                               const uint2 *list, int n, const float4 *my_ptab,
+                                               const float2 (&nz)[NH],
+                                               const unsigned char *smem, const uint2 *list, int n,
+                                               int n_subs, const float4 *my_ptab,
                                                const float4 *my_htab, const PairConst &K,
                                                float2 &fvdw, float2 &fpmf, float2 &fhdb,
                                                float2 (&fek)[NH]) {
+  const int subs = PACKED ? n_subs : 1;
   uint32_t close = 0u;
   // the next point's record is read one iteration ahead, its list entry two
-  uint2 e = list[0], en = list[1];
-  float4 Ap = *reinterpret_cast<const float4 *>(ta + (e.x & 0xffffu));
+  uint2 e = list[0], en = list[subs];
+  list += 2 * subs;
+  float4 Ap = entry_point(smem, e.x);
 #pragma unroll point_unroll(NH)
   for (int k = 0; k < n; ++k) {
-    const float4 An = *reinterpret_cast<const float4 *>(ta + (en.x & 0xffffu));
-    const uint2 e2 = list[k + 2];
-    const int pt = (int)(e.x >> 16);
+    const float4 An = entry_point(smem, en.x);
+    const uint2 e2 = *list;
+    list += subs;
+    const uint32_t po = e.x >> 18;
     float mn = 3.0e38f;
-    pair_block1<NH, NHB>(nx, ny, nz, Ap, my_ptab + pt * 2, my_htab + pt, K, fvdw, fpmf, fhdb,
-                         fek, mn);
+    pair_block1<NH, NHB>(
+        nx, ny, nz, Ap,
+        reinterpret_cast<const float4 *>(reinterpret_cast<const unsigned char *>(my_ptab) + po),
+        reinterpret_cast<const float4 *>(reinterpret_cast<const unsigned char *>(my_htab) +
+                                         po / 2),
+        K, fvdw, fpmf, fhdb, fek, mn);
     close |= (__any_sync(0xffffffffu, mn <= __uint_as_float(e.y)) ? 1u : 0u) << k;
     Ap = An;
     e = en;
@@ -533,18 +588,23 @@ __device__ __forceinline__ uint32_t chunk_fast(const float2 (&nx)[NH], const flo
 // close-range term are zero, and the soft LJ and the electrostatics are
 // pair_block1's own instructions: 15 packed FMA-pipe and 4 MUFU per atom pair
 // and point against its 22 and 6.
-template <int NH>
+template <int NH, bool PACKED>
 __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (&ny)[NH],
-                                          const float2 (&nz)[NH], const unsigned char *ta,
-                                          const uint2 *list, int n, const float4 *my_ptab,
-                                          const PairConst &K, float2 &fvdw, float2 (&fek)[NH]) {
-  uint32_t e = list[0].x, en = list[1].x;
-  float4 Ap = *reinterpret_cast<const float4 *>(ta + (e & 0xffffu));
+                                          const float2 (&nz)[NH], const unsigned char *smem,
+                                          const uint2 *list, int n, int n_subs,
+                                          const float4 *my_ptab, const PairConst &K, float2 &fvdw,
+                                          float2 (&fek)[NH]) {
+  const int subs = PACKED ? n_subs : 1;
+  uint32_t e = list[0].x, en = list[subs].x;
+  list += 2 * subs;
+  float4 Ap = entry_point(smem, e);
 #pragma unroll point_unroll(NH)
   for (int k = 0; k < n; ++k) {
-    const float4 An = *reinterpret_cast<const float4 *>(ta + (en & 0xffffu));
-    const uint32_t e2 = list[k + 2].x;
-    const float4 *pp = my_ptab + (e >> 16) * 2;
+    const float4 An = entry_point(smem, en);
+    const uint32_t e2 = list->x;
+    list += subs;
+    const float4 *pp = reinterpret_cast<const float4 *>(
+        reinterpret_cast<const unsigned char *>(my_ptab) + (e >> 18));
     float2 d2[NH], r[NH], den[NH], num[NH];
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
@@ -575,6 +635,18 @@ __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (
   }
 }
 
+// Largest value, NaN if there is one: of two values, of a warp's lanes.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+__device__ __forceinline__ float warp_max(float x) {
+  float y;
+  asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Where a warp's placed atoms are, over all lanes: the box of their
 // coordinates, its centre, and the largest distance of an atom from that.
 // Atoms without a usable position (not finite, or so far out that d^9
@@ -583,35 +655,26 @@ struct Region {
   float3 lo, hi, mid;
   float rad;
 };
+// n_my: atoms of this lane's replica (0 in a lane without one); nx = -x
 template <int NA>
 __device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
                                               const float2 (&ny)[NA / 2],
                                               const float2 (&nz)[NA / 2], int n_my) {
-  // n_my: atoms of this lane's replica (0 in a lane without one)
   const float big = 3.0e38f;
-  float lo[3] = {big, big, big}, hi[3] = {-big, -big, -big};
-  bool usable = true;
-#pragma unroll
-  for (int k = 0; k < NA; ++k) {
-    if (k < n_my) {
-      const float2 ax = nx[k >> 1], ay = ny[k >> 1], az = nz[k >> 1];
-      const float v[3] = {-((k & 1) ? ax.y : ax.x), -((k & 1) ? ay.y : ay.x),
-                          -((k & 1) ? az.y : az.x)};
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        usable = usable && fabsf(v[i]) < 5.0e3f;
-        lo[i] = fminf(lo[i], v[i]);
-        hi[i] = fmaxf(hi[i], v[i]);
-      }
-    }
-  }
+  float lo[3], hi[3];  // of the coordinates; m: largest of -x and of x
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
+    const float2(&n)[NA / 2] = i == 0 ? nx : i == 1 ? ny : nz;
+    float m0 = -big, m1 = -big;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[i] = fminf(lo[i], __shfl_xor_sync(0xffffffffu, lo[i], o));
-      hi[i] = fmaxf(hi[i], __shfl_xor_sync(0xffffffffu, hi[i], o));
-    }
+    for (int k = 0; k < NA; ++k)
+      if (k < n_my) {
+        const float v = (k & 1) ? n[k >> 1].y : n[k >> 1].x;
+        m0 = max_nan(m0, v);
+        m1 = max_nan(m1, -v);
+      }
+    lo[i] = -warp_max(m0);
+    hi[i] = warp_max(m1);
   }
   Region g;
   g.lo = make_float3(lo[0], lo[1], lo[2]);
@@ -619,19 +682,19 @@ __device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
   g.mid = make_float3(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]));
   float r2 = 0.f;
 #pragma unroll
-  for (int k = 0; k < NA; ++k) {
-    if (k < n_my) {
-      const float2 ax = nx[k >> 1], ay = ny[k >> 1], az = nz[k >> 1];
-      const float dx = g.mid.x + ((k & 1) ? ax.y : ax.x);
-      const float dy = g.mid.y + ((k & 1) ? ay.y : ay.x);
-      const float dz = g.mid.z + ((k & 1) ? az.y : az.x);
-      r2 = fmaxf(r2, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
-    }
+  for (int h = 0; h < NA / 2; ++h) {
+    const float2 dx = add2(dup2(g.mid.x), nx[h]);
+    const float2 dy = add2(dup2(g.mid.y), ny[h]);
+    const float2 dz = add2(dup2(g.mid.z), nz[h]);
+    const float2 d2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+    r2 = fmaxf(r2, fmaxf(2 * h < n_my ? d2.x : 0.f, 2 * h + 1 < n_my ? d2.y : 0.f));
   }
+  g.rad = sqrtf(warp_max(r2));
+  bool usable = true;  // false for NaN
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, o));
-  g.rad = sqrtf(r2);
-  if (!__all_sync(0xffffffffu, usable)) {
+  for (int i = 0; i < 3; ++i)
+    usable = usable && (lo[i] > hi[i] || (fabsf(lo[i]) < 5.0e3f && fabsf(hi[i]) < 5.0e3f));
+  if (!usable) {
     g.lo = make_float3(-big, -big, -big);
     g.hi = make_float3(big, big, big);
     g.rad = big;
@@ -639,16 +702,19 @@ __device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
   return g;
 }
 
-// Whether the point p is at least D away from the region: outside the box
-// grown by D, or outside the ball grown by D.
-__device__ __forceinline__ bool is_far(const Region &g, const float4 &p, float D) {
+// Squared distance of a point from the region's box.
+__device__ __forceinline__ float box_dist2(const Region &g, const float4 &p) {
   const float bx = fmaxf(fmaxf(g.lo.x - p.x, p.x - g.hi.x), 0.f);
   const float by = fmaxf(fmaxf(g.lo.y - p.y, p.y - g.hi.y), 0.f);
   const float bz = fmaxf(fmaxf(g.lo.z - p.z, p.z - g.hi.z), 0.f);
+  return fmaf(bz, bz, fmaf(by, by, bx * bx));
+}
+// Whether the point, at box_dist2 = b2, is at least D away from the region:
+// outside the box grown by D, or outside the ball grown by D.
+__device__ __forceinline__ bool is_far(const Region &g, const float4 &p, float b2, float D) {
   const float cx = g.mid.x - p.x, cy = g.mid.y - p.y, cz = g.mid.z - p.z;
   const float e = D + g.rad;
-  return fmaf(bz, bz, fmaf(by, by, bx * bx)) > D * D ||
-         fmaf(cz, cz, fmaf(cy, cy, cx * cx)) > e * e;
+  return b2 > D * D || fmaf(cz, cz, fmaf(cy, cy, cx * cx)) > e * e;
 }
 
 // Close-range terms of one protein point (calcenergy_d.cu:80-138): the
@@ -738,11 +804,13 @@ __device__ __forceinline__ void close_range(const float2 (&nx)[NA / 2], const fl
 // HB: atom pairs per warp that evaluate the H-bond term (at least what the
 // launch's items need, KRun.hb_pairs).  PIECES: the CTA runs the pieces of a
 // persistent schedule (KRun.pieces, REMC only), else all steps of unit
-// blockIdx.x.
+// blockIdx.x.  PACKED: units may have few replicas (KRun.packed); a kernel of
+// its own, since the distance between a lane's list entries as a variable
+// costs the pair loop 4% (headline interval 22.0 / 22.8 ms).
 // No producer warp: sm_100 splits the register file between the four
 // schedulers, so a 13th warp would put four warps on one scheduler and cap
 // every thread at 128 registers; 12 warps leave room for about 168.
-template <int MODE, int NA, int HB, bool PIECES>
+template <int MODE, int NA, int HB, bool PIECES, bool PACKED>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     dock_kernel(const __grid_constant__ KRun R) {
   static_assert(NA % 2 == 0, "atoms are processed in pairs");
@@ -753,7 +821,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const int MAXA = A * NA;
   // split launch: clusters of csize CTAs, rank crank, share one unit; CTA
   // crank takes the protein tiles crank, crank + csize, ...
-  const int csize = (MODE != KMODE_POSES && !PIECES && R.split > 1) ? R.split : 1;
+  const int csize = (!PIECES && R.split > 1) ? R.split : 1;
   const SmemLayout SL = smem_layout(A, P, NA, NS, csize);
   float4 *s_ptab = reinterpret_cast<float4 *>(smem + SL.ptab);
   float4 *s_htab = reinterpret_cast<float4 *>(smem + SL.htab);
@@ -763,6 +831,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   float *s_q = reinterpret_cast<float *>(smem + SL.slot_q);
   int *s_lt = reinterpret_cast<int *>(smem + SL.slot_t);
   int *s_atom = reinterpret_cast<int *>(smem + SL.slot_a);
+  SlotKde *s_kde = reinterpret_cast<SlotKde *>(smem + SL.slot_k);
   unsigned char *s_tiles = smem + SL.tiles;
   double *s_red = reinterpret_cast<double *>(smem + SL.red);
   float *s_hpc = reinterpret_cast<float *>(smem + SL.hpc);
@@ -860,6 +929,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
       s_atom[s] = a;
       s_lt[s] = a >= 0 ? TG.lig_t[a] : GD_NLT;
       s_q[s] = a >= 0 ? TG.lig_q[a] : 0.f;
+      SlotKde sk{0, 0, 0.0};
+      if (a >= 0) {
+        const int lt = TG.lig_t[a];
+        sk.begin = TG.kde_off[lt];
+        sk.end = TG.kde_off[lt + 1];
+        sk.inv_n = 1.0 / (double)max(1, sk.end - sk.begin);
+      }
+      s_kde[s] = sk;
     }
     // point types GD_NPT..PT_ROWS-1 (the padding points) get all-zero entries
     for (int i = threadIdx.x; i < A * NH * PT_ROWS; i += blockDim.x) {
@@ -908,11 +985,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 
   // ---- work of this piece ---------------------------------------------------
   int rep0, n_act, prt_conf, lane_rep;
+  int reps, rl;  // replicas held by a warp, and this lane's
   if (MODE == KMODE_POSES) {
-    rep0 = blockIdx.x * 32;
-    n_act = min(32, R.n_pose - rep0);
+    reps = PACKED ? R.packed : 32;
+    rl = lane & (reps - 1);
+    rep0 = unit * reps;
+    n_act = min(reps, R.n_pose - rep0);
     prt_conf = R.prt_conf;
-    lane_rep = rep0 + (lane < n_act ? lane : 0);
+    lane_rep = rep0 + (rl < n_act ? rl : 0);
   } else if (R.group_major) {
     // whole exchange groups: lane = group offset * n_tmp + temperature slot
     const int nt = I.n_tmp, nl = I.n_lig_conf;
@@ -920,17 +1000,28 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     n_act = R.cta_nrep[unit];
     rep0 = g0;
     prt_conf = g0 / nl;
-    const int ln = lane < n_act ? lane : 0;
+    reps = PACKED ? packed_reps(n_act) : 32;
+    rl = lane & (reps - 1);
+    const int ln = rl < n_act ? rl : 0;
     lane_rep = nt * nl * prt_conf + nl * (ln % nt) + (g0 % nl) + ln / nt;
   } else {
     rep0 = R.cta_rep0[unit];
     n_act = R.cta_nrep[unit];
     prt_conf = rep0 / (I.n_tmp * I.n_lig_conf);
-    lane_rep = rep0 + (lane < n_act ? lane : 0);
+    reps = PACKED ? packed_reps(n_act) : 32;
+    rl = lane & (reps - 1);
+    lane_rep = rep0 + (rl < n_act ? rl : 0);
   }
-  const int n_tiles = (T.pnp + TILE_PTS - 1) / TILE_PTS;
   const int crank0 = csize > 1 ? cluster_rank() : 0;
-  const int n_tl = (n_tiles - crank0 + csize - 1) / csize;  // tiles of this CTA
+  // A split unit's ranks take the protein's chunks in turn (rank r the chunks
+  // r, r + split, ...), and stage their own chunks side by side in tiles.
+  // Chunks have half the points then: a rank has few, and the tile groups
+  // wait for the one that got one more (plain 1,500-point complex on 8 CTAs:
+  // whole tiles in turn left four CTAs with 256 points and four with 128).
+  const int cp = csize > 1 ? CHUNK / 2 : CHUNK;  // points of a chunk
+  const int cpt = TILE_PTS / cp;                 // chunks of a staged tile
+  const int n_own = max(0, ((T.pnp + cp - 1) / cp - crank0 + csize - 1) / csize);  // of this CTA
+  const int n_tl = (n_own + cpt - 1) / cpt;      // its staged tiles
   const bool resident = R.resident != 0;
   const int launch_steps = (MODE != KMODE_REMC) ? 1 : (R.item_step ? I.n_run : R.n_steps);
   const int launch_base = (MODE == KMODE_REMC && R.item_step)  ? I.step0
@@ -949,11 +1040,22 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const float4 *src_a = T.pt_a + (size_t)prt_conf * T.pnp_pad;
   const float2 *src_b = T.pt_b;
   const int n_seq = passes * n_tl;
-  auto issue_tile = [&](int s, int t) {
+  // stages this CTA's tl-th tile in stage s
+  auto issue_tile = [&](int s, int tl) {
     unsigned char *dst = s_tiles + (size_t)s * STAGE_BYTES;
-    mbar_arrive_expect_tx(&s_full[s], STAGE_BYTES);
-    bulk_g2s(dst, src_a + (size_t)t * TILE_PTS, TILE_PTS * 16, &s_full[s]);
-    bulk_g2s(dst + TILE_PTS * 16, src_b + (size_t)t * TILE_PTS, TILE_PTS * 8, &s_full[s]);
+    if (csize == 1) {
+      mbar_arrive_expect_tx(&s_full[s], STAGE_BYTES);
+      bulk_g2s(dst, src_a + (size_t)tl * TILE_PTS, TILE_PTS * 16, &s_full[s]);
+      bulk_g2s(dst + TILE_PTS * 16, src_b + (size_t)tl * TILE_PTS, TILE_PTS * 8, &s_full[s]);
+      return;
+    }
+    const int n = min(cpt, n_own - tl * cpt);
+    mbar_arrive_expect_tx(&s_full[s], (uint32_t)(n * cp * 24));
+    for (int q = 0; q < n; ++q) {
+      const size_t p = (size_t)(crank0 + csize * (tl * cpt + q)) * cp;
+      bulk_g2s(dst + q * cp * 16, src_a + p, (uint32_t)(cp * 16), &s_full[s]);
+      bulk_g2s(dst + TILE_PTS * 16 + q * cp * 8, src_b + p, (uint32_t)(cp * 8), &s_full[s]);
+    }
   };
   int it = s_ctl->it;  // ring position of the piece's first tile
   const int tiles_key = item * MAX_PRT_KEY + prt_conf;
@@ -965,10 +1067,10 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     fence_proxy_async_smem();
     if (resident) {
       if (reload)
-        for (int tl = 0; tl < n_tl; ++tl) issue_tile(tl, crank0 + csize * tl);
+        for (int tl = 0; tl < n_tl; ++tl) issue_tile(tl, tl);
     } else {
       for (int q = 0; q < min(NS, n_seq); ++q)
-        issue_tile((it + q) % NS, crank0 + csize * (q % n_tl));
+        issue_tile((it + q) % NS, q % n_tl);
     }
     // the steps before this piece ran on another CTA: wait until it has
     // written their state back (bounded; code 4 if it never does)
@@ -994,16 +1096,17 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const int ag = warp / P, pg = warp % P;
   const int lw = pg * A + ag;
   const int lna = T.lna;
-  const bool active = lane < n_act;
+  const bool active = lane < n_act;  // holds a replica (lanes of the first group)
+  const int subs = PACKED ? 32 / reps : 1, sub = PACKED ? lane / reps : 0;
   const int rep = lane_rep;                    // local replica / pose index
   const int lig_conf = (MODE == KMODE_POSES) ? R.lig_conf : rep % I.n_lig_conf;
   const float4 *orig = T.lig + (size_t)lig_conf * lna;
-  LaneState &me = s_lane[lane];
+  LaneState &me = s_lane[rl];  // written by the first group's lanes
   const float lcx = T.lig_center[0], lcy = T.lig_center[1], lcz = T.lig_center[2];
   // slots of this warp: ag + A k, k < n_my hold atoms
   const int n_my = lna > ag ? min(NA, (lna - ag + A - 1) / A) : 0;
 
-  if (warp == 0) {
+  if (warp == 0 && sub == 0) {
     me.acs = 0;
     me.idx_tmp = 0;
     me.mbeta = 0.f;
@@ -1039,9 +1142,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const float *my_far = s_far + (size_t)ag * PT_ROWS;
   const double *my_fpmf = s_fpmf + (size_t)ag * PT_ROWS;
   uint2 *my_list = reinterpret_cast<uint2 *>(smem + SL.list) + (size_t)warp * LIST_LEN;
-  // entries past a chunk's points are read ahead: point 0 of the tile
-  if (lane < LIST_LEN - CHUNK) my_list[CHUNK + lane] = make_uint2(0u, 0u);
-  my_list[lane] = make_uint2(0u, 0u);
+  // padding points: the record, and the list entry (its vote never fires);
+  // entries past a chunk's points are read ahead, so they start as valid ones
+  const uint2 pad_entry =
+      make_uint2(list_entry((uint32_t)SL.pad, PAD_POINT_TYPE), __float_as_uint(-1.0f));
+  if (threadIdx.x == 0)
+    *reinterpret_cast<float4 *>(smem + SL.pad) =
+        make_float4(PAD_POINT_COORD, PAD_POINT_COORD, PAD_POINT_COORD, 0.f);
+  for (int i = lane; i < LIST_LEN; i += 32) my_list[i] = pad_entry;
   const bool mcc_on = MODE != KMODE_POSES && (I.flags & GD_MC_MCC) != 0u;
   // atom pairs of this warp with an H-bond term for some point type: the
   // first my_nhb pairs (capable atoms come first in the slot order)
@@ -1052,13 +1160,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   // warps whose atoms need fewer H-bond pairs than the launch's HB take a
   // variant with one pair less (most warps of a ligand: the capable atoms
   // come first in the slot order, dealt round robin over the atom groups)
-  constexpr int kHB1 = HB > 1 ? HB - 1 : HB;
+  // (the packed kernel's one HB is every pair; most warps need two at most)
+  constexpr int kHB1 = PACKED ? (HB < 2 ? HB : 2) : HB > 1 ? HB - 1 : HB;
 
   for (int si = 0; si < n_steps; ++si) {
     const int step = step_base + si;
 
     // ---- warp 0 proposes the move and publishes it -------------------------
-    if (warp == 0) {
+    if (warp == 0 && sub == 0) {
       float m_new[6];
       if (MODE == KMODE_REMC) {
         uint32_t k0, k1;
@@ -1088,6 +1197,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll
       for (int i = 0; i < 9; ++i) me.rot[i] = rot[i];
     }
+    // this warp's atoms, loaded while warp 0 is at its move
+    float4 at0[NA];
+#pragma unroll
+    for (int k = 0; k < NA; ++k)
+      at0[k] = (k < n_my) ? orig[s_atom[ag + A * k]] : make_float4(FAR, FAR, FAR, 0.f);
     named_sync(1, W * 32);
 
     // ---- place this warp's atoms (negated: d = atom - point = (-point)... ---
@@ -1102,8 +1216,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     float2 *my_hpc2 = reinterpret_cast<float2 *>(s_hpc) + (size_t)(pg * A + ag) * NH * 32 + lane;
 #pragma unroll
     for (int k = 0; k < NA; ++k) {
-      const float4 o =
-          (k < n_my) ? orig[s_atom[ag + A * k]] : make_float4(FAR, FAR, FAR, 0.f);
+      const float4 o = at0[k];
       const float x = q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx;
       const float y = q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy;
       const float z = q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz;
@@ -1119,7 +1232,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     }
 #pragma unroll
     for (int h = 0; h < NH; ++h) my_hpc2[h * 32] = make_float2(0.f, 0.f);
-    const Region G = warp_region<NA>(nx, ny, nz, active ? n_my : 0);
+    const Region G = warp_region<NA>(nx, ny, nz, rl < n_act ? n_my : 0);
     double far_pmf = 0.0;  // PMF of this lane's far points (every lane's replica)
 
     // ---- pair terms over the protein tiles -----------------------------------
@@ -1128,18 +1241,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     double *my_red = s_red + (size_t)lw * NRED * 32 + lane;
 #pragma unroll
     for (int i = 0; i < NRED; ++i) my_red[i * 32] = 0.0;
-    // resident: the tile groups take the 32-point chunks round robin
-    // (chunk c to group c mod P), which balances them to within one chunk.
+    // resident: the tile groups take the CTA's chunks round robin (chunk c
+    // to group c mod P), which balances them to within one chunk.
     // Streaming: the same split of every tile of the ring, and every warp
     // waits for every stage and reports it done, chunk or not
-    constexpr int CPT = TILE_PTS / CHUNK;  // chunks per tile
     for (int tl = 0; tl < n_tl; ++tl, ++it) {
-      const int t = crank0 + csize * tl;  // protein tile
-      const int nvalid = min(TILE_PTS, T.pnp - t * TILE_PTS);
-      const int nvalid2 = nvalid;
-      const int k0 = ((pg - (t * CPT) % P) % P + P) % P;
-      const int kstep = P;
-      if (resident && k0 * CHUNK >= nvalid2) continue;  // no chunk of this tile here
+      const int n_ck = min(cpt, n_own - tl * cpt);  // chunks of this tile
+      const int k0 = ((pg - (tl * cpt) % P) % P + P) % P;
+      if (resident && k0 >= n_ck) continue;  // no chunk of this tile here
       const int s = resident ? tl : (it % NS);
       // resident tiles: the phase of their latest load (s_ctl->gen loads so far)
       const uint32_t ph = resident ? (uint32_t)((s_ctl->gen - 1) & 1) : (uint32_t)((it / NS) & 1);
@@ -1147,8 +1256,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
       const float4 *ta = reinterpret_cast<const float4 *>(s_tiles + (size_t)s * STAGE_BYTES);
       const float2 *tb =
           reinterpret_cast<const float2 *>(s_tiles + (size_t)s * STAGE_BYTES + TILE_PTS * 16);
-      for (int j0 = k0 * CHUNK; j0 < nvalid2; j0 += kstep * CHUNK) {
-        const int j1 = min(nvalid2, j0 + CHUNK);
+      const uint32_t tile_at = (uint32_t)(SL.tiles + (size_t)s * STAGE_BYTES);
+      for (int ck = k0; ck < n_ck; ck += P) {
+        const int j0 = ck * cp;  // its points in the staged tile and the protein
+        const int p0 = (crank0 + csize * (tl * cpt + ck)) * cp;
+        const int j1 = j0 + min(cp, T.pnp - p0);
         float2 fvdw = dup2(0.f), fpmf = dup2(0.f), fhdb = dup2(0.f);
         float fnear = 0.f, fpsp = 0.f;
         float2 fek[NH];  // sum of ele_p / d per atom (far-field electrostatics)
@@ -1160,44 +1272,61 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         // close-range votes are collected in a mask and served after the
         // branch-free pass, so consecutive points' chains overlap
         // lane j looks at point j: the warp lists the points that are not far
-        // of all its atoms in all lanes, then the far ones (the far form)
+        // of all its atoms in all lanes, then the far ones (the far form); of
+        // the former, those that can have a close-range term come first, so
+        // that packed lanes meet them in few iterations
         const int jl = j0 + lane;
         const bool valid = jl < j1;
-        const uint32_t meta_l = valid ? __float_as_uint(tb[jl].y) : (uint32_t)PAD_POINT_TYPE;
+        const float2 pb_l = valid ? tb[jl] : make_float2(0.f, __uint_as_float(PAD_POINT_TYPE));
+        const uint32_t meta_l = __float_as_uint(pb_l.y);
         const int pt_l = (int)(meta_l & META_TYPE_MASK);
-        const bool far_l =
-            MODE != KMODE_POSES && valid && is_far(G, ta[valid ? jl : j0], my_far[pt_l]);
-        const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
-        const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
-        const int n_near = __popc(near_m), n_far = __popc(far_m);
         float thr_l = T.near4[((meta_l & META_HPC_BIT) ? 1 : 0) |
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
+        const float4 p_l = ta[valid ? jl : j0];
+        const float b2_l = box_dist2(G, p_l);
+        const bool far_l = MODE != KMODE_POSES && valid && is_far(G, p_l, b2_l, my_far[pt_l]);
+        const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
+        const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
+        const uint32_t close_m =
+            subs > 1 ? __ballot_sync(0xffffffffu, valid && !far_l && b2_l <= thr_l) : 0u;
+        // (after the order, which is the same with the MCC score on)
         if (mcc_on) thr_l = fmaxf(thr_l, T.near_mcc2);
+        // iterations of each part: a list entry for each subset
+        const int n_near = __popc(near_m), n_far = __popc(far_m);
+        const int it_near = (n_near + subs - 1) / subs, it_far = (n_far + subs - 1) / subs;
+        const int far0 = it_near * subs;
         const uint32_t below = (1u << lane) - 1u;
         __syncwarp();  // the previous chunk's list has been read
-        if (valid)
-          my_list[far_l ? n_near + __popc(far_m & below) : __popc(near_m & below)] =
-              make_uint2((uint32_t)(jl * 16) | ((uint32_t)pt_l << 16), __float_as_uint(thr_l));
-        __syncwarp();
-        const unsigned char *tab = reinterpret_cast<const unsigned char *>(ta);
-        if (n_far) {
-          if (far_l) far_pmf += my_fpmf[pt_l];
-          chunk_far<NH>(nx, ny, nz, tab, my_list + n_near, n_far, my_ptab, K, fvdw, fek);
+        if (valid) {
+          int at = far0 + __popc(far_m & below);
+          if (!far_l)
+            at = (close_m >> lane) & 1u ? __popc(close_m & below)
+                                        : __popc(close_m) + __popc(near_m & ~close_m & below);
+          my_list[at] = make_uint2(list_entry(tile_at + (uint32_t)jl * 16u, pt_l), __float_as_uint(thr_l));
         }
-        if (n_near) {
+        if (subs > 1) {  // padding points fill both parts
+          if (n_near + lane < far0) my_list[n_near + lane] = pad_entry;
+          if (n_far + lane < it_far * subs) my_list[far0 + n_far + lane] = pad_entry;
+        }
+        __syncwarp();
+        if (it_far) {
+          if (far_l) far_pmf += my_fpmf[pt_l];
+          chunk_far<NH, PACKED>(nx, ny, nz, smem, my_list + far0 + sub, it_far, subs, my_ptab, K,
+                                fvdw, fek);
+        }
+        if (it_near) {
           const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && my_hmask[pt_l] != 0u);
-          // three variants per kernel: no H-bond term, HB - 1 pairs (warps that
-          // need no more) and HB pairs; each is a long unrolled body, so more
-          // of them would cost more in instruction fetch than they save
-          const uint32_t close =
-              (chunk_hdb && my_nhb > 0)
-                  ? (my_nhb <= kHB1
-                         ? chunk_fast<NH, kHB1>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab,
-                                                K, fvdw, fpmf, fhdb, fek)
-                         : chunk_fast<NH, HB>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab,
-                                              K, fvdw, fpmf, fhdb, fek))
-                  : chunk_fast<NH, 0>(nx, ny, nz, tab, my_list, n_near, my_ptab, my_htab, K,
-                                      fvdw, fpmf, fhdb, fek);
+          // three variants per kernel: no H-bond term, kHB1 pairs (warps that
+          // need no more) and HB pairs; each is a long body, so more of them
+          // would cost more in instruction fetch than they save
+          auto near_part = [&](auto hb) {
+            return chunk_fast<NH, decltype(hb)::value, PACKED>(nx, ny, nz, smem, my_list + sub,
+                                                               it_near, subs, my_ptab, my_htab,
+                                                               K, fvdw, fpmf, fhdb, fek);
+          };
+          const uint32_t close = !chunk_hdb || my_nhb <= 0 ? near_part(Int<0>{})
+                                 : my_nhb <= kHB1          ? near_part(Int<kHB1>{})
+                                                           : near_part(Int<HB>{});
           if (close) {
             // the chunk's hydrophobic sums in registers, added to the per-atom
             // sums once per chunk
@@ -1205,11 +1334,15 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll
             for (int h = 0; h < NH; ++h) hacc[h] = make_float2(0.f, 0.f);
             for (uint32_t m = close; m != 0u; m &= m - 1u) {
-              const int j = (int)(my_list[__ffs(m) - 1].x & 0xffffu) >> 4;
-              const uint32_t meta = __float_as_uint(tb[j].y);
-              close_range<NA>(nx, ny, nz, ta[j], tb[j].x, meta,
+              // this lane's point of the iteration (a padding point has no term)
+              const uint32_t e = my_list[(__ffs(m) - 1) * subs + sub].x;
+              const int j = ((int)entry_at(e) - (int)tile_at) / 16;
+              const bool real = e != pad_entry.x;
+              const float2 pb = real ? tb[j] : make_float2(0.f, __uint_as_float(PAD_POINT_TYPE));
+              const uint32_t meta = __float_as_uint(pb.y);
+              close_range<NA>(nx, ny, nz, entry_point(smem, e), pb.x, meta,
                               my_ptab + (int)(meta & META_TYPE_MASK) * 2, T, s_q, s_lt, s_atom,
-                              hacc, A, ag, n_my, inv_el1, fnear, fpsp, mcc_on, t * TILE_PTS + j,
+                              hacc, A, ag, n_my, inv_el1, fnear, fpsp, mcc_on, p0 + j - j0,
                               my_red);
             }
 #pragma unroll
@@ -1240,7 +1373,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
             const int q = it - s_ctl->first_it;  // position within the piece
             if (q + NS < n_seq) {
               fence_proxy_async_smem();
-              issue_tile(s, crank0 + csize * ((q + NS) % n_tl));
+              issue_tile(s, (q + NS) % n_tl);
             }
           }
         }
@@ -1250,46 +1383,52 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     // the far points' PMF, summed over the lanes that hold them
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) far_pmf += __shfl_xor_sync(0xffffffffu, far_pmf, o);
-    my_red[2 * 32] += far_pmf;
+    if (sub == 0) my_red[2 * 32] += far_pmf;
 
-    // ---- KDE ------------------------------------------------------------------
+    // ---- KDE and LHM position restraints ---------------------------------------
+    // One task per ligand atom (its KDE points) and per MCS record, dealt over
+    // the ranks and warps; the lane groups share a task's points or atoms.  A
+    // loop of small bodies, not unrolled: once a step, its instructions come
+    // from beyond the first instruction cache.
     double dkde = 0.0, dlhm = 0.0;
-#pragma unroll
-    for (int k = 0; k < NA; ++k) {
-      if (k < n_my && k % P == pg && crank0 == 0) {  // rank 0 of a split
-        const int lt = s_lt[ag + A * k];
-        const int kb = T.kde_off[lt], ke = T.kde_off[lt + 1];
-        if (ke > kb) {
-          const float2 ax = nx[k >> 1], ay = ny[k >> 1], az = nz[k >> 1];
-          const float x = -((k & 1) ? ax.y : ax.x);
-          const float y = -((k & 1) ? ay.y : ay.x);
-          const float z = -((k & 1) ? az.y : az.x);
+    auto placed = [&](int a) {
+      const float4 o = orig[a];
+      return make_float3(q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx,
+                         q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy,
+                         q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz);
+    };
+#pragma unroll 1
+    for (int i = crank0 + csize * lw; i < lna + T.pos; i += csize * W) {
+      if (i < lna) {
+        const SlotKde sk = s_kde[i];
+        if (sk.end > sk.begin) {
+          const float3 x = placed(s_atom[i]);
           float kv = 0.f;
-          for (int q = kb; q < ke; ++q) {
+#pragma unroll 1
+          for (int q = sk.begin + sub; q < sk.end; q += subs) {
             const float4 K = T.kde[q];
-            const float dx = x - K.x, dy = y - K.y, dz = z - K.z;
+            const float dx = x.x - K.x, dy = x.y - K.y, dz = x.z - K.z;
             kv += fex2(T.kde2 * LOG2E * fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
           }
-          dkde += (double)kv / (double)(ke - kb);
+          dkde += (double)kv * sk.inv_n;
         }
-      }
-    }
-    // ---- LHM position restraints: MCS records m = lw, lw + W, ... -----------
-    for (int m = crank0 == 0 ? lw : T.pos; m < T.pos; m += W) {
-      float sv = 0.f;
-      const float4 *Mm = T.mcs + (size_t)m * lna;
-      for (int l = 0; l < lna; ++l) {
-        const float4 M = Mm[l];
-        if (M.w != 0.0f) {
-          const float4 o = orig[l];
-          const float x = q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx;
-          const float y = q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy;
-          const float z = q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz;
-          const float dx = x - M.x, dy = y - M.y, dz = z - M.z;
-          sv += fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      } else {
+        const int m = i - lna;
+        float sv = 0.f;
+        const float4 *Mm = T.mcs + (size_t)m * lna;
+        const double2 w = T.mcs_w[m];
+#pragma unroll 1
+        for (int l = sub; l < lna; l += subs) {
+          const float4 M = Mm[l];
+          if (M.w != 0.0f) {
+            const float3 x = placed(l);
+            const float dx = x.x - M.x, dy = x.y - M.y, dz = x.z - M.z;
+            sv += fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+          }
         }
+        sv = sum_subs(sv, reps);
+        if (sub == 0) dlhm += w.x * sqrt((double)sv * w.y);
       }
-      dlhm += (double)T.mcs_tcc[m] * sqrt((double)sv / (double)T.mcs_cnt[m]);
     }
 
     // ---- cross-warp reduction and finalisation (warp 0) ----------------------
@@ -1315,7 +1454,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         if (i < NRED) {
           double acc = 0.0;
           for (int w = 0; w < W; ++w) acc += s_red[((size_t)w * NRED + i) * 32 + lane];
-          xs[i * 32 + lane] = acc;
+          xs[i * 32 + lane] = sum_subs(acc, reps);
         } else {
           const int j = i - NRED;  // atom pair (ag, h) = (j / NH, j % NH)
           float2 v = make_float2(0.f, 0.f);
@@ -1324,33 +1463,42 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
             v.x += x.x;
             v.y += x.y;
           }
-          xh2[j * 32 + lane] = v;
+          xh2[j * 32 + lane] = make_float2(sum_subs(v.x, reps), sum_subs(v.y, reps));
         }
       }
       cluster_sync_all();
-      // then all ranks' buffers in rank order into slot 0 (terms) and tile
-      // group 0's slots (the atom pairs' hydrophobic restraints)
-      for (int i = lw; i < NRED + A * NH; i += W) {
+      // then all ranks' buffers (all loads in flight) in rank order
+      // into slot 0 (terms) and tile group 0's slots (the atom pairs'
+      // hydrophobic restraints); packed lanes take a task for each lane group
+      for (int i = lw * subs + sub; i < NRED + A * NH; i += W * subs) {
         if (i < NRED) {
+          double v[MAX_SPLIT];
+#pragma unroll
+          for (int r = 0; r < MAX_SPLIT; ++r) v[r] = r < csize ? cluster_map(xs, r)[i * 32 + rl] : 0.0;
           double acc = 0.0;
-          for (int r = 0; r < csize; ++r) acc += cluster_map(xs, r)[i * 32 + lane];
-          s_red[(size_t)i * 32 + lane] = acc;
+#pragma unroll
+          for (int r = 0; r < MAX_SPLIT; ++r) acc += v[r];
+          s_red[(size_t)i * 32 + rl] = acc;
         } else {
           const int j = i - NRED, ai = j / NH, hp = j % NH;
+          float2 x[MAX_SPLIT];
+#pragma unroll
+          for (int r = 0; r < MAX_SPLIT; ++r)
+            x[r] = r < csize ? cluster_map(xh2, r)[j * 32 + rl] : make_float2(0.f, 0.f);
           float2 v = make_float2(0.f, 0.f);
-          for (int r = 0; r < csize; ++r) {
-            const float2 x = cluster_map(xh2, r)[j * 32 + lane];
-            v.x += x.x;
-            v.y += x.y;
+#pragma unroll
+          for (int r = 0; r < MAX_SPLIT; ++r) {
+            v.x += x[r].x;
+            v.y += x[r].y;
           }
           if (ai + 2 * hp * A < lna)
-            s_hpc2[hpc_pair_at(0, ai, hp, lane, A, NH)] = hpc_transform(T, s_lt, A, ai, hp, v);
+            s_hpc2[hpc_pair_at(0, ai, hp, rl, A, NH)] = hpc_transform(T, s_lt, A, ai, hp, v);
         }
       }
       named_sync(1, W * 32);
       if (warp == 0)
-        finish_step<MODE>(R, I, me, s_red, s_hpc, s_lt, 1, 1, A, NH, lane, rep, active, prt_conf,
-                          lig_conf, step, crank0 == 0, true);
+        finish_step<MODE>(R, I, me, s_red, s_hpc, A, NH, lane, reps, rep, active, prt_conf,
+                          lig_conf, step, crank0 == 0);
     } else {
       // spread over the warps (tasks i = lw, lw + W, ...): the cross-warp sum
       // of each of the NRED terms (in warp-slot order, into slot 0) and the
@@ -1361,18 +1509,18 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         if (i < NRED) {
           double acc = 0.0;
           for (int w = 0; w < W; ++w) acc += s_red[((size_t)w * NRED + i) * 32 + lane];
-          s_red[(size_t)i * 32 + lane] = acc;
+          s_red[(size_t)i * 32 + lane] = sum_subs(acc, reps);
         } else {
           const int ai = (i - NRED) / NH, hp = (i - NRED) % NH;
           if (ai + 2 * hp * A >= lna) continue;
-          const float2 r = hpc_restraint(T, s_hpc2, s_lt, P, A, NH, ai, hp, lane);
+          const float2 r = hpc_restraint(T, s_hpc2, s_lt, P, A, NH, ai, hp, lane, reps);
           s_hpc2[hpc_pair_at(0, ai, hp, lane, A, NH)] = r;
         }
       }
       named_sync(1, W * 32);
       if (warp == 0)
-        finish_step<MODE>(R, I, me, s_red, s_hpc, s_lt, 1, P, A, NH, lane, rep, active, prt_conf,
-                          lig_conf, step, true, true);
+        finish_step<MODE>(R, I, me, s_red, s_hpc, A, NH, lane, reps, rep, active, prt_conf,
+                          lig_conf, step, true);
     }
     // the next step's first barrier orders warp 0's updates (and its use of
     // s_red for the exchange) before any other warp touches them again
@@ -1416,6 +1564,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   }
 }
 
+#if GD_DOCK_PART == 0
 // Temperature exchange, one thread per (item, protein conf, ligand conf)
 // group (exchangereplicas_d.cu:26-79).  Pairs of adjacent temperature
 // indices (2 pair + mode_t, 2 pair + mode_t + 1) swap their slots when
@@ -1519,25 +1668,31 @@ __global__ void fma_peak_kernel(float *out, int iters) {
   const float s = a0 + a1 + a2 + a3 + a4 + a5 + a6 + a7;
   if (s == 12345.678f) out[blockIdx.x] = s;
 }
+#endif  // GD_DOCK_PART == 0
 
 // ---------------------------------------------------------------------------
-template <int MODE, int NA, int HB, bool PIECES>
+template <int MODE, int NA, int HB, bool PIECES, bool PACKED>
 static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *occ) {
-  const int split = (MODE != KMODE_POSES && !PIECES && R.split > 1) ? R.split : 1;
+  const int split = (!PIECES && R.split > 1) ? R.split : 1;
   const size_t smem = dock_smem_bytes(R.A, R.P, NA, R.n_stages, split);
   const int threads = R.A * R.P * 32;
-  cudaError_t e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES>,
+  cudaError_t e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, PACKED>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (occ)  // occupancy query instead of a launch
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dock_kernel<MODE, NA, HB, PIECES>,
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dock_kernel<MODE, NA, HB, PIECES, PACKED>,
                                                          threads, smem);
   if (split == 1) {
-    dock_kernel<MODE, NA, HB, PIECES><<<grid, threads, smem, s>>>(R);
+    dock_kernel<MODE, NA, HB, PIECES, PACKED><<<grid, threads, smem, s>>>(R);
     return cudaGetLastError();
   }
   // clusters of `split` CTAs (grid = units x split), on SMs of one GPC
-  if (split > 8 || grid % split) return cudaErrorInvalidValue;
+  if (split > MAX_SPLIT || grid % split) return cudaErrorInvalidValue;
+  if (split > 8) {  // beyond the portable size
+    e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, PACKED>,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -1550,49 +1705,76 @@ static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *o
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, dock_kernel<MODE, NA, HB, PIECES>, R);
-}
-
-template <int MODE, int NA, int HB>
-static cudaError_t launch_nahb(const KRun &R, int grid, cudaStream_t s, int *occ) {
-  if constexpr (MODE == KMODE_REMC) {
-    if (R.pieces) return launch_kernel<MODE, NA, HB, true>(R, grid, s, occ);
-  } else {
-    if (R.pieces) return cudaErrorInvalidValue;  // schedules are for MC steps
-  }
-  return launch_kernel<MODE, NA, HB, false>(R, grid, s, occ);
+  return cudaLaunchKernelEx(&cfg, dock_kernel<MODE, NA, HB, PIECES, PACKED>, R);
 }
 
 // Three H-bond bounds per NA: at most two or three pairs (ligands where up
 // to about a third or half of the atoms have the term, the common cases), or
-// every pair.
-template <int MODE, int NA>
+// every pair, which is the packed kernel's only one.
+template <int MODE, int NA, bool PIECES, bool PACKED>
 static cudaError_t launch_na(const KRun &R, int grid, cudaStream_t s, int *occ) {
   constexpr int NH = NA / 2;
   constexpr int HB2 = NH < 2 ? NH : 2;
   constexpr int HB3 = NH < 3 ? NH : 3;
-  if (R.hb_pairs <= HB2) return launch_nahb<MODE, NA, HB2>(R, grid, s, occ);
-  if (R.hb_pairs <= HB3) return launch_nahb<MODE, NA, HB3>(R, grid, s, occ);
-  return launch_nahb<MODE, NA, NH>(R, grid, s, occ);
+  if constexpr (!PACKED) {
+    if (R.hb_pairs <= HB2) return launch_kernel<MODE, NA, HB2, PIECES, false>(R, grid, s, occ);
+    if (R.hb_pairs <= HB3) return launch_kernel<MODE, NA, HB3, PIECES, false>(R, grid, s, occ);
+  }
+  return launch_kernel<MODE, NA, NH, PIECES, PACKED>(R, grid, s, occ);
 }
 
-template <int MODE>
-static cudaError_t launch_mode(const KRun &R, int NA, int grid, cudaStream_t s, int *occ) {
+// The kernel variants are compiled in several objects of this source
+// (GD_DOCK_PART 1 .. 5; part 0 holds everything else).
+template <int MODE, bool PIECES, bool PACKED>
+cudaError_t launch_part(const KRun &R, int NA, int grid, cudaStream_t s, int *occ);
+
+#if GD_DOCK_PART > 0
+template <int MODE, bool PIECES, bool PACKED>
+cudaError_t launch_part(const KRun &R, int NA, int grid, cudaStream_t s, int *occ) {
   switch (NA) {
-    case 2: return launch_na<MODE, 2>(R, grid, s, occ);
-    case 4: return launch_na<MODE, 4>(R, grid, s, occ);
-    case 6: return launch_na<MODE, 6>(R, grid, s, occ);
-    case 8: return launch_na<MODE, 8>(R, grid, s, occ);
-    case 10: return launch_na<MODE, 10>(R, grid, s, occ);
+    case 2: return launch_na<MODE, 2, PIECES, PACKED>(R, grid, s, occ);
+    case 4: return launch_na<MODE, 4, PIECES, PACKED>(R, grid, s, occ);
+    case 6: return launch_na<MODE, 6, PIECES, PACKED>(R, grid, s, occ);
+    case 8: return launch_na<MODE, 8, PIECES, PACKED>(R, grid, s, occ);
+    case 10: return launch_na<MODE, 10, PIECES, PACKED>(R, grid, s, occ);
     default: return cudaErrorInvalidValue;
   }
 }
+#define GD_DOCK_VARIANT(MODE, PIECES, PACKED)                                                  \
+  template cudaError_t launch_part<MODE, PIECES, PACKED>(const KRun &, int, int, cudaStream_t, \
+                                                         int *)
+#if GD_DOCK_PART == 1
+GD_DOCK_VARIANT(KMODE_POSES, false, false);
+GD_DOCK_VARIANT(KMODE_POSES, false, true);
+#elif GD_DOCK_PART == 2
+GD_DOCK_VARIANT(KMODE_REMC, false, false);
+#elif GD_DOCK_PART == 3
+GD_DOCK_VARIANT(KMODE_REMC, true, false);
+#elif GD_DOCK_PART == 4
+GD_DOCK_VARIANT(KMODE_REMC, false, true);
+GD_DOCK_VARIANT(KMODE_REMC, true, true);
+#else
+GD_DOCK_VARIANT(KMODE_INIT, false, false);
+GD_DOCK_VARIANT(KMODE_INIT, false, true);
+#endif
 
+#else
 static cudaError_t dock_dispatch(const KRun &R, int NA, int grid, cudaStream_t s, int *occ) {
+  if (R.pieces && R.mode != KMODE_REMC) return cudaErrorInvalidValue;  // for MC steps
+  const bool packed = R.packed != 0;
   switch (R.mode) {
-    case KMODE_POSES: return launch_mode<KMODE_POSES>(R, NA, grid, s, occ);
-    case KMODE_REMC: return launch_mode<KMODE_REMC>(R, NA, grid, s, occ);
-    default: return launch_mode<KMODE_INIT>(R, NA, grid, s, occ);
+    case KMODE_POSES:
+      return packed ? launch_part<KMODE_POSES, false, true>(R, NA, grid, s, occ)
+                    : launch_part<KMODE_POSES, false, false>(R, NA, grid, s, occ);
+    case KMODE_REMC:
+      if (R.pieces)
+        return packed ? launch_part<KMODE_REMC, true, true>(R, NA, grid, s, occ)
+                      : launch_part<KMODE_REMC, true, false>(R, NA, grid, s, occ);
+      return packed ? launch_part<KMODE_REMC, false, true>(R, NA, grid, s, occ)
+                    : launch_part<KMODE_REMC, false, false>(R, NA, grid, s, occ);
+    default:
+      return packed ? launch_part<KMODE_INIT, false, true>(R, NA, grid, s, occ)
+                    : launch_part<KMODE_INIT, false, false>(R, NA, grid, s, occ);
   }
 }
 
@@ -1642,5 +1824,7 @@ cudaError_t launch_fma_peak(float *out, int n_blocks, int iters, cudaStream_t s)
   fma_peak_kernel<<<n_blocks, 256, 0, s>>>(out, iters);
   return cudaGetLastError();
 }
+
+#endif  // GD_DOCK_PART
 
 }  // namespace gd

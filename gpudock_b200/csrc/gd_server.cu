@@ -95,6 +95,7 @@ struct Lane {
   Tile tile;
   int ns = 0, res = 0, gm = 0, spe = 0;
   int split = 1;                    // CTAs (a cluster) per request unit
+  int packed = 0;                   // some unit has at most 16 replicas (KRun.packed)
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   // the lane's kernel error word, in pinned host memory the kernels write
@@ -117,8 +118,9 @@ struct Lane {
   } desc[2];
 };
 
-// (A, P, NA, stages, resident, group-major, steps per exchange, split, sub-lane)
-using LaneKey = std::tuple<int, int, int, int, int, int, int, int, int>;
+// (A, P, NA, stages, resident, group-major, steps per exchange, split, packed,
+// sub-lane)
+using LaneKey = std::tuple<int, int, int, int, int, int, int, int, int, int>;
 constexpr int kMaxLanes = 512;
 // Lanes per launch shape.  A lane relaunches only when the slowest CTA of its
 // launch has finished, so its other SMs wait meanwhile unless other lanes'
@@ -165,11 +167,11 @@ namespace {
 // Device bytes a request holds while active (tables + replica state, and
 // its per-step record with GD_MC_RECORD).
 size_t request_bytes(const gd_complex *cx, const gd_mc_params *mc, int n_rep) {
-  size_t b = (size_t)TAB_ROWS * GD_NPT * 24;
+  size_t b = (size_t)TAB_ROWS * GD_NPT * 28;
   b += (size_t)cx->lig.n_conf * cx->lig.lna * 16 + (size_t)cx->lig.lna * 8;
   b += (size_t)GD_NLT * cx->psp.n_col * 4;
   b += (size_t)cx->kde.pnk * 16 + (GD_NLT + 1) * 4;
-  b += (size_t)cx->mcs.pos * cx->lig.lna * 16 + (size_t)cx->mcs.pos * 8;
+  b += (size_t)cx->mcs.pos * cx->lig.lna * 16 + (size_t)cx->mcs.pos * 16;
   b += (size_t)n_rep * (6 + GD_NTERM + 3) * 4 + 3 * MAX_TMP * 4;
   // MCC reference map: one bit per (atom, padded point)
   b += (size_t)cx->lig.lna * ((cx->prt.pnp + TILE_PTS - 1) / TILE_PTS) * (TILE_PTS / 8);
@@ -226,12 +228,13 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
   pick_stages(T, t, &ns, &res, split);
   const bool gm = (32 % r->mc.n_tmp) == 0;
   const int spe = r->mc.steps_per_exchange;
+  const int packed = has_packed_units(T.n_prt, T.n_lig, r->mc.n_tmp) ? 1 : 0;
   // the shape's least loaded lane; a new one while that lane holds requests
   // and the shape has fewer than kSubLanes
   Lane *best = nullptr;
   int n_sub = 0;
   for (int sub = 0; sub < kSubLanes; ++sub) {
-    auto it = S->lanes.find(LaneKey{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, spe, split, sub});
+    auto it = S->lanes.find(LaneKey{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, spe, split, packed, sub});
     if (it == S->lanes.end()) break;
     ++n_sub;
     Lane *L = it->second.get();
@@ -242,7 +245,7 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
     *out = best;
     return GD_OK;
   }
-  const LaneKey key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, spe, split, n_sub};
+  const LaneKey key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, spe, split, packed, n_sub};
   auto L = std::make_unique<Lane>();
   L->tile = t;
   L->ns = ns;
@@ -250,6 +253,7 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
   L->gm = gm ? 1 : 0;
   L->spe = spe;
   L->split = split;
+  L->packed = packed;
   const int slot = (int)S->lanes.size();
   if (slot >= kMaxLanes) return fail(GD_ENOMEM, "more than %d lanes in the server", kMaxLanes);
   GD_CUDA(cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking));
@@ -390,6 +394,7 @@ gd_status launch_lane(gd_server *S, Lane &L, const std::vector<Req *> &rs, int m
   R.err = L.h_err;
   R.busy_ns = S->d_busy_ns;
   R.split = L.split;
+  R.packed = L.packed;
   for (const Req *r : rs) R.hb_pairs = std::max(R.hb_pairs, hb_pairs_of(r->item.T, L.tile.A));
   GD_CUDA(launch_dock(R, L.tile.NA, (int)n_cta * L.split, s));
   S->ctx->launches += 1;
