@@ -22,7 +22,7 @@ LIBDIR = os.path.join(HERE, "_lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libgpudock.so")
 SOURCES = ["gd_kernels.cu", "gd_api.cu", "gd_ensemble.cu", "gd_server.cu", "gd_noalloc.cu",
-           "gd_similarity.cu", "gd_load.cpp"]
+           "gd_poses.cu", "gd_similarity.cu", "gd_load.cpp"]
 # the kernel variants of gd_kernels.cu are compiled in parts, in parallel
 PARTS = {"gd_kernels.cu": [f"-DGD_DOCK_PART={k}" for k in range(6)]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -85,7 +85,10 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 int lna_bucket(int lna) { return std::min(((lna + 7) / 8) * 8, MAX_LNA); }
 
 int split_for(gd_ctx *ctx, const KTables &T, int run_units, double min_cost) {
-  if (ctx->split_mode > 0) return ctx->split_mode;
+  return ctx->split_mode > 0 ? ctx->split_mode : split_rule(ctx, T, run_units, min_cost);
+}
+
+int split_rule(gd_ctx *ctx, const KTables &T, int run_units, double min_cost) {
   // the largest power of two <= cost / min_cost and <= SMs / units, at most
   // 8: a run that fills the GPU with units gains nothing from splitting
   const double cost = (double)lna_bucket(T.lna) * T.pnp;
@@ -833,14 +836,25 @@ extern "C" gd_status gd_complex_upload_shared(gd_ctx *ctx, const gd_complex *cx,
 // ---------------------------------------------------------------------------
 // Pose energies
 // ---------------------------------------------------------------------------
-static gd_status poses_launch(gd_ctx *ctx, const gd_dcomplex *d, const Tile &tile, int prt_conf,
-                              int lig_conf, int n_pose, const float *poses, float *terms,
-                              double *raw, KItem **d_item) {
+// The unit of a small call: with few poses the launch would leave most SMs
+// idle, so a unit's points are split over a cluster (as MC units, split_rule),
+// and then the poses over more units of 16 or 8 poses (lane packing).
+static void pose_units(gd_ctx *ctx, const KTables &T, int n_pose, int *split, int *packed) {
+  int per = 32;
+  auto units = [&](int p) { return (n_pose + p - 1) / p; };
+  *split = split_rule(ctx, T, units(32), kRunSplitCost);
+  while (per > 8 && units(per / 2) > units(per) && units(per / 2) * *split <= ctx->n_sm) per /= 2;
+  *packed = per < 32 ? per : 0;
+}
+
+gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int lig_conf,
+                           int n_pose, const float *poses, float *terms, double *raw,
+                           void *work) {
+  const Tile tile = tile_for(ctx, d->T);
   KRun R{};
   R.mode = KMODE_POSES;
   R.A = tile.A;
   R.P = tile.P;
-  pick_stages(d->T, tile, &R.n_stages, &R.resident);
   R.prt_conf = prt_conf;
   R.lig_conf = lig_conf;
   R.n_pose = n_pose;
@@ -849,15 +863,21 @@ static gd_status poses_launch(gd_ctx *ctx, const gd_dcomplex *d, const Tile &til
   R.raw = raw;
   R.err = ctx->d_err;
   R.hb_pairs = hb_pairs_of(d->T, tile.A);
-  KItem it{};
-  it.T = d->T;
-  it.n_tmp = 1;
-  it.n_lig_conf = d->T.n_lig;
-  it.n_prt = d->T.n_prt;
-  GD_CUDA(cudaMallocAsync((void **)d_item, sizeof(KItem), ctx->stream));
-  GD_CUDA(cudaMemcpyAsync(*d_item, &it, sizeof(KItem), cudaMemcpyHostToDevice, ctx->stream));
-  R.items = *d_item;
-  GD_CUDA(launch_dock(R, tile.NA, (n_pose + 31) / 32, ctx->stream));
+  R.pose_item.T = d->T;
+  R.pose_item.n_tmp = 1;
+  R.pose_item.n_lig_conf = d->T.n_lig;
+  R.pose_item.n_prt = d->T.n_prt;
+  int grid = 0;
+  if (work) {
+    GD_CUDA(pose_cells(&R, work, &grid, ctx->stream));
+    ctx->launches += 4;
+  } else {
+    pose_units(ctx, d->T, n_pose, &R.split, &R.packed);
+    const int per = R.packed ? R.packed : 32;
+    grid = (n_pose + per - 1) / per * R.split;
+  }
+  pick_stages(d->T, tile, &R.n_stages, &R.resident, std::max(1, R.split));
+  GD_CUDA(launch_dock(R, tile.NA, grid, ctx->stream));
   ctx->launches += 1;
   return GD_OK;
 }
@@ -875,10 +895,12 @@ extern "C" gd_status gd_energy_poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int 
   if (n_pose == 0) return GD_OK;
   if (!poses || !terms) return fail(GD_EINVAL, "poses/terms NULL");
   GD_CUDA(cudaSetDevice(ctx->device));
-  KItem *dit = nullptr;
-  gd_status st = poses_launch(ctx, d, tile_for(ctx, d->T), prt_conf, lig_conf, n_pose, poses,
-                              terms, raw, &dit);
-  if (dit) cudaFreeAsync(dit, ctx->stream);
+  void *work = nullptr;
+  const size_t bytes = pose_work_bytes(d->T, n_pose);
+  if (bytes) GD_CUDA(cudaMallocAsync(&work, bytes, ctx->stream));
+  const gd_status st =
+      poses_launch(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, work);
+  if (work) cudaFreeAsync(work, ctx->stream);
   return st;
 }
 

@@ -131,6 +131,10 @@ inline bool injected_alloc_failure(gd_ctx *c) {
 // shapes are chosen (and autotuned) per bucket and cover its largest size.
 int lna_bucket(int lna);
 Tile tile_for(gd_ctx *ctx, const KTables &T);
+// The energy launch of a pose call (gd_api.cu): poses, terms and raw are
+// device pointers, work pose_work_bytes of device memory (nullptr without).
+gd_status poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int lig_conf, int n_pose,
+                       const float *poses, float *terms, double *raw, void *work);
 // CTAs (a thread-block cluster) that share each 32-replica unit of a complex
 // in MC launches: a function of the complex (ligand-size bucket x protein
 // points) and of the units of its own run, never of what else runs, so
@@ -141,6 +145,8 @@ Tile tile_for(gd_ctx *ctx, const KTables &T);
 // kServeSplitCost, so that splitting under load costs little throughput.
 constexpr double kRunSplitCost = 4500.0;
 constexpr double kServeSplitCost = 42500.0;
+int split_rule(gd_ctx *ctx, const KTables &T, int run_units, double min_cost);
+// The split of an MC run: the context's own (gd_ctx_set_split), else the rule's.
 int split_for(gd_ctx *ctx, const KTables &T, int run_units, double min_cost);
 // 32-replica units of a complex's replicas (n_prt x n_lig x n_tmp): whole
 // exchange groups per unit when n_tmp divides 32.

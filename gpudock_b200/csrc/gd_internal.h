@@ -118,6 +118,15 @@ struct KItem {
   int *acs_mc;              // [n_rep]
 };
 
+// The cells of a pose call (gd_poses.cu): a grid over the translations; poses
+// without a usable translation are in cell n_cells.
+struct PoseGrid {
+  float lo[3], edge, inv_edge;
+  float margin;   // how far outside its cell a pose can lie (rounding)
+  int n[3], n_cells;
+  int n_blocks;   // blocks of up to 32 poses of one cell
+};
+
 // Launch descriptor of one dock_kernel launch (by value).
 struct KRun {
   int mode;              // KMode
@@ -134,11 +143,17 @@ struct KRun {
   int fused_exchange;    // group_major only: exchange inside the kernel after
                          // every spe MC steps
   int spe;               // MC steps per exchange
-  // poses (item 0)
+  // poses: the item is passed by value, so that a call needs no copy of it
+  KItem pose_item;
   int prt_conf, lig_conf, n_pose;
   const float *poses;    // [n_pose][6]
   float *terms;          // [n_pose][GD_NTERM]
   double *raw;           // [n_pose][GD_NRAW] or nullptr
+  // poses dealt into cells (nullptr: unit u holds poses 32 u ..): block b
+  // holds poses pose_order[32 b ..] of cell pose_cell[b], whose first block
+  // is cell_first[cell] and which holds cell_count[cell] poses
+  const PoseGrid *pose_grid;
+  const int *pose_order, *pose_cell, *cell_first, *cell_count;
   // REMC: the first MC step and the step count are KItem.step0 / n_run with
   // item_step (complexes at different steps in one launch), else the first
   // step is *step_ptr when step_ptr is set (graph replay), else step0
@@ -215,6 +230,14 @@ struct KGroup {
 };
 
 size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split = 1);
+
+// Device workspace that a pose call wants for dealing its poses into cells, 0
+// for a call too small to gain from them (gd_poses.cu).
+size_t pose_work_bytes(const KTables &T, int n_pose);
+// Deals the poses of R (n_pose, poses) into cells, using pose_work_bytes of
+// workspace until the energy launch has ended; fills R's cell arrays and the
+// launch's grid.
+cudaError_t pose_cells(KRun *R, void *work, int *grid, cudaStream_t s);
 
 // Kernel launchers (gd_kernels.cu); return the launch status.
 cudaError_t launch_dock(const KRun &R, int NA, int grid, cudaStream_t s);

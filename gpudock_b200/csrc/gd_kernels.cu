@@ -702,6 +702,29 @@ __device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
   return g;
 }
 
+// The region of the translations of a pose block's cell (unbounded without
+// cells, and for the cell of poses that have no usable translation).
+__device__ __forceinline__ Region pose_region(const KRun &R, int unit, float cx, float cy,
+                                              float cz) {
+  const float big = 3.0e38f;
+  Region g;
+  g.lo = make_float3(-big, -big, -big);
+  g.hi = make_float3(big, big, big);
+  g.mid = make_float3(0.f, 0.f, 0.f);
+  g.rad = big;
+  if (!R.pose_grid) return g;
+  const PoseGrid &P = *R.pose_grid;
+  const int cell = R.pose_cell[unit];
+  if (cell >= P.n_cells) return g;
+  const int x = cell % P.n[0], y = cell / P.n[0] % P.n[1], z = cell / P.n[0] / P.n[1];
+  const float m = P.margin;
+  g.lo = make_float3(cx + P.lo[0] + x * P.edge - m, cy + P.lo[1] + y * P.edge - m,
+                     cz + P.lo[2] + z * P.edge - m);
+  g.hi = make_float3(g.lo.x + P.edge + 2.f * m, g.lo.y + P.edge + 2.f * m,
+                     g.lo.z + P.edge + 2.f * m);
+  return g;
+}
+
 // Squared distance of a point from the region's box.
 __device__ __forceinline__ float box_dist2(const Region &g, const float4 &p) {
   const float bx = fmaxf(fmaxf(g.lo.x - p.x, p.x - g.hi.x), 0.f);
@@ -911,12 +934,16 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     wait_dep = pz.w != 0;
   }
 
+  // a pose launch's grid is an upper bound of its blocks
+  if (MODE == KMODE_POSES && R.pose_grid && unit >= R.pose_grid->n_blocks) break;
+
   // ---- item of this piece into shared memory, pair tables -----------------
   const int item = (MODE == KMODE_POSES) ? 0 : R.cta_item[unit];
   if (item != s_ctl->item) {
     // one read of the descriptor (it may live in pinned host memory), then
     // the shared-memory copy
-    const uint32_t *src = reinterpret_cast<const uint32_t *>(&R.items[item]);
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(
+        MODE == KMODE_POSES ? &R.pose_item : &R.items[item]);
     uint32_t *dst = reinterpret_cast<uint32_t *>(s_item);
     for (int i = threadIdx.x; i < (int)(sizeof(KItem) / 4); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
@@ -991,8 +1018,13 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     rl = lane & (reps - 1);
     rep0 = unit * reps;
     n_act = min(reps, R.n_pose - rep0);
+    if (R.pose_grid) {
+      const int cell = R.pose_cell[unit];
+      n_act = min(32, R.cell_count[cell] - 32 * (unit - R.cell_first[cell]));
+    }
     prt_conf = R.prt_conf;
     lane_rep = rep0 + (rl < n_act ? rl : 0);
+    if (R.pose_grid) lane_rep = R.pose_order[lane_rep];
   } else if (R.group_major) {
     // whole exchange groups: lane = group offset * n_tmp + temperature slot
     const int nt = I.n_tmp, nl = I.n_lig_conf;
@@ -1232,7 +1264,22 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     }
 #pragma unroll
     for (int h = 0; h < NH; ++h) my_hpc2[h * 32] = make_float2(0.f, 0.f);
-    const Region G = warp_region<NA>(nx, ny, nz, rl < n_act ? n_my : 0);
+    // where the warp's atoms are: as placed; for poses in cells, the cell grown
+    // by the atoms' largest distance from the ligand's centre (any rotation)
+    Region G;
+    float reach = 0.f;
+    if (MODE != KMODE_POSES) {
+      G = warp_region<NA>(nx, ny, nz, rl < n_act ? n_my : 0);
+    } else {
+      G = pose_region(R, unit, lcx, lcy, lcz);
+#pragma unroll
+      for (int k = 0; k < NA; ++k)
+        if (k < n_my)
+          reach = fmaxf(reach, fmaf(at0[k].z, at0[k].z, fmaf(at0[k].y, at0[k].y,
+                                                             at0[k].x * at0[k].x)));
+      reach = sqrtf(reach) * 1.0001f + 1e-3f;
+      if (!(reach < 5.0e3f)) reach = 3.0e38f;  // also NaN: nothing is far
+    }
     double far_pmf = 0.0;  // PMF of this lane's far points (every lane's replica)
 
     // ---- pair terms over the protein tiles -----------------------------------
@@ -1284,7 +1331,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
         const float4 p_l = ta[valid ? jl : j0];
         const float b2_l = box_dist2(G, p_l);
-        const bool far_l = MODE != KMODE_POSES && valid && is_far(G, p_l, b2_l, my_far[pt_l]);
+        const bool far_l = valid && is_far(G, p_l, b2_l, my_far[pt_l] + reach);
         const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
         const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
         const uint32_t close_m =

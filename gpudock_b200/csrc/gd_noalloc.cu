@@ -1,33 +1,32 @@
 // gd_noalloc.cu -- pose energies without any device allocation.
 //
 // gd_energy_poses (host buffers) stages its poses, terms and raw sums, and the
-// launch's item descriptor, in memory it obtains from cudaMallocAsync for each
+// workspace of a large call, in memory it obtains from cudaMallocAsync for each
 // call. gd_energy_poses_noalloc computes the same thing with the same kernel
 // but stages everything in one fixed file-scope device array, so it never
 // calls an allocator. The array is sized for GD_NOALLOC_MAX_POSES poses per
 // call; larger calls are rejected before anything is launched.
 //
 // Scratch layout (each section starts on a 256-byte boundary):
-//   [KItem descriptor][poses  max x 6 f32][terms  max x 10 f32][raw  max x 9 f64]
-// Every byte the kernel reads from it (descriptor, poses) is written by the
-// call before the launch, and the kernel writes every terms/raw element of the
-// n_pose poses it is given, so nothing in it has to start at zero.
+//   [poses  max x 6 f32][terms  max x 10 f32][raw  max x 9 f64][cells of the poses]
+// Every byte the kernels read from it is written by the call before, and they
+// write every terms/raw element of the n_pose poses, so nothing in it has to
+// start at zero.
 #include <cstring>
 
 #include "gd_common.h"
 
 namespace {
 
-using gd::KItem;
-using gd::KRun;
-
 constexpr size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
-constexpr size_t kItemBytes = align256(sizeof(KItem));
 constexpr size_t kPoseBytes = align256(sizeof(float) * 6 * GD_NOALLOC_MAX_POSES);
 constexpr size_t kTermBytes = align256(sizeof(float) * GD_NTERM * GD_NOALLOC_MAX_POSES);
 constexpr size_t kRawBytes = align256(sizeof(double) * GD_NRAW * GD_NOALLOC_MAX_POSES);
-constexpr size_t kScratchBytes = kItemBytes + kPoseBytes + kTermBytes + kRawBytes;
+// pose_work_bytes of the largest call: 8 bytes a pose, 132 a block of 32 poses
+// (up to one more per 320 poses) and its small arrays
+constexpr size_t kWorkBytes = align256(16 * GD_NOALLOC_MAX_POSES + 16384);
+constexpr size_t kScratchBytes = kPoseBytes + kTermBytes + kRawBytes + kWorkBytes;
 static_assert(kScratchBytes < (3u << 20), "pose scratch is meant to stay a few MB");
 
 // One copy per device (each device's context has its own instance).
@@ -72,37 +71,16 @@ extern "C" gd_status gd_energy_poses_noalloc(gd_ctx *ctx, const gd_dcomplex *d, 
   unsigned char *base = ctx->noalloc_scratch;
   if (!base) return gd::fail(GD_EINVAL, "gd_energy_poses_noalloc: context has no scratch address");
   GD_CUDA(cudaSetDevice(ctx->device));
-  KItem *d_item = reinterpret_cast<KItem *>(base);
-  float *d_poses = reinterpret_cast<float *>(base + kItemBytes);
-  float *d_terms = reinterpret_cast<float *>(base + kItemBytes + kPoseBytes);
-  double *d_raw = reinterpret_cast<double *>(base + kItemBytes + kPoseBytes + kTermBytes);
-
-  const gd::Tile tile = gd::tile_for(ctx, d->T);
-  KRun R{};
-  R.mode = gd::KMODE_POSES;
-  R.A = tile.A;
-  R.P = tile.P;
-  gd::pick_stages(d->T, tile, &R.n_stages, &R.resident);
-  R.prt_conf = prt_conf;
-  R.lig_conf = lig_conf;
-  R.n_pose = n_pose;
-  R.poses = d_poses;
-  R.terms = d_terms;
-  R.raw = raw ? d_raw : nullptr;
-  R.err = ctx->d_err;
-  R.hb_pairs = gd::hb_pairs_of(d->T, tile.A);
-  R.items = d_item;
-  KItem it{};
-  it.T = d->T;
-  it.n_tmp = 1;
-  it.n_lig_conf = d->T.n_lig;
-  it.n_prt = d->T.n_prt;
-
+  float *d_poses = reinterpret_cast<float *>(base);
+  float *d_terms = reinterpret_cast<float *>(base + kPoseBytes);
+  double *d_raw = reinterpret_cast<double *>(base + kPoseBytes + kTermBytes);
+  const size_t work = gd::pose_work_bytes(d->T, n_pose);
+  if (work > kWorkBytes) return gd::fail(GD_EINVAL, "internal: pose workspace of %zu bytes", work);
   const size_t pose_b = sizeof(float) * 6 * (size_t)n_pose;
-  GD_CUDA(cudaMemcpyAsync(d_item, &it, sizeof(KItem), cudaMemcpyHostToDevice, ctx->stream));
   GD_CUDA(cudaMemcpyAsync(d_poses, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream));
-  GD_CUDA(gd::launch_dock(R, tile.NA, (n_pose + 31) / 32, ctx->stream));
-  ctx->launches += 1;
+  GD_TRY(gd::poses_launch(ctx, d, prt_conf, lig_conf, n_pose, d_poses, d_terms,
+                          raw ? d_raw : nullptr,
+                          work ? base + kPoseBytes + kTermBytes + kRawBytes : nullptr));
   cudaError_t e = cudaMemcpyAsync(terms, d_terms, sizeof(float) * GD_NTERM * (size_t)n_pose,
                                   cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess && raw)

@@ -1,0 +1,219 @@
+// gd_poses.cu -- the poses of a large energy call dealt into cells of their
+// translation, so that a CTA's 32 poses lie close together and most protein
+// points are far of all of them (the far form of the pair terms,
+// gd_kernels.cu).
+//
+// Which points take the far form follows from the cell alone, never from the
+// other poses of the CTA, and the cells from the box of the call's
+// translations: a pose's energy does not depend on the order of the poses.
+// Poses without a usable translation (not finite, or beyond kFarOut) get a
+// cell of their own, for which no point is far.
+//
+// Four short launches (about 10 us together): the box of the translations;
+// every pose's cell and its rank in it; the cells' first 32-pose blocks; the
+// poses in block order.
+#include <algorithm>
+
+#include "gd_common.h"
+
+namespace gd {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kMaxCells = 4096;
+constexpr float kFarOut = 4.0e3f;
+// Poses per cell: a cell's last block is half empty on average, so about 5% of
+// the blocks' lanes are idle.
+constexpr int kPosesPerCell = 320;
+constexpr float kMinEdge = 0.75f;  // smaller cells gain little (the ligand is larger)
+
+int max_cells(int n_pose) { return std::max(1, std::min(kMaxCells, n_pose / kPosesPerCell)); }
+int max_blocks(int n_pose) { return (n_pose + 31) / 32 + max_cells(n_pose) + 1; }
+
+// Workspace of a call (see pose_work_bytes).
+struct Work {
+  unsigned *box;    // [6] largest ordered(-t), ordered(t) per axis, 0: none
+  PoseGrid *grid;
+  int *count;       // [max_cells + 1] poses of each cell
+  int *first;       // [max_cells + 1] its first block
+  int2 *at;         // [n] {cell, rank}
+  int *order;       // [max_blocks * 32]
+  int *block_cell;  // [max_blocks]
+  size_t zero, total;
+};
+
+Work layout(unsigned char *p, int n) {
+  Work w{};
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    unsigned char *q = p + o;
+    o += (bytes + 255) & ~size_t(255);
+    return q;
+  };
+  w.box = (unsigned *)take(6 * sizeof(unsigned));
+  w.count = (int *)take((max_cells(n) + 1) * sizeof(int));
+  w.zero = o;  // up to here the call starts from zeros
+  w.grid = (PoseGrid *)take(sizeof(PoseGrid));
+  w.first = (int *)take((max_cells(n) + 1) * sizeof(int));
+  w.at = (int2 *)take((size_t)n * sizeof(int2));
+  w.order = (int *)take((size_t)max_blocks(n) * 32 * sizeof(int));
+  w.block_cell = (int *)take((size_t)max_blocks(n) * sizeof(int));
+  w.total = o;
+  return w;
+}
+
+// Unsigned integers in the order of the floats; 0 is below every one.
+__device__ __forceinline__ unsigned ordered(float x) {
+  const unsigned u = __float_as_uint(x);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float unordered(unsigned u) {
+  return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
+}
+
+__device__ __forceinline__ bool usable(const float t[3]) {
+  return fabsf(t[0]) < kFarOut && fabsf(t[1]) < kFarOut && fabsf(t[2]) < kFarOut;
+}
+
+__global__ void __launch_bounds__(kThreads) box_kernel(const float *poses, int n, unsigned *box) {
+  unsigned m[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
+    const float t[3] = {poses[(size_t)i * 6], poses[(size_t)i * 6 + 1], poses[(size_t)i * 6 + 2]};
+    if (!usable(t)) continue;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      m[k] = max(m[k], ordered(-t[k]));
+      m[3 + k] = max(m[3 + k], ordered(t[k]));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+    if ((threadIdx.x & 31) == 0 && m[k] != 0u) atomicMax(&box[k], m[k]);
+  }
+}
+
+// The grid over the box: the smallest edge (from kMinEdge on, in steps of
+// 10%) that needs at most max_cells cells.
+__device__ PoseGrid make_grid(const unsigned *box, int max_cells) {
+  PoseGrid g;
+  float range[3] = {0.f, 0.f, 0.f};
+  float most = 0.f;
+  for (int k = 0; k < 3; ++k) {
+    g.lo[k] = box[k] ? -unordered(box[k]) : 0.f;
+    range[k] = box[3 + k] ? unordered(box[3 + k]) - g.lo[k] : 0.f;
+    most = fmaxf(most, range[k]);
+  }
+  g.edge = kMinEdge;
+  for (;;) {
+    double cells = 1.0;
+    for (int k = 0; k < 3; ++k) {
+      g.n[k] = max(1, (int)ceilf(range[k] / g.edge));
+      cells *= g.n[k];
+    }
+    if (cells <= (double)max_cells) break;
+    g.edge *= 1.1f;
+  }
+  g.inv_edge = 1.0f / g.edge;
+  g.n_cells = g.n[0] * g.n[1] * g.n[2];
+  // how far past its cell's walls rounding can leave a pose
+  g.margin = 1e-3f + 1e-5f * most;
+  g.n_blocks = 0;
+  return g;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    cell_kernel(const float *poses, int n, int max_cells, const unsigned *box, PoseGrid *grid,
+                int *count, int2 *at) {
+  __shared__ PoseGrid g;
+  if (threadIdx.x == 0) {
+    g = make_grid(box, max_cells);
+    if (blockIdx.x == 0) *grid = g;
+  }
+  __syncthreads();
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= n) return;
+  const float t[3] = {poses[(size_t)i * 6], poses[(size_t)i * 6 + 1], poses[(size_t)i * 6 + 2]};
+  int cell = g.n_cells;  // no usable translation
+  if (usable(t)) {
+    int c[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      c[k] = min(g.n[k] - 1, max(0, (int)((t[k] - g.lo[k]) * g.inv_edge)));
+    cell = (c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
+  }
+  at[i] = make_int2(cell, atomicAdd(&count[cell], 1));
+}
+
+// Exclusive scan of the cells' block counts (one block).
+__global__ void __launch_bounds__(1024) scan_kernel(PoseGrid *grid, const int *count, int *first) {
+  __shared__ int warp_sum[32];
+  const int n = grid->n_cells + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (int c0 = 0; c0 < n; c0 += 1024) {
+    const int c = c0 + threadIdx.x;
+    const int b = c < n ? (count[c] + 31) / 32 : 0;
+    int s = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += x;
+    }
+    if (lane == 31) warp_sum[warp] = s;
+    __syncthreads();
+    if (warp == 0) {
+      int v = warp_sum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += x;
+      }
+      warp_sum[lane] = v;
+    }
+    __syncthreads();
+    if (c < n) first[c] = base + (warp ? warp_sum[warp - 1] : 0) + s - b;
+    base += warp_sum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) grid->n_blocks = base;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    order_kernel(int n, const int2 *at, const int *first, int *order, int *block_cell) {
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= n) return;
+  const int2 a = at[i];
+  const int b = first[a.x] + a.y / 32;
+  order[b * 32 + a.y % 32] = i;
+  if (a.y % 32 == 0) block_cell[b] = a.x;
+}
+
+}  // namespace
+
+size_t pose_work_bytes(const KTables &T, int n_pose) {
+  // Cells pay once their launches are a small part of the call (1e12 pairs/s):
+  // about 3% at 5e8 pairs.
+  if (n_pose < 4096 || (double)n_pose * T.lna * T.pnp < 5e8) return 0;
+  return layout(nullptr, n_pose).total;
+}
+
+cudaError_t pose_cells(KRun *R, void *work, int *grid, cudaStream_t s) {
+  const int n = R->n_pose, cells = max_cells(n);
+  const Work w = layout(static_cast<unsigned char *>(work), n);
+  cudaError_t e = cudaMemsetAsync(work, 0, w.zero, s);
+  if (e != cudaSuccess) return e;
+  const int blocks = (n + kThreads - 1) / kThreads;
+  box_kernel<<<std::min(blocks, 148 * 4), kThreads, 0, s>>>(R->poses, n, w.box);
+  cell_kernel<<<blocks, kThreads, 0, s>>>(R->poses, n, cells, w.box, w.grid, w.count, w.at);
+  scan_kernel<<<1, 1024, 0, s>>>(w.grid, w.count, w.first);
+  order_kernel<<<blocks, kThreads, 0, s>>>(n, w.at, w.first, w.order, w.block_cell);
+  R->pose_grid = w.grid;
+  R->pose_order = w.order;
+  R->pose_cell = w.block_cell;
+  R->cell_first = w.first;
+  R->cell_count = w.count;
+  *grid = max_blocks(n);
+  return cudaGetLastError();
+}
+
+}  // namespace gd
