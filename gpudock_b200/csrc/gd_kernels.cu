@@ -41,13 +41,19 @@ namespace gd {
 
 constexpr int STAGE_BYTES = TILE_PTS * (16 + 8);
 constexpr int CHUNK = 32;  // points per FP32 partial before the FP64 flush
-// Protein points per iteration of the pair loops: two overlap their chains
-// where a warp holds few atom pairs.  With more, one: a warp alternates
-// between the near and the far loop of every chunk, and bodies of two points
-// no longer fit the instruction caches together (headline interval with NH =
-// 5: 26.2 ms with two points in both loops, 23.4 with one in the far loop,
-// 22.4 with one in both; ncu's no-instruction stall 0.87 / 0.37 / 0.17).
-__host__ __device__ constexpr int point_unroll(int NH) { return NH <= 2 ? 2 : 1; }
+// Protein points per iteration of the pair loops.  Two overlap their chains,
+// but a warp alternates between the near and the far loop of every chunk, and
+// both bodies have to stay in the instruction caches: the near loop takes two
+// up to two atom pairs, the shorter far loop up to four (packed lanes have few
+// points per loop).  Near / far points per iteration, NH = 4: 131,072 poses x 48
+// x 2,000 in 13.0 (1 / 1), 12.8 (1 / 2), 13.4 (2 / 1), 13.9 ms (2 / 2); 65,536 x
+// 48 x 16,000 in 36.7, 34.4, 35.5, 34.1 ms.  NH = 5, headline interval: 22.4 (1
+// / 1), 23.4 (2 / 1), 26.2 ms (2 / 2; ncu's no-instruction stall 0.17, 0.37,
+// 0.87 per issue).
+__host__ __device__ constexpr int near_unroll(int NH) { return NH <= 2 ? 2 : 1; }
+__host__ __device__ constexpr int far_unroll(int NH, bool packed) {
+  return NH <= 2 || (NH <= 4 && !packed) ? 2 : 1;
+}
 constexpr float LOG2E = 1.4426950408889634f;
 // coordinate of the padding atoms: far from every point, and close enough
 // that d^9 to any point stays finite in FP32
@@ -561,7 +567,7 @@ __device__ __forceinline__ uint32_t chunk_fast(const float2 (&nx)[NH], const flo
   uint2 e = list[0], en = list[subs];
   list += 2 * subs;
   float4 Ap = entry_point(smem, e.x);
-#pragma unroll point_unroll(NH)
+#pragma unroll near_unroll(NH)
   for (int k = 0; k < n; ++k) {
     const float4 An = entry_point(smem, en.x);
     const uint2 e2 = *list;
@@ -598,7 +604,7 @@ __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (
   uint32_t e = list[0].x, en = list[subs].x;
   list += 2 * subs;
   float4 Ap = entry_point(smem, e);
-#pragma unroll point_unroll(NH)
+#pragma unroll far_unroll(NH, PACKED)
   for (int k = 0; k < n; ++k) {
     const float4 An = entry_point(smem, en);
     const uint32_t e2 = list->x;
