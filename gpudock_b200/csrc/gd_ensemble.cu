@@ -186,6 +186,42 @@ void ens_free(Ens &E) {
   E.ctx = nullptr;
 }
 
+// CTAs per unit of each complex of a run.  A run with fewer units than SMs ends
+// with its costliest unit, so the unit with the most work per CTA is split
+// further first, while its CTAs still have kRunSplitCost pairs each and the
+// run's CTAs fit on the GPU at once (a screen of 24 ligands of 12 .. 96 atoms
+// against 6,000 points: 8 CTAs for the largest, 2 for the smallest, 148 in
+// all, where the same split for all was 4).  A complex whose run has room
+// for every unit's own most gets that, as alone.
+std::vector<int> run_splits(gd_ctx *ctx, const std::vector<KItem> &items) {
+  const size_t n = items.size();
+  std::vector<int> split(n, 1), units(n), most(n);
+  long long ctas = 0;
+  for (size_t i = 0; i < n; ++i) {
+    units[i] = units_of(items[i].n_prt, items[i].n_lig_conf, items[i].n_tmp);
+    most[i] = split_for(ctx, items[i].T, 1, kRunSplitCost);
+    ctas += units[i];
+  }
+  if (ctx->split_mode > 0) return most;
+  // (cost per CTA, item), costliest first
+  std::vector<std::pair<double, int>> heap;
+  auto cost = [&](int i) { return (double)lna_bucket(items[i].T.lna) * items[i].T.pnp / split[i]; };
+  for (size_t i = 0; i < n; ++i) heap.emplace_back(cost((int)i), -(int)i);
+  std::make_heap(heap.begin(), heap.end());
+  while (!heap.empty()) {
+    std::pop_heap(heap.begin(), heap.end());
+    const int i = -heap.back().second;
+    heap.pop_back();
+    const long long more = (long long)units[i] * split[i];
+    if (2 * split[i] > most[i] || ctas + more > ctx->n_sm) continue;
+    split[i] *= 2;
+    ctas += more;
+    heap.emplace_back(cost(i), -i);
+    std::push_heap(heap.begin(), heap.end());
+  }
+  return split;
+}
+
 gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
                     const gd_mc_params *mc) {
   E.ctx = ctx;
@@ -263,12 +299,11 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
   std::map<Key, std::vector<std::tuple<double, int, int, int>>> ctas;  // cost, item, rep0, n
   std::map<Key, Plan> plans;
   std::vector<KGroup> groups;
-  int run_units = 0;  // units of the whole run (the split rule's bound)
-  for (const KItem &I : E.items) run_units += units_of(I.n_prt, I.n_lig_conf, I.n_tmp);
+  const std::vector<int> splits = run_splits(ctx, E.items);
   for (int i = 0; i < n; ++i) {
     const KItem &I = E.items[i];
     Tile t = tile_for(ctx, I.T);
-    const int split = split_for(ctx, I.T, run_units, kRunSplitCost);
+    const int split = splits[i];
     int ns, res;
     pick_stages(I.T, t, &ns, &res, split);
     const int nt = I.n_tmp, nl = I.n_lig_conf;

@@ -61,3 +61,24 @@ def test_packed_streamed(ctx):
     out, mb = _run(ctx, d, 8, steps=(10,))
     ctx.set_split(0)
     _check_records(cx, out, mb)
+
+
+@pytest.mark.parametrize("n", [3, 21, 150])
+def test_batch_splits(ctx, n):
+    """A batch whose complexes get different numbers of CTAs per unit (all
+    their own most; the costliest more; one each): recorded states and
+    decisions of every complex."""
+    raw, _, _ = synth.default_ff()
+    prt = synth.make_protein(np.random.Generator(np.random.PCG64(93)),
+                             synth.ComplexSpec(pnp=1900, lna=8), 8.0, raw)
+    cxs = [synth.make_complex(synth.ComplexSpec(pnp=1900, lna=8 + (i * 88) // n, n_lig=1 + i % 4),
+                              seed=94 + i, protein=prt) for i in range(n)]
+    _, mb = lib.set_temperature(8, 0.004, 0.04)
+    base = lib.DeviceComplex(ctx, cxs[0])
+    dcxs = [lib.DeviceComplex(ctx, cx, share=base) for cx in cxs]
+    b = lib.Batch(ctx, dcxs, [abi.mc_params(10, 10, mb, seed=12, flags=FLAGS) for _ in cxs])
+    b.init()
+    b.run(10)
+    for i in range(0, n, max(1, n // 12)):
+        _check_records(cxs[i], b.read(i), mb, steps=(0,))
+    b.close()
