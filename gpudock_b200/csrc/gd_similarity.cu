@@ -7,20 +7,24 @@
 // against conformation i's contact map, where a contact is a ligand-atom /
 // protein-point pair with dst <= pmf0[ligand type][point type].  With A and
 // B the two maps: tp = |A & B|, fn = |A| - tp, fp = |B| - tp and tn = the
-// remaining pairs, so the matrix is a popcount "product" of bit maps:
-//   contacts  one CTA per conformation places its ligand and writes its map,
-//             32 protein points per word (a warp ballot), with its count;
-//   union     the OR of all maps word by word: words that no conformation
-//             sets are dropped (the maps of a trajectory near one pocket are
-//             sparse and overlap);
-//   gather    the kept words of every map, contiguous;
-//   pairs     64 x 64 tiles of (i, j): popc(A & B) summed over the kept words
-//             through shared memory, then the MCC from the four counts.
+// remaining pairs, so the matrix is a popcount "product" of bit maps.  The
+// maps of a trajectory near one pocket are sparse and overlap: a few percent
+// of the pairs are a contact of some conformation, and only those get a bit:
+//   contacts  one CTA per conformation places its ligand and tests its atoms
+//             against the points near the ligand's box; the contacts go into
+//             the union of all maps, their number is kept;
+//   rank      the number of union bits below each word of the union;
+//   maps      the contacts again, now as bits numbered by their rank;
+//   pairs     64 x 64 tiles of (i, j), i <= j: popc(A & B) over the maps'
+//             words through shared memory, then both entries' MCC.
 // Placement and distances follow the reference's float operations in its
 // order (no contraction): the rotation comes from the host (PlaceLigand runs
 // on the host in the reference, with sinf / cosf), x = r0 x + r1 y + r2 z +
 // m + centre and dst = sqrtf(dx dx + dy dy + dz dz), so every contact and
-// every entry is the reference's bit for bit.
+// every entry is the reference's bit for bit.  The test itself is on the
+// squared distance: the correctly rounded root never falls as its argument
+// grows, so dst <= pmf0 holds exactly up to the largest float whose root is at
+// most pmf0 (contact_bound).
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -43,13 +47,56 @@ constexpr int kSimThreads = 256;
 constexpr int kPairTile = 64;   // conformations per tile side
 constexpr int kPairChunk = 32;  // words per shared-memory chunk
 
+constexpr int kCandidates = 2048;  // points looked at per round
+constexpr int kRowWords = 8192;    // largest map kept in shared memory
+
+// The largest float whose correctly rounded square root is at most p (-1:
+// none).
+__device__ __forceinline__ float contact_bound(float p) {
+  if (!(p >= 0.f)) return -1.f;
+  if (__float_as_uint(p) >= 0x7f800000u) return p;  // infinity
+  // p^2 is within a few units in the last place of it
+  uint32_t b = __float_as_uint(__fmul_rn(p, p));
+  while (b < 0x7f800000u && __fsqrt_rn(__uint_as_float(b)) <= p) ++b;
+  while (b > 0u && !(__fsqrt_rn(__uint_as_float(b)) <= p)) --b;
+  return __uint_as_float(b);
+}
+
+__global__ void bound_kernel(const float4 *tab, float *bound) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // [GD_NLT][32]
+  if (i >= GD_NLT * 32) return;
+  const int lt = i / 32, pt = i % 32;
+  bound[i] = pt < GD_NPT ? contact_bound(tab[lt * GD_NPT + pt].z) : -1.f;
+}
+
+// Contacts of conformation blockIdx.x.  MAPS = false: into the union's bits
+// (contact l * pnp + s of atom l and point s), and their number.  MAPS = true:
+// as the conformation's map of Kp words, bits numbered by the contact's rank
+// in the union.  Bound by latency and L2 reads of the points: the atoms are
+// tested against the few points within reach of the ligand's box (600
+// conformations x 40 x 4,000: 27 us a pass; testing every pair took 227 us).
+// The second pass costs less than keeping every conformation's contacts.
+template <bool MAPS>
 __global__ void __launch_bounds__(kSimThreads)
-    contacts_kernel(KTables T, const SimConf *confs, uint32_t *bits, int *pop, int W) {
-  extern __shared__ float4 s_lig[];  // placed atoms, ligand type in .w
-  __shared__ int s_pop;
+    contacts_kernel(KTables T, const SimConf *confs, const float *bound, uint32_t *uni, int *pop,
+                    const int *base, uint32_t *maps, int Kp) {
+  extern __shared__ float4 s_lig[];  // placed atoms, ligand type in .w; the map's words
+  uint32_t *s_row = reinterpret_cast<uint32_t *>(s_lig + T.lna);
+  __shared__ float s_bound[GD_NLT * 32];
+  __shared__ uint16_t s_cand[kCandidates];
+  __shared__ int s_n, s_pop;
+  __shared__ unsigned s_box[6];  // largest ordered(-x), ordered(x) per axis
   const SimConf c = confs[blockIdx.x];
-  const int lna = T.lna;
-  for (int l = threadIdx.x; l < lna; l += blockDim.x) {
+  const int lna = T.lna, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool row = MAPS && Kp <= kRowWords;
+  uint32_t *out = MAPS ? maps + (size_t)blockIdx.x * Kp : nullptr;
+  for (int i = threadIdx.x; i < GD_NLT * 32; i += kSimThreads) s_bound[i] = bound[i];
+  if (row)
+    for (int i = threadIdx.x; i < Kp; i += kSimThreads) s_row[i] = 0u;
+  if (threadIdx.x < 6) s_box[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) s_n = s_pop = 0;
+  __syncthreads();
+  for (int l = threadIdx.x; l < lna; l += kSimThreads) {
     const float4 o = T.lig[(size_t)c.lig * lna + l];
     float v[3];
 #pragma unroll
@@ -59,57 +106,118 @@ __global__ void __launch_bounds__(kSimThreads)
       a = __fadd_rn(a, __fmul_rn(c.r[3 * k + 2], o.z));
       a = __fadd_rn(a, c.m[k]);
       v[k] = __fadd_rn(a, T.lig_center[k]);
+      if (v[k] == v[k]) {  // an atom without a position has no contact
+        const unsigned u = __float_as_uint(v[k]), w = __float_as_uint(-v[k]);
+        atomicMax(&s_box[k], w & 0x80000000u ? ~w : w | 0x80000000u);
+        atomicMax(&s_box[3 + k], u & 0x80000000u ? ~u : u | 0x80000000u);
+      }
     }
     s_lig[l] = make_float4(v[0], v[1], v[2], __int_as_float(T.lig_t[l]));
   }
-  if (threadIdx.x == 0) s_pop = 0;
   __syncthreads();
+  float lo[3], hi[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const unsigned a = s_box[k], b = s_box[3 + k];
+    lo[k] = -__uint_as_float(a & 0x80000000u ? a & 0x7fffffffu : ~a);
+    hi[k] = __uint_as_float(b & 0x80000000u ? b & 0x7fffffffu : ~b);
+  }
   const float4 *P = T.pt_a + (size_t)c.prt * T.pnp_pad;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t K = (size_t)lna * W;
-  uint32_t *out = bits + (size_t)blockIdx.x * K;
   int my_pop = 0;
-  // a warp takes 32 points (one word column) against every atom
-  for (int w = warp; w < W; w += kSimThreads / 32) {
-    const int s = w * 32 + lane;
-    const bool valid = s < T.pnp;
-    const float4 p = valid ? P[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int pt = valid ? (int)(__float_as_uint(T.pt_b[s].y) & META_TYPE_MASK) : 0;
-    for (int l = 0; l < lna; ++l) {
-      const float4 a = s_lig[l];
-      const float dx = __fsub_rn(a.x, p.x);
-      const float dy = __fsub_rn(a.y, p.y);
-      const float dz = __fsub_rn(a.z, p.z);
-      const float d2 =
-          __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-      const float pmf0 = T.tab_a[__float_as_int(a.w) * GD_NPT + pt].z;
-      const bool hit = valid && __fsqrt_rn(d2) <= pmf0;
-      const uint32_t word = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) {
-        out[(size_t)l * W + w] = word;
-        my_pop += __popc(word);
+  for (int s0 = 0; s0 < T.pnp; s0 += kCandidates) {
+    const int s1 = min(T.pnp, s0 + kCandidates);
+    // points within reach (near_mcc2: the largest pmf0 squared, with margin)
+    for (int i = s0 + warp * 32; i < s1; i += kSimThreads) {
+      const int s = i + lane;
+      bool near = false;
+      if (s < s1) {
+        const float4 p = P[s];
+        const float bx = fmaxf(fmaxf(lo[0] - p.x, p.x - hi[0]), 0.f);
+        const float by = fmaxf(fmaxf(lo[1] - p.y, p.y - hi[1]), 0.f);
+        const float bz = fmaxf(fmaxf(lo[2] - p.z, p.z - hi[2]), 0.f);
+        near = fmaf(bz, bz, fmaf(by, by, bx * bx)) <= T.near_mcc2;
+      }
+      const uint32_t m = __ballot_sync(0xffffffffu, near);
+      int at = 0;
+      if (lane == 0 && m) at = atomicAdd(&s_n, __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (near) s_cand[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(s - s0);
+    }
+    __syncthreads();
+    // a warp takes a point against 32 atoms at a time
+    const int n = s_n;
+    for (int q = warp; q < n; q += kSimThreads / 32) {
+      const int s = s0 + s_cand[q];
+      const float4 p = P[s];
+      const int pt = (int)(__float_as_uint(T.pt_b[s].y) & META_TYPE_MASK);
+      for (int l = lane; l < lna; l += 32) {
+        const float4 a = s_lig[l];
+        const float dx = __fsub_rn(a.x, p.x);
+        const float dy = __fsub_rn(a.y, p.y);
+        const float dz = __fsub_rn(a.z, p.z);
+        const float d2 =
+            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+        if (!(d2 <= s_bound[__float_as_int(a.w) * 32 + pt])) continue;
+        const size_t id = (size_t)l * T.pnp + s;
+        const uint32_t bit = 1u << (id & 31);
+        if (!MAPS) {
+          ++my_pop;
+          // most contacts are in the union already
+          if (!(__ldcg(&uni[id >> 5]) & bit)) atomicOr(&uni[id >> 5], bit);
+        } else {
+          const int r = base[id >> 5] + __popc(uni[id >> 5] & (bit - 1u));
+          if (row)
+            atomicOr(&s_row[r >> 5], 1u << (r & 31));
+          else
+            atomicOr(&out[r >> 5], 1u << (r & 31));
+        }
       }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
   }
-  if (lane == 0) atomicAdd(&s_pop, my_pop);
-  __syncthreads();
-  if (threadIdx.x == 0) pop[blockIdx.x] = s_pop;
+  if (!MAPS) {
+    my_pop = __reduce_add_sync(0xffffffffu, my_pop);
+    if (lane == 0 && my_pop) atomicAdd(&s_pop, my_pop);
+    __syncthreads();
+    if (threadIdx.x == 0) pop[blockIdx.x] = s_pop;
+  } else if (row) {
+    for (int i = threadIdx.x; i < Kp; i += kSimThreads) out[i] = s_row[i];
+  }
 }
 
-__global__ void union_kernel(const uint32_t *bits, int n, size_t K, uint32_t *mask) {
-  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
-  uint32_t m = 0u;
-  for (int i = 0; i < n; ++i) m |= bits[(size_t)i * K + k];
-  mask[k] = m;
-}
-
-__global__ void gather_kernel(const uint32_t *bits, int n, size_t K, const int *act, int n_act,
-                              int Kp, uint32_t *comp) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n * Kp) return;
-  const int i = (int)(t / Kp), a = (int)(t % Kp);
-  comp[t] = a < n_act ? bits[(size_t)i * K + act[a]] : 0u;
+// base[w] = number of union bits below word w, base[K] = all (one block).
+__global__ void __launch_bounds__(1024) rank_kernel(const uint32_t *uni, int K, int *base) {
+  __shared__ int s_sum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int k0 = 0; k0 < K; k0 += 1024) {
+    const int k = k0 + threadIdx.x;
+    const int b = k < K ? __popc(uni[k]) : 0;
+    int v = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += x;
+    }
+    if (lane == 31) s_sum[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+      int t = s_sum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += x;
+      }
+      s_sum[lane] = t;
+    }
+    __syncthreads();
+    if (k < K) base[k] = before + (warp ? s_sum[warp - 1] : 0) + v - b;
+    before += s_sum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) base[K] = before;
 }
 
 // CalculateContactModeScore's arithmetic: the four sums as floats multiplied
@@ -124,11 +232,32 @@ __device__ __forceinline__ float contact_mcc(int tp, int fn, int fp, int tn) {
   return dividend != 0.0f ? __fdiv_rn(__int2float_rn(num), dividend) : GD_CMCC_INVALID;
 }
 
+// Entries of the matrix.  With a bit per contact of the union, in place of the
+// 32-bit words that hold one, the maps are several times shorter: 600
+// conformations 145 -> 17 us, 3,001 (upper triangle only) 9.3 -> 0.66 ms for the
+// whole call.  Bound by the ALU pipe (carry-save counting).
+// Tile pair t of the upper triangle of tiles x tiles: its row and column.
+__device__ __forceinline__ void tile_of(int t, int tiles, int *row, int *col) {
+  // row r starts at r tiles - r (r - 1) / 2
+  int r = (int)((2.0f * tiles + 1.0f -
+                 sqrtf(fmaxf(0.f, (2.0f * tiles + 1.0f) * (2.0f * tiles + 1.0f) - 8.0f * t))) *
+                0.5f);
+  auto start = [&](int x) { return (long long)x * tiles - (long long)x * (x - 1) / 2; };
+  while (r > 0 && start(r) > t) --r;
+  while (start(r + 1) <= t) ++r;
+  *row = r;
+  *col = r + (int)(t - start(r));
+}
+
 __global__ void __launch_bounds__(kSimThreads)
-    pairs_kernel(const uint32_t *comp, const int *pop, int n, int Kp, int total, float *S) {
-  __shared__ uint32_t sa[kPairTile][kPairChunk + 1];
-  __shared__ uint32_t sb[kPairTile][kPairChunk + 1];
-  const int i0 = blockIdx.y * kPairTile, j0 = blockIdx.x * kPairTile;
+    pairs_kernel(const uint32_t *comp, const int *pop, int n, int Kp, int total, int tiles,
+                 float *S) {
+  __shared__ uint32_t s_mem[2 * kPairTile * (kPairChunk + 1)];
+  uint32_t(*sa)[kPairChunk + 1] = reinterpret_cast<uint32_t(*)[kPairChunk + 1]>(s_mem);
+  uint32_t(*sb)[kPairChunk + 1] = sa + kPairTile;
+  int ti, tj;
+  tile_of(blockIdx.x, tiles, &ti, &tj);
+  const int i0 = ti * kPairTile, j0 = tj * kPairTile;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   // Carry-save counting (Harley and Seal; Mula, Kurz and Lemire, "Faster
   // population counts using AVX2 instructions", 2018): the AND words of an
@@ -184,17 +313,27 @@ __global__ void __launch_bounds__(kSimThreads)
 #pragma unroll
     for (int c = 0; c < 4; ++c)
       acc[r][c] = 4 * acc[r][c] + 2 * __popc(twos[r][c]) + __popc(ones[r][c]);
+  // the tile's counts through shared memory (its words have been read), so
+  // that both (i, j) and (j, i) are written along rows
+  int *s_tp = reinterpret_cast<int *>(s_mem);  // [kPairTile][kPairTile + 1]
+  static_assert(kPairTile * (kPairTile + 1) <= 2 * kPairTile * (kPairChunk + 1), "count tile");
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + 16 * r;
-    if (i >= n) continue;
+  for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int j = j0 + tx + 16 * c;
-      if (j >= n) continue;
-      const int tp = acc[r][c];
-      const int fn = pop[i] - tp, fp = pop[j] - tp;
-      S[(size_t)i * n + j] = contact_mcc(tp, fn, fp, total - tp - fn - fp);
+    for (int c = 0; c < 4; ++c)
+      s_tp[(ty + 16 * r) * (kPairTile + 1) + tx + 16 * c] = acc[r][c];
+  __syncthreads();
+  for (int q = tid; q < kPairTile * kPairTile; q += kSimThreads) {
+    const int r = q / kPairTile, c = q % kPairTile;
+    if (i0 + r < n && j0 + c < n) {
+      const int tp = s_tp[r * (kPairTile + 1) + c];
+      const int fn = pop[i0 + r] - tp, fp = pop[j0 + c] - tp;
+      S[(size_t)(i0 + r) * n + j0 + c] = contact_mcc(tp, fn, fp, total - tp - fn - fp);
+    }
+    if (ti != tj && j0 + r < n && i0 + c < n) {
+      const int tp = s_tp[c * (kPairTile + 1) + r];
+      const int fn = pop[j0 + r] - tp, fp = pop[i0 + c] - tp;
+      S[(size_t)(j0 + r) * n + i0 + c] = contact_mcc(tp, fn, fp, total - tp - fn - fp);
     }
   }
 }
@@ -263,57 +402,53 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
   }
   GD_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  const int W = (T.pnp + 31) / 32;
-  const size_t K = (size_t)T.lna * W;
+  const size_t K = ((size_t)T.lna * T.pnp + 31) / 32;  // words of the union
   const int total = T.lna * T.pnp;
   const size_t n = (size_t)n_conf;
   gd_status st = GD_OK;
   {
     SimBuffers B{s, {}};
     SimConf *d_conf = nullptr;
-    uint32_t *d_bits = nullptr, *d_mask = nullptr;
-    int *d_pop = nullptr;
-    float *d_S = nullptr;
+    uint32_t *d_uni = nullptr, *d_maps = nullptr;
+    float *d_bound = nullptr, *d_S = nullptr;
+    int *d_pop = nullptr, *d_base = nullptr;
     cudaError_t e = B.get(&d_conf, n);
-    if (e == cudaSuccess) e = B.get(&d_bits, n * K);
+    if (e == cudaSuccess) e = B.get(&d_uni, K);
+    if (e == cudaSuccess) e = B.get(&d_bound, (size_t)GD_NLT * 32);
     if (e == cudaSuccess) e = B.get(&d_pop, n);
-    if (e == cudaSuccess) e = B.get(&d_mask, K);
+    if (e == cudaSuccess) e = B.get(&d_base, K + 1);
     if (e == cudaSuccess && !S_dev) e = B.get(&d_S, n * n);
     if (S_dev) d_S = S_dev;
     if (e != cudaSuccess) return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
     GD_CUDA(cudaMemcpyAsync(d_conf, hc.data(), sizeof(SimConf) * n, cudaMemcpyHostToDevice, s));
-    contacts_kernel<<<n_conf, kSimThreads, sizeof(float4) * T.lna, s>>>(T, d_conf, d_bits, d_pop,
-                                                                       W);
+    GD_CUDA(cudaMemsetAsync(d_uni, 0, sizeof(uint32_t) * K, s));
+    bound_kernel<<<(GD_NLT * 32 + 255) / 256, 256, 0, s>>>(T.tab_a, d_bound);
     GD_CUDA(cudaGetLastError());
-    union_kernel<<<(unsigned)((K + 255) / 256), 256, 0, s>>>(d_bits, n_conf, K, d_mask);
+    contacts_kernel<false><<<n_conf, kSimThreads, sizeof(float4) * T.lna, s>>>(
+        T, d_conf, d_bound, d_uni, d_pop, nullptr, nullptr, 0);
     GD_CUDA(cudaGetLastError());
-    std::vector<uint32_t> mask(K);
-    GD_CUDA(cudaMemcpyAsync(mask.data(), d_mask, sizeof(uint32_t) * K, cudaMemcpyDeviceToHost, s));
+    rank_kernel<<<1, 1024, 0, s>>>(d_uni, (int)K, d_base);
+    GD_CUDA(cudaGetLastError());
+    int n_bits = 0;
+    GD_CUDA(cudaMemcpyAsync(&n_bits, d_base + K, sizeof(int), cudaMemcpyDeviceToHost, s));
     GD_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> act;
-    for (size_t k = 0; k < K; ++k)
-      if (mask[k]) act.push_back((int)k);
-    const int n_act = (int)act.size();
-    const int Kp = (n_act + kPairChunk - 1) / kPairChunk * kPairChunk;
-    int *d_act = nullptr;
-    uint32_t *d_comp = nullptr;
-    e = B.get(&d_act, act.size());
-    if (e == cudaSuccess) e = B.get(&d_comp, n * (size_t)Kp);
-    if (e != cudaSuccess) return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
-    if (n_act)
-      GD_CUDA(cudaMemcpyAsync(d_act, act.data(), sizeof(int) * act.size(), cudaMemcpyHostToDevice,
-                              s));
+    const int Kp = (n_bits + 32 * kPairChunk - 1) / (32 * kPairChunk) * kPairChunk;
     if (Kp) {
-      const size_t cells = n * (size_t)Kp;
-      gather_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(d_bits, n_conf, K, d_act,
-                                                                     n_act, Kp, d_comp);
+      e = B.get(&d_maps, n * (size_t)Kp);
+      if (e != cudaSuccess)
+        return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
+      const bool row = Kp <= kRowWords;
+      if (!row) GD_CUDA(cudaMemsetAsync(d_maps, 0, sizeof(uint32_t) * n * Kp, s));
+      contacts_kernel<true><<<n_conf, kSimThreads,
+                              sizeof(float4) * T.lna + (row ? sizeof(uint32_t) * Kp : 0), s>>>(
+          T, d_conf, d_bound, d_uni, d_pop, d_base, d_maps, Kp);
       GD_CUDA(cudaGetLastError());
     }
-    const unsigned tiles = (unsigned)((n + kPairTile - 1) / kPairTile);
-    pairs_kernel<<<dim3(tiles, tiles), kSimThreads, 0, s>>>(d_comp, d_pop, n_conf, Kp, total,
-                                                            d_S);
+    const int tiles = (n_conf + kPairTile - 1) / kPairTile;
+    pairs_kernel<<<(unsigned)((long long)tiles * (tiles + 1) / 2), kSimThreads, 0, s>>>(
+        d_maps, d_pop, n_conf, Kp, total, tiles, d_S);
     GD_CUDA(cudaGetLastError());
-    ctx->launches += Kp ? 4 : 3;
+    ctx->launches += Kp ? 5 : 4;
     if (!S_dev)
       GD_CUDA(cudaMemcpyAsync(S_host, d_S, sizeof(float) * n * n, cudaMemcpyDeviceToHost, s));
     st = ctx_check(ctx);
