@@ -169,7 +169,7 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
-  cudaFree(c->d_err);
+  cudaFreeHost(c->h_err);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -205,15 +205,11 @@ gd_status kernel_error(int code) {
 }
 
 gd_status ctx_check(gd_ctx *c) {
-  int h = 0;
-  GD_CUDA(cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   GD_CUDA(cudaStreamSynchronize(c->stream));
-  if (h != 0) {
-    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-    cudaStreamSynchronize(c->stream);
-    return kernel_error(h);
-  }
-  return GD_OK;
+  const int code = *(volatile int *)c->h_err;
+  if (code == 0) return GD_OK;
+  *(volatile int *)c->h_err = 0;
+  return kernel_error(code);
 }
 
 }  // namespace gd
@@ -406,18 +402,19 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
     }
     c->own_stream = true;
   }
-  e = cudaMalloc(&c->d_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(int));
+  e = cudaMallocHost((void **)&c->h_err, 256 + kStageBytes);
   if (e != cudaSuccess) {
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
-    return fail(GD_ENOMEM, "cudaMalloc error word: %s", cudaGetErrorString(e));
+    return fail(GD_ENOMEM, "pinned host memory: %s", cudaGetErrorString(e));
   }
+  std::memset(c->h_err, 0, 256);
+  c->stage = reinterpret_cast<unsigned char *>(c->h_err) + 256;
   // the fixed scratch of gd_energy_poses_noalloc is committed now, not on
   // that entry point's first call
   const gd_status st = noalloc_attach(c);
   if (st != GD_OK) {
-    cudaFree(c->d_err);
+    cudaFreeHost(c->h_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return st;
@@ -442,23 +439,38 @@ extern "C" uint64_t gd_ctx_launch_count(const gd_ctx *c) { return c ? c->launche
 // ---------------------------------------------------------------------------
 // Device layout of a complex
 // ---------------------------------------------------------------------------
-// Stream-ordered allocation on the context stream: neither this nor the
-// matching cudaFreeAsync in dcx_release synchronises the device, so a
-// server uploading and releasing requests never stalls the kernels of other
-// streams.
+// The tables of a complex, collected on the host and placed in one device
+// allocation by one copy (a request's upload: 18 allocations and copies of a
+// few hundred bytes to a few hundred KB took about 150 us).  Stream-ordered on
+// the context stream: neither this nor the matching cudaFreeAsync in dcx_release
+// synchronises the device, so a server uploading and releasing requests never
+// stalls the kernels of other streams.
+struct TableUpload {
+  gd_dcomplex *d;
+  std::vector<unsigned char> host;
+  std::vector<std::pair<const void **, size_t>> at;  // pointer to set, offset
+};
+
 template <typename T>
-static gd_status upload(gd_dcomplex *d, const std::vector<T> &h, const T **out) {
-  void *p = nullptr;
+static gd_status upload(TableUpload &U, const std::vector<T> &h, const T **out) {
   const size_t n = std::max<size_t>(h.size(), 1) * sizeof(T);
-  if (injected_alloc_failure(d->ctx))
+  if (injected_alloc_failure(U.d->ctx))
     return fail(GD_ENOMEM, "cudaMallocAsync of %zu bytes: out of memory (injected)", n);
-  GD_CUDA(cudaMallocAsync(&p, n, d->ctx->stream));
-  d->allocs.push_back(p);
-  d->bytes += n;
-  if (!h.empty())
-    GD_CUDA(cudaMemcpyAsync(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice,
-                            d->ctx->stream));
-  *out = (const T *)p;
+  const size_t o = (U.host.size() + 255) & ~size_t(255);
+  U.host.resize(o + n);
+  if (!h.empty()) std::memcpy(U.host.data() + o, h.data(), h.size() * sizeof(T));
+  U.at.emplace_back(reinterpret_cast<const void **>(out), o);
+  U.d->bytes += n;
+  return GD_OK;
+}
+
+static gd_status upload_finish(TableUpload &U) {
+  cudaStream_t s = U.d->ctx->stream;
+  unsigned char *p = nullptr;
+  GD_CUDA(cudaMallocAsync((void **)&p, U.host.size(), s));
+  U.d->allocs.push_back(p);
+  GD_CUDA(cudaMemcpyAsync(p, U.host.data(), U.host.size(), cudaMemcpyHostToDevice, s));
+  for (const auto &x : U.at) *x.first = p + x.second;
   return GD_OK;
 }
 
@@ -529,7 +541,8 @@ static void order_points(const gd_protein &P, const bool *hb_type, std::vector<i
 }
 
 // Packs the protein conformations into {x, y, z, ele} and {hpp, meta}.
-static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, gd_dcomplex *d) {
+static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, TableUpload &U) {
+  gd_dcomplex *d = U.d;
   KTables &T = d->T;
   const int pnp = P.pnp;
   const int pnp_pad = (pnp + TILE_PTS - 1) / TILE_PTS * TILE_PTS;
@@ -563,8 +576,8 @@ static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, gd_dco
     std::memcpy(&mf, &meta, 4);
     pb[s] = make_float2(P.hpp[p], mf);
   }
-  GD_TRY(upload(d, pa, &T.pt_a));
-  GD_TRY(upload(d, pb, &T.pt_b));
+  GD_TRY(upload(U, pa, &T.pt_a));
+  GD_TRY(upload(U, pb, &T.pt_b));
   T.pnp = pnp;
   T.pnp_pad = pnp_pad;
   T.n_prt = P.n_conf;
@@ -592,7 +605,8 @@ static float far_distance(const gd_enepara &F, int i, int j, float max_pmf0) {
 }
 
 // Ligand, pocket template and force-field tables of a complex.
-static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
+static gd_status upload_ligand(const gd_complex *cx, TableUpload &U) {
+  gd_dcomplex *d = U.d;
   const gd_ligand &L = cx->lig;
   const gd_enepara &F = *cx->ff;
   KTables &T = d->T;
@@ -643,13 +657,13 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
     // no valid atom: 0 x inf = NaN, as the reference's 0 / 0
     mw[m] = make_double2((double)cx->mcs.tcc[m], 1.0 / (double)c);
   }
-  GD_TRY(upload(d, ta, &T.tab_a));
-  GD_TRY(upload(d, tb, &T.tab_b));
-  GD_TRY(upload(d, tf, &T.tab_far));
-  GD_TRY(upload(d, lg, &T.lig));
-  GD_TRY(upload(d, lt, &T.lig_t));
-  GD_TRY(upload(d, lq, &T.lig_q));
-  GD_TRY(upload(d, psp, &T.psp));
+  GD_TRY(upload(U, ta, &T.tab_a));
+  GD_TRY(upload(U, tb, &T.tab_b));
+  GD_TRY(upload(U, tf, &T.tab_far));
+  GD_TRY(upload(U, lg, &T.lig));
+  GD_TRY(upload(U, lt, &T.lig_t));
+  GD_TRY(upload(U, lq, &T.lig_q));
+  GD_TRY(upload(U, psp, &T.psp));
   {
     // residues where some atom type of this ligand has a nonzero psp entry:
     // the kernel reads the table only there (elsewhere it adds zero)
@@ -661,12 +675,12 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
       if (present[t])
         for (int r = 0; r < n_col; ++r)
           if (psp[(size_t)t * n_col + r] != 0.0f) mask[r >> 5] |= 1u << (r & 31);
-    GD_TRY(upload(d, mask, &T.psp_mask));
+    GD_TRY(upload(U, mask, &T.psp_mask));
   }
-  GD_TRY(upload(d, kd, &T.kde));
-  GD_TRY(upload(d, koff, &T.kde_off));
-  GD_TRY(upload(d, mc, &T.mcs));
-  GD_TRY(upload(d, mw, &T.mcs_w));
+  GD_TRY(upload(U, kd, &T.kde));
+  GD_TRY(upload(U, koff, &T.kde_off));
+  GD_TRY(upload(U, mc, &T.mcs));
+  GD_TRY(upload(U, mw, &T.mcs_w));
 
   T.lna = lna;
   T.n_lig = L.n_conf;
@@ -708,7 +722,7 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
       if (hb == (pass == 0)) order.push_back(a);
       if (hb && pass == 0) ++T.n_hb;
     }
-  GD_TRY(upload(d, order, &T.lig_order));
+  GD_TRY(upload(U, order, &T.lig_order));
   for (int i = 0; i < GD_NLT; ++i) {
     T.hpl0[i] = F.hpl0[i];
     T.hpl1[i] = F.hpl1[i];
@@ -731,7 +745,8 @@ static gd_status upload_ligand(const gd_complex *cx, gd_dcomplex *d) {
 // its start pose (relative coordinates + centre, util.C:230-247) against the
 // complex's first protein conformation, in the reference's single-precision
 // order; one bit per (atom, point), rows of pnp_pad / 32 words.
-static gd_status upload_mcc_ref(const gd_complex *cx, int prt_conf, gd_dcomplex *d) {
+static gd_status upload_mcc_ref(const gd_complex *cx, int prt_conf, TableUpload &U) {
+  gd_dcomplex *d = U.d;
   const gd_ligand &L = cx->lig;
   const gd_protein &P = cx->prt;
   const gd_enepara &F = *cx->ff;
@@ -747,16 +762,30 @@ static gd_status upload_mcc_ref(const gd_complex *cx, int prt_conf, gd_dcomplex 
   float max_pmf0 = 0.f;
   for (int i = 0; i < GD_NLT; ++i)
     for (int j = 0; j < GD_NPT; ++j) max_pmf0 = std::max(max_pmf0, F.pmf0[i][j]);
+  T.near_mcc2 = max_pmf0 * max_pmf0 * 1.0001f + 1e-3f;
+  // points within reach of the ligand's box (the others have no contact)
+  float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+  std::vector<float> at((size_t)L.lna * 3);
   for (int a = 0; a < L.lna; ++a) {
-    const float lx = L.x[a] + L.center[0];
-    const float ly = L.y[a] + L.center[1];
-    const float lz = L.z[a] + L.center[2];
-    for (int s = 0; s < P.pnp; ++s) {
-      const int p = order[s];
-      const size_t i = (size_t)pc * P.pnp + p;
-      const float dx = lx - P.x[i];
-      const float dy = ly - P.y[i];
-      const float dz = lz - P.z[i];
+    const float v[3] = {L.x[a] + L.center[0], L.y[a] + L.center[1], L.z[a] + L.center[2]};
+    for (int k = 0; k < 3; ++k) {
+      at[(size_t)a * 3 + k] = v[k];
+      lo[k] = std::min(lo[k], v[k]);
+      hi[k] = std::max(hi[k], v[k]);
+    }
+  }
+  for (int s = 0; s < P.pnp; ++s) {
+    const int p = order[s];
+    const size_t i = (size_t)pc * P.pnp + p;
+    const float px = P.x[i], py = P.y[i], pz = P.z[i];
+    const float bx = std::max(0.f, std::max(lo[0] - px, px - hi[0]));
+    const float by = std::max(0.f, std::max(lo[1] - py, py - hi[1]));
+    const float bz = std::max(0.f, std::max(lo[2] - pz, pz - hi[2]));
+    if (bx * bx + by * by + bz * bz > T.near_mcc2) continue;
+    for (int a = 0; a < L.lna; ++a) {
+      const float dx = at[(size_t)a * 3] - px;
+      const float dy = at[(size_t)a * 3 + 1] - py;
+      const float dz = at[(size_t)a * 3 + 2] - pz;
       const float dst = sqrtf(dx * dx + dy * dy + dz * dz);
       if (dst <= F.pmf0[L.t[a]][P.t[p]]) {
         bits[(size_t)a * words + (s >> 5)] |= 1u << (s & 31);
@@ -764,10 +793,9 @@ static gd_status upload_mcc_ref(const gd_complex *cx, int prt_conf, gd_dcomplex 
       }
     }
   }
-  GD_TRY(upload(d, bits, &T.mcc_ref));
+  GD_TRY(upload(U, bits, &T.mcc_ref));
   T.mcc_words = words;
   T.mcc_nref = (float)nref;
-  T.near_mcc2 = max_pmf0 * max_pmf0 * 1.0001f + 1e-3f;
   return GD_OK;
 }
 
@@ -793,6 +821,7 @@ static gd_status complex_upload_common(gd_ctx *ctx, const gd_complex *cx,
   ctx_retain(ctx);
   gd_status st = GD_OK;
   try {
+    TableUpload U{d, {}, {}};
     if (share) {
       d->protein_owner = const_cast<gd_dcomplex *>(share);
       dcx_retain(d->protein_owner);
@@ -802,10 +831,11 @@ static gd_status complex_upload_common(gd_ctx *ctx, const gd_complex *cx,
       d->T.pnp_pad = share->T.pnp_pad;
       d->T.n_prt = n_prt;
     } else {
-      st = upload_protein(cx->prt, *cx->ff, d);
+      st = upload_protein(cx->prt, *cx->ff, U);
     }
-    if (st == GD_OK) st = upload_ligand(cx, d);
-    if (st == GD_OK) st = upload_mcc_ref(cx, share ? prt_conf0 : 0, d);
+    if (st == GD_OK) st = upload_ligand(cx, U);
+    if (st == GD_OK) st = upload_mcc_ref(cx, share ? prt_conf0 : 0, U);
+    if (st == GD_OK) st = upload_finish(U);
     if (st == GD_OK) {
       cudaError_t e = cudaStreamSynchronize(ctx->stream);
       if (e != cudaSuccess) st = fail(GD_ECUDA, "upload: %s", cudaGetErrorString(e));
@@ -861,7 +891,7 @@ gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int 
   R.poses = poses;
   R.terms = terms;
   R.raw = raw;
-  R.err = ctx->d_err;
+  R.err = ctx->h_err;
   R.hb_pairs = hb_pairs_of(d->T, tile.A);
   R.pose_item.T = d->T;
   R.pose_item.n_tmp = 1;
@@ -912,33 +942,48 @@ extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_
   if (n_pose == 0) return GD_OK;
   if (!poses || !terms) return fail(GD_EINVAL, "poses/terms NULL");
   GD_CUDA(cudaSetDevice(ctx->device));
-  float *dp = nullptr, *dt = nullptr;
-  double *dr = nullptr;
+  const size_t pose_b = sizeof(float) * 6 * (size_t)n_pose;
+  const size_t term_b = sizeof(float) * GD_NTERM * (size_t)n_pose;
+  const size_t raw_b = raw ? sizeof(double) * GD_NRAW * (size_t)n_pose : 0;
+  auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t total = up(pose_b) + up(term_b) + raw_b;
+  // a small call passes through the context's pinned memory, which the kernel
+  // reads and writes directly: no allocation and no copy in the stream
+  if (total <= kStageBytes && pose_work_bytes(d->T, n_pose) == 0) {
+    std::unique_lock<std::mutex> lk(ctx->stage_mu, std::try_to_lock);
+    if (lk.owns_lock()) {
+      unsigned char *p = ctx->stage;
+      std::memcpy(p, poses, pose_b);
+      const gd_status st = gd_energy_poses_dev(
+          ctx, d, prt_conf, lig_conf, n_pose, reinterpret_cast<float *>(p),
+          reinterpret_cast<float *>(p + up(pose_b)),
+          raw ? reinterpret_cast<double *>(p + up(pose_b) + up(term_b)) : nullptr);
+      if (st != GD_OK) return st;
+      GD_TRY(ctx_check(ctx));
+      std::memcpy(terms, p + up(pose_b), term_b);
+      if (raw) std::memcpy(raw, p + up(pose_b) + up(term_b), raw_b);
+      return GD_OK;
+    }
+  }
+  unsigned char *p = nullptr;
   gd_status st = GD_OK;
-  cudaError_t e = cudaMallocAsync(&dp, sizeof(float) * 6 * (size_t)n_pose, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMallocAsync(&dt, sizeof(float) * GD_NTERM * (size_t)n_pose, ctx->stream);
-  if (e == cudaSuccess && raw)
-    e = cudaMallocAsync(&dr, sizeof(double) * GD_NRAW * (size_t)n_pose, ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dp, poses, sizeof(float) * 6 * (size_t)n_pose, cudaMemcpyHostToDevice,
-                        ctx->stream);
+  cudaError_t e = cudaMallocAsync((void **)&p, total, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(p, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) {
     st = fail(GD_ENOMEM, "pose buffers: %s", cudaGetErrorString(e));
   } else {
-    st = gd_energy_poses_dev(ctx, d, prt_conf, lig_conf, n_pose, dp, dt, dr);
+    float *dt = reinterpret_cast<float *>(p + up(pose_b));
+    double *dr = raw ? reinterpret_cast<double *>(p + up(pose_b) + up(term_b)) : nullptr;
+    st = gd_energy_poses_dev(ctx, d, prt_conf, lig_conf, n_pose, reinterpret_cast<float *>(p), dt,
+                             dr);
     if (st == GD_OK) {
-      e = cudaMemcpyAsync(terms, dt, sizeof(float) * GD_NTERM * (size_t)n_pose,
-                          cudaMemcpyDeviceToHost, ctx->stream);
+      e = cudaMemcpyAsync(terms, dt, term_b, cudaMemcpyDeviceToHost, ctx->stream);
       if (e == cudaSuccess && raw)
-        e = cudaMemcpyAsync(raw, dr, sizeof(double) * GD_NRAW * (size_t)n_pose,
-                            cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(raw, dr, raw_b, cudaMemcpyDeviceToHost, ctx->stream);
       if (e != cudaSuccess) st = fail(GD_ECUDA, "copy back: %s", cudaGetErrorString(e));
     }
   }
-  if (dp) cudaFreeAsync(dp, ctx->stream);
-  if (dt) cudaFreeAsync(dt, ctx->stream);
-  if (dr) cudaFreeAsync(dr, ctx->stream);
+  if (p) cudaFreeAsync(p, ctx->stream);
   if (st != GD_OK) {
     cudaStreamSynchronize(ctx->stream);
     return st;

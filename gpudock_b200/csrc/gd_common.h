@@ -64,6 +64,11 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 
 }  // namespace gd
 
+// Bytes of a context's pinned staging memory.
+namespace gd {
+constexpr size_t kStageBytes = 1 << 20;
+}
+
 // Handles are reference counted: a complex keeps its context (and a shared
 // protein's owner) alive, a REMC run or batch keeps its complexes alive, so
 // callers may destroy them in any order.
@@ -71,7 +76,12 @@ struct gd_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  int *d_err = nullptr;
+  // pinned host memory that kernels access directly: the error word (read once
+  // the stream has ended, no copy), then kStageBytes through which small
+  // results and pose calls pass, used under stage_mu
+  int *h_err = nullptr;
+  unsigned char *stage = nullptr;
+  std::mutex stage_mu;
   uint64_t launches = 0;
   int n_sm = 148;
   int sched_mode = 0;      // GD_SCHED_*

@@ -8,6 +8,11 @@
 
 namespace gd {
 
+// Error word of a launch, in host memory: any thread may write its code.
+__device__ __forceinline__ void report(int *err, int code) {
+  *reinterpret_cast<volatile int *>(err) = code;
+}
+
 // ---------------------------------------------------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11).  Stream layout:
 //   key  = { seed_lo, seed_hi ^ stream_id }
@@ -198,7 +203,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
                                           uint32_t limit = (1u << 22)) {
   for (uint32_t i = 0; i < limit; ++i)
     if (mbar_try_wait(bar, parity)) return true;
-  if (err) atomicExch(err, code);
+  if (err) report(err, code);
   return false;
 }
 
@@ -273,7 +278,7 @@ __device__ __forceinline__ bool wait_progress(const int *p, int target, int *err
     if (ld_acquire(p) >= target) return true;
     __nanosleep(256);
   }
-  if (err) atomicExch(err, code);
+  if (err) report(err, code);
   return false;
 }
 

@@ -188,6 +188,11 @@ struct KRun {
   int *progress;         // [units] MC steps done (absolute step count)
   int *err;              // error word: 2 bounded wait ran out, 3 hb_pairs too
                          // low, 4 a piece's predecessor never finished
+  // nullptr, or: the launch's last CTA to end adds 1 to *done_flag (host
+  // memory), once every CTA's results are visible; *done_count (device, 0
+  // before the launch and again after it) counts the CTAs that have ended
+  unsigned *done_flag;
+  unsigned *done_count;
   unsigned long long *busy_ns;  // nullptr, or: each CTA adds the nanoseconds
                                 // from its start to its end (SM occupancy)
   uint32_t wait_limit;   // polls of a piece's dependency wait (0: 2^24, ~4 s)

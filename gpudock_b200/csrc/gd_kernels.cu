@@ -1194,7 +1194,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const int my_nhb =
       32 - __clz(__reduce_or_sync(0xffffffffu, lane < PT_ROWS ? my_hmask[lane] : 0u));
   // the host's bound must cover this warp; report it if not (code 3)
-  if (my_nhb > HB && lane == 0) atomicExch(R.err, 3);
+  if (my_nhb > HB && lane == 0) report(R.err, 3);
   // warps whose atoms need fewer H-bond pairs than the launch's HB take a
   // variant with one pair less (most warps of a ligand: the capable atoms
   // come first in the slot order, dealt round robin over the atom groups)
@@ -1614,6 +1614,18 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   if (R.busy_ns) {  // the CTA's time on its SM, for occupancy statistics
     __syncthreads();
     if (threadIdx.x == 0) atomicAdd(R.busy_ns, global_ns() - t_start);
+  }
+  if (R.done_flag) {
+    __syncthreads();  // every warp's results are written
+    if (threadIdx.x == 0) {
+      __threadfence_system();
+      // wraps back to 0 with the last CTA
+      if (atomicInc(R.done_count, gridDim.x - 1) == gridDim.x - 1) {
+        __threadfence_system();
+        volatile unsigned *flag = R.done_flag;
+        *flag = *flag + 1u;
+      }
+    }
   }
 }
 

@@ -71,6 +71,9 @@ struct Req {
   Clock::time_point t_submit, t_start, t_done;
   // device side while active
   gd_dcomplex *dcx = nullptr;
+  // its replica state: one allocation that starts with the results, so that
+  // they leave in one copy
+  unsigned char *d_state = nullptr;
   float *d_m_old = nullptr, *d_e_old = nullptr, *d_mb = nullptr, *d_cmcc = nullptr;
   int *d_idx = nullptr, *d_acs = nullptr, *d_acx = nullptr;
   gd_record *d_rec = nullptr;     // [n_rep][steps_total] with GD_MC_RECORD
@@ -97,25 +100,32 @@ struct Lane {
   int split = 1;                    // CTAs (a cluster) per request unit
   int packed = 0;                   // some unit has at most 16 replicas (KRun.packed)
   cudaStream_t stream = nullptr;
-  cudaEvent_t done = nullptr;
-  // the lane's kernel error word, in pinned host memory the kernels write
-  // directly (read after `done`)
+  // the lane's kernel error word and its count of ended launches, in pinned
+  // host memory that the kernels write directly, and the launch's CTA counter
+  // (KRun.done_flag): an event per launch, or a kernel that the stream orders
+  // after another one still running, holds back the other lanes that share the
+  // stream's hardware queue (16 requests on 3 idle servers' streams: 64 ms)
   int *h_err = nullptr;
+  unsigned *h_done = nullptr;
+  unsigned *d_count = nullptr;
+  unsigned n_issued = 0;            // launches to be counted in h_done
+  cudaEvent_t done = nullptr;       // or, behind an exchange kernel, an event
+  bool by_event = false;
   bool busy = false;                // a launch is in flight
+  bool init = false;                // it is an INIT launch
+  Clock::time_point t_asked;        // of the last look at the stream's state
   std::vector<Req *> members;       // active requests of this shape
   std::vector<Req *> fresh;         // admitted, not yet initialised
   std::vector<Req *> in_flight;     // the requests of the launch in flight
   // Launch descriptors in pinned host memory that the kernels read directly
-  // (no copy in the lane's stream, so a launch is one or two kernels and an
-  // event): one set for the INIT launch and one for the MC launch that
-  // follows it on the stream.  A set is rewritten only when the lane's
-  // previous launch has ended.
+  // (no copy in the lane's stream, so a launch is one kernel).  Rewritten only
+  // when the lane's previous launch has ended.
   struct Desc {
     KItem *items = nullptr;
     int *cta = nullptr;  // [3][cap_cta]
     KGroup *groups = nullptr;
     size_t cap_items = 0, cap_cta = 0, cap_groups = 0;
-  } desc[2];
+  } desc;
 };
 
 // (A, P, NA, stages, resident, group-major, steps per exchange, split, packed,
@@ -155,6 +165,8 @@ struct gd_server {
   // error words of the lanes (device, zeroed) and their pinned host copies,
   // allocated once with the server
   int *h_err_pool = nullptr;  // lanes' error words (pinned, written by kernels)
+  unsigned *h_done_pool = nullptr;   // lanes' ended launches (in the same block)
+  unsigned *d_count_pool = nullptr;  // lanes' CTA counters (behind d_busy_ns)
   // nanoseconds the server's CTAs spent on their SMs (all launches)
   unsigned long long *d_busy_ns = nullptr;
   // the scheduler thread's time spent issuing launches (written by the
@@ -186,14 +198,9 @@ std::vector<T> vcopy(const T *p, size_t n) {
 
 void release_device(Req *r) {
   cudaStream_t s = r->stream;
-  if (r->d_m_old) cudaFreeAsync(r->d_m_old, s);
-  if (r->d_e_old) cudaFreeAsync(r->d_e_old, s);
-  if (r->d_cmcc) cudaFreeAsync(r->d_cmcc, s);
-  if (r->d_mb) cudaFreeAsync(r->d_mb, s);
-  if (r->d_idx) cudaFreeAsync(r->d_idx, s);
-  if (r->d_acs) cudaFreeAsync(r->d_acs, s);
-  if (r->d_acx) cudaFreeAsync(r->d_acx, s);
+  if (r->d_state) cudaFreeAsync(r->d_state, s);
   if (r->d_rec) cudaFreeAsync(r->d_rec, s);
+  r->d_state = nullptr;
   r->d_m_old = r->d_e_old = r->d_mb = r->d_cmcc = nullptr;
   r->d_idx = r->d_acs = r->d_acx = nullptr;
   r->d_rec = nullptr;
@@ -259,6 +266,8 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
   GD_CUDA(cudaStreamCreateWithFlags(&L->stream, cudaStreamNonBlocking));
   GD_CUDA(cudaEventCreateWithFlags(&L->done, cudaEventDisableTiming));
   L->h_err = S->h_err_pool + slot;
+  L->h_done = S->h_done_pool + slot;
+  L->d_count = S->d_count_pool + slot;
   *out = L.get();
   S->lanes[key] = std::move(L);
   return GD_OK;
@@ -278,13 +287,17 @@ gd_status admit(gd_server *S, Req *r) {
   const size_t n = (size_t)r->n_rep;
   if (injected_alloc_failure(S->ctx))
     return fail(GD_ENOMEM, "request state: out of memory (injected)");
-  GD_CUDA(cudaMallocAsync(&r->d_m_old, n * 6 * sizeof(float), s));
-  GD_CUDA(cudaMallocAsync(&r->d_e_old, n * GD_NTERM * sizeof(float), s));
-  GD_CUDA(cudaMallocAsync(&r->d_cmcc, n * sizeof(float), s));
-  GD_CUDA(cudaMallocAsync(&r->d_mb, MAX_TMP * sizeof(float), s));
-  GD_CUDA(cudaMallocAsync(&r->d_idx, n * sizeof(int), s));
-  GD_CUDA(cudaMallocAsync(&r->d_acs, n * sizeof(int), s));
-  GD_CUDA(cudaMallocAsync(&r->d_acx, MAX_TMP * sizeof(int), s));
+  // [results: energies, moves, acceptance, temperature index][exchange
+  // counters][MCC][temperatures]
+  const size_t words = n * (GD_NTERM + 6 + 1 + 1) + MAX_TMP + n + MAX_TMP;
+  GD_CUDA(cudaMallocAsync((void **)&r->d_state, words * 4, s));
+  r->d_e_old = reinterpret_cast<float *>(r->d_state);
+  r->d_m_old = r->d_e_old + n * GD_NTERM;
+  r->d_acs = reinterpret_cast<int *>(r->d_m_old + n * 6);
+  r->d_idx = r->d_acs + n;
+  r->d_acx = r->d_idx + n;
+  r->d_cmcc = reinterpret_cast<float *>(r->d_acx + MAX_TMP);
+  r->d_mb = r->d_cmcc + n;
   GD_CUDA(cudaMemsetAsync(r->d_acx, 0, MAX_TMP * sizeof(int), s));
   const bool record = (r->mc.flags & GD_MC_RECORD) != 0;
   if (record) {
@@ -364,7 +377,7 @@ gd_status launch_lane(gd_server *S, Lane &L, const std::vector<Req *> &rs, int m
                    [](const auto &a, const auto &b) { return std::get<0>(a) > std::get<0>(b); });
   const size_t n_cta = ctas.size();
   // the lane's previous launch has ended, so its descriptor set is free
-  Lane::Desc &D = L.desc[mode == KMODE_INIT ? 0 : 1];
+  Lane::Desc &D = L.desc;
   GD_TRY(grow(&D.items, &D.cap_items, items.size()));
   GD_TRY(grow(&D.cta, &D.cap_cta, 3 * n_cta));
   GD_TRY(grow(&D.groups, &D.cap_groups, std::max<size_t>(groups.size(), 1)));
@@ -392,6 +405,12 @@ gd_status launch_lane(gd_server *S, Lane &L, const std::vector<Req *> &rs, int m
   R.n_steps = 0;  // per item (item_step)
   R.item_step = 1;
   R.err = L.h_err;
+  L.by_event = !groups.empty();
+  L.init = mode == KMODE_INIT;
+  if (!L.by_event) {
+    R.done_flag = L.h_done;
+    R.done_count = L.d_count;
+  }
   R.busy_ns = S->d_busy_ns;
   R.split = L.split;
   R.packed = L.packed;
@@ -404,8 +423,25 @@ gd_status launch_lane(gd_server *S, Lane &L, const std::vector<Req *> &rs, int m
     GD_CUDA(launch_exchange(D.items, D.groups, (int)groups.size(), 1, -1, nullptr, s));
     S->ctx->launches += 1;
     S->n_launch += 1;
+    GD_CUDA(cudaEventRecord(L.done, s));
+  } else {
+    L.n_issued += 1;
   }
+  L.t_asked = Clock::now();
   return GD_OK;
+}
+
+// Whether the lane's launch has ended: cudaSuccess, cudaErrorNotReady or the
+// launch's error.
+cudaError_t lane_state(Lane &L) {
+  if (L.by_event) return cudaEventQuery(L.done);
+  if (*(volatile unsigned *)L.h_done == L.n_issued) return cudaSuccess;
+  // a kernel that ended by an error counts nothing: ask the stream now and then
+  if (Clock::now() - L.t_asked < std::chrono::milliseconds(200)) return cudaErrorNotReady;
+  L.t_asked = Clock::now();
+  const cudaError_t q = cudaStreamQuery(L.stream);
+  if (q == cudaSuccess && *(volatile unsigned *)L.h_done != L.n_issued) return cudaErrorUnknown;
+  return q;
 }
 
 // MC steps of every request of a lane's next launch.  A request's CTAs take
@@ -438,23 +474,26 @@ void plan_steps(gd_server *S, const std::vector<Req *> &rs) {
 gd_status copy_out(Req *r) {
   cudaStream_t s = r->stream;
   const size_t n = (size_t)r->n_rep;
-  r->energy.resize(n * GD_NTERM);
-  r->movematrix.resize(n * 6);
-  r->acs.resize(n);
-  r->idx.resize(n);
-  r->acx.resize(r->mc.n_tmp);
-  GD_CUDA(cudaMemcpyAsync(r->energy.data(), r->d_e_old, n * GD_NTERM * 4, cudaMemcpyDeviceToHost,
-                          s));
-  GD_CUDA(cudaMemcpyAsync(r->movematrix.data(), r->d_m_old, n * 24, cudaMemcpyDeviceToHost, s));
-  GD_CUDA(cudaMemcpyAsync(r->acs.data(), r->d_acs, n * 4, cudaMemcpyDeviceToHost, s));
-  GD_CUDA(cudaMemcpyAsync(r->idx.data(), r->d_idx, n * 4, cudaMemcpyDeviceToHost, s));
-  GD_CUDA(cudaMemcpyAsync(r->acx.data(), r->d_acx, r->mc.n_tmp * 4, cudaMemcpyDeviceToHost, s));
+  const size_t words = n * (GD_NTERM + 6 + 1 + 1) + r->mc.n_tmp;
+  std::vector<uint32_t> out(words);
+  GD_CUDA(cudaMemcpyAsync(out.data(), r->d_state, words * 4, cudaMemcpyDeviceToHost, s));
   if (r->d_rec) {
     r->rec.resize(n * (size_t)r->mc.steps_total);
     GD_CUDA(cudaMemcpyAsync(r->rec.data(), r->d_rec, r->rec.size() * sizeof(gd_record),
                             cudaMemcpyDeviceToHost, s));
   }
   GD_CUDA(cudaStreamSynchronize(s));
+  const uint32_t *w = out.data();
+  auto take = [&](auto &v, size_t count) {
+    v.resize(count);
+    std::memcpy(v.data(), w, count * 4);
+    w += count;
+  };
+  take(r->energy, n * GD_NTERM);
+  take(r->movematrix, n * 6);
+  take(r->acs, n);
+  take(r->idx, n);
+  take(r->acx, (size_t)r->mc.n_tmp);
   return GD_OK;
 }
 
@@ -533,7 +572,7 @@ void scheduler(gd_server *S) {
     for (auto &kv : S->lanes) {
       Lane &L = *kv.second;
       if (L.busy) {
-        const cudaError_t q = cudaEventQuery(L.done);
+        const cudaError_t q = lane_state(L);
         if (q == cudaErrorNotReady) continue;
         L.busy = false;
         progressed = true;
@@ -549,8 +588,8 @@ void scheduler(gd_server *S) {
             lane_failed.emplace_back(r, st);
             continue;
           }
-          r->step += r->n_run;
-          if (r->step >= r->mc.steps_total) {
+          if (!L.init) r->step += r->n_run;
+          if (!L.init && r->step >= r->mc.steps_total) {
             const gd_status cs = copy_out(r);
             if (cs == GD_OK)
               finished.push_back(r);
@@ -586,17 +625,18 @@ void scheduler(gd_server *S) {
       if (L.busy || (L.members.empty() && L.fresh.empty())) continue;
       const auto t_issue = Clock::now();
       gd_status st = GD_OK;
+      // new requests are initialised by a launch of their own, which the next
+      // MC launch does not have to wait for in the stream
+      std::vector<Req *> now;
       if (!L.fresh.empty()) {
-        st = launch_lane(S, L, L.fresh, KMODE_INIT);
-        for (Req *r : L.fresh) L.members.push_back(r);
-        L.fresh.clear();
+        now.swap(L.fresh);
+        for (Req *r : now) L.members.push_back(r);
+        st = launch_lane(S, L, now, KMODE_INIT);
+      } else {
+        now = L.members;
+        plan_steps(S, now);
+        st = launch_lane(S, L, now, KMODE_REMC);
       }
-      if (st == GD_OK) {
-        plan_steps(S, L.members);
-        st = launch_lane(S, L, L.members, KMODE_REMC);
-      }
-      if (st == GD_OK && cudaEventRecord(L.done, L.stream) != cudaSuccess)
-        st = fail(GD_ECUDA, "server: event record");
       if (st != GD_OK) {
         cudaStreamSynchronize(L.stream);
         for (Req *r : L.members) lane_failed.emplace_back(r, st);
@@ -605,7 +645,7 @@ void scheduler(gd_server *S) {
       }
       S->host_launch_s.store(S->host_launch_s.load() +
                              std::chrono::duration<double>(Clock::now() - t_issue).count());
-      L.in_flight = L.members;
+      L.in_flight.swap(now);
       L.busy = true;
       S->n_iter += 1;
       progressed = true;
@@ -619,11 +659,11 @@ void scheduler(gd_server *S) {
       if (!failed.empty() || !lane_failed.empty() || !cancelled.empty() || !finished.empty())
         S->done_cv.notify_all();
     }
-    if (!progressed) std::this_thread::sleep_for(std::chrono::microseconds(100));
+    if (!progressed) std::this_thread::sleep_for(std::chrono::microseconds(50));
   }
   // stopping: wait for the lanes' launches to end
   for (auto &kv : S->lanes)
-    if (kv.second->busy) cudaEventSynchronize(kv.second->done);
+    if (kv.second->busy) cudaStreamSynchronize(kv.second->stream);
 }
 
 gd_status copy_request(gd_server *S, int protein_id, const gd_complex *cx,
@@ -693,15 +733,18 @@ extern "C" gd_status gd_server_create(int device, size_t hbm_budget_bytes, int m
   S->budget = hbm_budget_bytes;
   S->max_active = max_active > 0 ? max_active : 2 * ctx->n_sm;
   S->steps_per_launch = steps_per_launch;
-  if (cudaMalloc(&S->d_busy_ns, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMemset(S->d_busy_ns, 0, sizeof(unsigned long long)) != cudaSuccess ||
-      cudaMallocHost(&S->h_err_pool, kMaxLanes * sizeof(int)) != cudaSuccess) {
+  const size_t dev_b = sizeof(unsigned long long) + kMaxLanes * sizeof(unsigned);
+  if (cudaMalloc(&S->d_busy_ns, dev_b) != cudaSuccess ||
+      cudaMemset(S->d_busy_ns, 0, dev_b) != cudaSuccess ||
+      cudaMallocHost(&S->h_err_pool, 2 * kMaxLanes * sizeof(int)) != cudaSuccess) {
     if (S->d_busy_ns) cudaFree(S->d_busy_ns);
     ctx_release(ctx);
     delete S;
     return fail(GD_ENOMEM, "server error words");
   }
-  std::memset(S->h_err_pool, 0, kMaxLanes * sizeof(int));
+  std::memset(S->h_err_pool, 0, 2 * kMaxLanes * sizeof(int));
+  S->h_done_pool = reinterpret_cast<unsigned *>(S->h_err_pool + kMaxLanes);
+  S->d_count_pool = reinterpret_cast<unsigned *>(S->d_busy_ns + 1);
   S->th = std::thread(scheduler, S);
   *out = S;
   return GD_OK;
@@ -889,11 +932,10 @@ extern "C" gd_status gd_server_destroy(gd_server *S) {
   for (auto &kv : S->lanes) {
     Lane &L = *kv.second;
     cudaStreamSynchronize(L.stream);
-    for (Lane::Desc &D : L.desc) {
-      if (D.items) cudaFreeHost(D.items);
-      if (D.cta) cudaFreeHost(D.cta);
-      if (D.groups) cudaFreeHost(D.groups);
-    }
+    Lane::Desc &D = L.desc;
+    if (D.items) cudaFreeHost(D.items);
+    if (D.cta) cudaFreeHost(D.cta);
+    if (D.groups) cudaFreeHost(D.groups);
     cudaEventDestroy(L.done);
     cudaStreamDestroy(L.stream);
   }
