@@ -125,6 +125,49 @@ Tile tile_for(gd_ctx *ctx, const KTables &T) {
   return default_tile(hi);
 }
 
+// Pinned blocks of the contexts.  Pinning memory takes 1 .. 3 ms up to 1 MB, so
+// the first context pins blocks for kPinnedSlots contexts at once; they are
+// unpinned with the last of them.  Contexts beyond that pin their own.
+static constexpr size_t kPinnedBlock = 256 + kStageBytes;
+static constexpr int kPinnedSlots = 4;
+static std::mutex g_pinned_mu;
+static unsigned char *g_pinned = nullptr;
+static unsigned g_pinned_used = 0;  // a bit per block
+
+static cudaError_t pinned_acquire(void **p) {
+  std::lock_guard<std::mutex> g(g_pinned_mu);
+  if (!g_pinned) {
+    const cudaError_t e = cudaHostAlloc((void **)&g_pinned, kPinnedBlock * kPinnedSlots,
+                                        cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+      g_pinned = nullptr;
+      return e;
+    }
+  }
+  for (int k = 0; k < kPinnedSlots; ++k)
+    if (!(g_pinned_used >> k & 1u)) {
+      g_pinned_used |= 1u << k;
+      *p = g_pinned + (size_t)k * kPinnedBlock;
+      return cudaSuccess;
+    }
+  return cudaHostAlloc(p, kPinnedBlock, cudaHostAllocPortable);
+}
+
+static void pinned_release(void *p) {
+  if (!p) return;
+  std::lock_guard<std::mutex> g(g_pinned_mu);
+  unsigned char *q = static_cast<unsigned char *>(p);
+  if (!g_pinned || q < g_pinned || q >= g_pinned + kPinnedBlock * kPinnedSlots) {
+    cudaFreeHost(p);
+    return;
+  }
+  g_pinned_used &= ~(1u << ((q - g_pinned) / kPinnedBlock));
+  if (g_pinned_used == 0) {
+    cudaFreeHost(g_pinned);
+    g_pinned = nullptr;
+  }
+}
+
 void ctx_retain(gd_ctx *c) {
   if (c) c->refs++;
 }
@@ -169,7 +212,8 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
-  cudaFreeHost(c->h_err);
+  if (c->pool) cudaMemPoolDestroy(c->pool);
+  pinned_release(c->h_err);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -402,19 +446,35 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
     }
     c->own_stream = true;
   }
-  e = cudaMallocHost((void **)&c->h_err, 256 + kStageBytes);
+  e = pinned_acquire((void **)&c->h_err);
   if (e != cudaSuccess) {
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return fail(GD_ENOMEM, "pinned host memory: %s", cudaGetErrorString(e));
   }
   std::memset(c->h_err, 0, 256);
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  uint64_t keep = kKeepBytes;
+  e = cudaMemPoolCreate(&c->pool, &props);
+  if (e == cudaSuccess)
+    e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) {
+    if (c->pool) cudaMemPoolDestroy(c->pool);
+    pinned_release(c->h_err);
+    if (c->own_stream) cudaStreamDestroy(c->stream);
+    delete c;
+    return fail(GD_ENOMEM, "memory pool: %s", cudaGetErrorString(e));
+  }
   c->stage = reinterpret_cast<unsigned char *>(c->h_err) + 256;
   // the fixed scratch of gd_energy_poses_noalloc is committed now, not on
   // that entry point's first call
   const gd_status st = noalloc_attach(c);
   if (st != GD_OK) {
-    cudaFreeHost(c->h_err);
+    cudaMemPoolDestroy(c->pool);
+    pinned_release(c->h_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return st;
@@ -927,7 +987,7 @@ extern "C" gd_status gd_energy_poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int 
   GD_CUDA(cudaSetDevice(ctx->device));
   void *work = nullptr;
   const size_t bytes = pose_work_bytes(d->T, n_pose);
-  if (bytes) GD_CUDA(cudaMallocAsync(&work, bytes, ctx->stream));
+  if (bytes) GD_CUDA(work_alloc(ctx, &work, bytes));
   const gd_status st =
       poses_launch(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, work);
   if (work) cudaFreeAsync(work, ctx->stream);
@@ -967,7 +1027,7 @@ extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_
   }
   unsigned char *p = nullptr;
   gd_status st = GD_OK;
-  cudaError_t e = cudaMallocAsync((void **)&p, total, ctx->stream);
+  cudaError_t e = work_alloc(ctx, (void **)&p, total);
   if (e == cudaSuccess) e = cudaMemcpyAsync(p, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) {
     st = fail(GD_ENOMEM, "pose buffers: %s", cudaGetErrorString(e));

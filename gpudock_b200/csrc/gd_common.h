@@ -64,9 +64,10 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 
 }  // namespace gd
 
-// Bytes of a context's pinned staging memory.
+// Bytes of workspace a context keeps between calls, and of its pinned staging.
 namespace gd {
-constexpr size_t kStageBytes = 1 << 20;
+constexpr size_t kKeepBytes = 64 << 20;
+constexpr size_t kStageBytes = 256 << 10;
 }
 
 // Handles are reference counted: a complex keeps its context (and a shared
@@ -81,6 +82,11 @@ struct gd_ctx {
   // results and pose calls pass, used under stage_mu
   int *h_err = nullptr;
   unsigned char *stage = nullptr;
+  // the calls' own workspaces (poses, similarity): a pool that keeps up to
+  // kKeepBytes mapped between calls, destroyed with the context (from the
+  // device's default pool, which unmaps at every synchronisation, they took
+  // 50 .. 100 us each)
+  cudaMemPool_t pool = nullptr;
   std::mutex stage_mu;
   uint64_t launches = 0;
   int n_sm = 148;
@@ -123,6 +129,10 @@ void ctx_release(gd_ctx *c);
 void dcx_retain(gd_dcomplex *d);
 void dcx_release(gd_dcomplex *d);
 gd_status ctx_check(gd_ctx *c);
+// Stream-ordered workspace of a call (freed with cudaFreeAsync).
+inline cudaError_t work_alloc(gd_ctx *c, void **p, size_t bytes) {
+  return cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+}
 // Status for a nonzero kernel error word (KRun.err).
 gd_status kernel_error(int code);
 // Loads the module that holds the fixed pose-scratch array of

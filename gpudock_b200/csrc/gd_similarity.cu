@@ -340,15 +340,15 @@ __global__ void __launch_bounds__(kSimThreads)
 
 // Device buffers of one call, freed on every path.
 struct SimBuffers {
-  cudaStream_t s;
+  gd_ctx *ctx;
   std::vector<void *> ptrs;
   ~SimBuffers() {
-    for (void *p : ptrs) cudaFreeAsync(p, s);
+    for (void *p : ptrs) cudaFreeAsync(p, ctx->stream);
   }
   template <typename T>
   cudaError_t get(T **p, size_t count) {
     void *v = nullptr;
-    const cudaError_t e = cudaMallocAsync(&v, std::max<size_t>(count, 1) * sizeof(T), s);
+    const cudaError_t e = work_alloc(ctx, &v, std::max<size_t>(count, 1) * sizeof(T));
     if (e == cudaSuccess) ptrs.push_back(v);
     *p = (T *)v;
     return e;
@@ -407,7 +407,7 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
   const size_t n = (size_t)n_conf;
   gd_status st = GD_OK;
   {
-    SimBuffers B{s, {}};
+    SimBuffers B{ctx, {}};
     SimConf *d_conf = nullptr;
     uint32_t *d_uni = nullptr, *d_maps = nullptr;
     float *d_bound = nullptr, *d_S = nullptr;
