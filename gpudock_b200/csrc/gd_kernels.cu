@@ -942,6 +942,16 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 
   // a pose launch's grid is an upper bound of its blocks
   if (MODE == KMODE_POSES && R.pose_grid && unit >= R.pose_grid->n_blocks) break;
+  // this lane's pose, on its way while the tables are set up (a small call's
+  // poses are in host memory)
+  float pose[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (MODE == KMODE_POSES && warp == 0 && !R.pose_grid) {
+    const int per = PACKED ? R.packed : 32, p = unit * per + (lane & (per - 1));
+    if (p < R.n_pose) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) pose[i] = __ldg(&R.poses[(size_t)p * 6 + i]);
+    }
+  }
 
   // ---- item of this piece into shared memory, pair tables -----------------
   const int item = (MODE == KMODE_POSES) ? 0 : R.cta_item[unit];
@@ -971,43 +981,50 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
       }
       s_kde[s] = sk;
     }
-    // point types GD_NPT..PT_ROWS-1 (the padding points) get all-zero entries
+    __syncthreads();
+    // The pair tables from the slots' types (a padding atom's row is all zero;
+    // point types GD_NPT .. PT_ROWS-1, the padding points, get zeros).  Each
+    // phase's table reads depend on shared memory only and are independent of
+    // one another: a launch's first CTA waits for this (set-up of a small pose
+    // call 17 K of 60 K cycles with chained reads).
     for (int i = threadIdx.x; i < A * NH * PT_ROWS; i += blockDim.x) {
       const int pt = i % PT_ROWS, h = (i / PT_ROWS) % NH, ag = i / (PT_ROWS * NH);
       const int s0 = ag + A * (2 * h), s1 = s0 + A;
-      const int ptc = pt < GD_NPT ? pt : 0;
-      const int r0 = (s0 < lna && pt < GD_NPT ? TG.lig_t[TG.lig_order[s0]] : GD_NLT) * GD_NPT + ptc;
-      const int r1 = (s1 < lna && pt < GD_NPT ? TG.lig_t[TG.lig_order[s1]] : GD_NLT) * GD_NPT + ptc;
+      const int r0 = (pt < GD_NPT ? s_lt[s0] * GD_NPT + pt : GD_NLT * GD_NPT);
+      const int r1 = (pt < GD_NPT ? s_lt[s1] * GD_NPT + pt : GD_NLT * GD_NPT);
       const float4 a0 = TG.tab_a[r0], a1 = TG.tab_a[r1];
+      const float2 b0 = TG.tab_b[r0], b1 = TG.tab_b[r1];
       s_ptab[2 * i] = make_float4(a0.x, a1.x, -a0.y, -a1.y);
       s_ptab[2 * i + 1] = make_float4(-a0.z, -a1.z, a0.w, a1.w);
       // H-bond term where hdb0 > 0.1 (calcenergy_d.cu:115-126)
-      const float2 b0 = TG.tab_b[r0], b1 = TG.tab_b[r1];
       const bool h0 = b0.x > 0.1f, h1 = b1.x > 0.1f;
       s_htab[i] = make_float4(h0 ? -b0.x : 0.f, h1 ? -b1.x : 0.f, h0 ? b0.y : 0.f,
                               h1 ? b1.y : 0.f);
     }
+    // far form: the group's largest distance for each point type
+    for (int i = threadIdx.x; i < A * PT_ROWS; i += blockDim.x) {
+      const int pt = i % PT_ROWS, ag = i / PT_ROWS;
+      float fd = 0.f;
+      if (pt < GD_NPT) {
+#pragma unroll
+        for (int k = 0; k < NA; ++k) fd = fmaxf(fd, TG.tab_far[s_lt[ag + A * k] * GD_NPT + pt]);
+      }
+      s_far[i] = fd;
+    }
+    __syncthreads();
+    // which pairs have an H-bond term, and the group's PMF sum
     for (int i = threadIdx.x; i < A * PT_ROWS; i += blockDim.x) {
       const int pt = i % PT_ROWS, ag = i / PT_ROWS;
       uint32_t m = 0;
-      for (int h = 0; h < NH && pt < GD_NPT; ++h) {
-        const int s0 = ag + A * (2 * h), s1 = s0 + A;
-        const int r0 = (s0 < lna ? TG.lig_t[TG.lig_order[s0]] : GD_NLT) * GD_NPT + pt;
-        const int r1 = (s1 < lna ? TG.lig_t[TG.lig_order[s1]] : GD_NLT) * GD_NPT + pt;
-        if (TG.tab_b[r0].x > 0.1f || TG.tab_b[r1].x > 0.1f) m |= 1u << h;
+      double fp = 0.0;
+#pragma unroll
+      for (int h = 0; h < NH; ++h) {
+        const int q = (ag * NH + h) * PT_ROWS + pt;
+        const float4 H = s_htab[q], P1 = s_ptab[2 * q + 1];
+        if (H.x != 0.f || H.y != 0.f) m |= 1u << h;
+        fp += (double)P1.z + (double)P1.w;
       }
       s_hmask[i] = m;
-      // far form: the group's largest distance and its PMF sum
-      float fd = 0.f;
-      double fp = 0.0;
-      for (int k = 0; k < NA && pt < GD_NPT; ++k) {
-        const int s = ag + A * k;
-        if (s >= lna) break;
-        const int r = TG.lig_t[TG.lig_order[s]] * GD_NPT + pt;
-        fd = fmaxf(fd, TG.tab_far[r]);
-        fp += (double)TG.tab_a[r].w;
-      }
-      s_far[i] = fd;
       s_fpmf[i] = fp;
     }
     __syncthreads();  // every thread has read s_ctl->item
@@ -1226,7 +1243,10 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
           m_new[i] = away ? __fadd_rn(__fmul_rn(I.move_scale[i], 44.5f), 0.0f) : 0.0f;
       } else {
 #pragma unroll
-        for (int i = 0; i < 6; ++i) m_new[i] = active ? R.poses[(size_t)rep * 6 + i] : 0.f;
+        for (int i = 0; i < 6; ++i) {
+          m_new[i] = pose[i];
+          if (R.pose_grid) m_new[i] = active ? R.poses[(size_t)rep * 6 + i] : 0.f;
+        }
       }
       float rot[9];
       make_rot(m_new[3], m_new[4], m_new[5], rot);
@@ -1444,8 +1464,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     // loop of small bodies, not unrolled: once a step, its instructions come
     // from beyond the first instruction cache.
     double dkde = 0.0, dlhm = 0.0;
-    auto placed = [&](int a) {
-      const float4 o = orig[a];
+    auto placed = [&](const float4 &o) {
       return make_float3(q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx,
                          q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy,
                          q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz);
@@ -1455,11 +1474,13 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
       if (i < lna) {
         const SlotKde sk = s_kde[i];
         if (sk.end > sk.begin) {
-          const float3 x = placed(s_atom[i]);
+          const float3 x = placed(orig[s_atom[i]]);
           float kv = 0.f;
+          float4 Kn = T.kde[min(sk.begin + sub, sk.end - 1)];
 #pragma unroll 1
           for (int q = sk.begin + sub; q < sk.end; q += subs) {
-            const float4 K = T.kde[q];
+            const float4 K = Kn;
+            Kn = T.kde[min(q + subs, sk.end - 1)];  // one point ahead
             const float dx = x.x - K.x, dy = x.y - K.y, dz = x.z - K.z;
             kv += fex2(T.kde2 * LOG2E * fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
           }
@@ -1470,11 +1491,14 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         float sv = 0.f;
         const float4 *Mm = T.mcs + (size_t)m * lna;
         const double2 w = T.mcs_w[m];
+        float4 Mn = Mm[min(sub, lna - 1)], on = orig[min(sub, lna - 1)];
 #pragma unroll 1
         for (int l = sub; l < lna; l += subs) {
-          const float4 M = Mm[l];
+          const float4 M = Mn, o = on;
+          Mn = Mm[min(l + subs, lna - 1)];  // one atom ahead
+          on = orig[min(l + subs, lna - 1)];
           if (M.w != 0.0f) {
-            const float3 x = placed(l);
+            const float3 x = placed(o);
             const float dx = x.x - M.x, dy = x.y - M.y, dz = x.z - M.z;
             sv += fmaf(dz, dz, fmaf(dy, dy, dx * dx));
           }
