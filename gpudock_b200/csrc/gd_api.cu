@@ -168,6 +168,50 @@ static void pinned_release(void *p) {
   }
 }
 
+// The workspaces of calls come from one memory pool per device, shared by its
+// contexts (stream-ordered, so safe between them) and destroyed with the last
+// of them.  It keeps up to kKeepBytes mapped between calls; the device's default
+// pool unmaps at every synchronisation, which cost 50 .. 100 us per allocation,
+// and a pool's first allocation takes milliseconds, so contexts do not have one
+// each.
+struct WorkPool {
+  cudaMemPool_t pool = nullptr;
+  int users = 0;
+};
+static std::mutex g_work_mu;
+static std::map<int, WorkPool> g_work;  // by device
+
+static cudaError_t work_pool_acquire(int device, cudaMemPool_t *out) {
+  std::lock_guard<std::mutex> g(g_work_mu);
+  WorkPool &w = g_work[device];
+  if (!w.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = kKeepBytes;
+    cudaError_t e = cudaMemPoolCreate(&w.pool, &props);
+    if (e == cudaSuccess)
+      e = cudaMemPoolSetAttribute(w.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      if (w.pool) cudaMemPoolDestroy(w.pool);
+      w.pool = nullptr;
+      return e;
+    }
+  }
+  w.users += 1;
+  *out = w.pool;
+  return cudaSuccess;
+}
+
+static void work_pool_release(int device) {
+  std::lock_guard<std::mutex> g(g_work_mu);
+  WorkPool &w = g_work[device];
+  if (--w.users > 0) return;
+  cudaMemPoolDestroy(w.pool);
+  w = WorkPool{};
+}
+
 void ctx_retain(gd_ctx *c) {
   if (c) c->refs++;
 }
@@ -212,7 +256,7 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
-  if (c->pool) cudaMemPoolDestroy(c->pool);
+  work_pool_release(c->device);
   pinned_release(c->h_err);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -453,16 +497,8 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
     return fail(GD_ENOMEM, "pinned host memory: %s", cudaGetErrorString(e));
   }
   std::memset(c->h_err, 0, 256);
-  cudaMemPoolProps props = {};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = device;
-  uint64_t keep = kKeepBytes;
-  e = cudaMemPoolCreate(&c->pool, &props);
-  if (e == cudaSuccess)
-    e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  e = work_pool_acquire(device, &c->pool);
   if (e != cudaSuccess) {
-    if (c->pool) cudaMemPoolDestroy(c->pool);
     pinned_release(c->h_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -473,7 +509,7 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
   // that entry point's first call
   const gd_status st = noalloc_attach(c);
   if (st != GD_OK) {
-    cudaMemPoolDestroy(c->pool);
+    work_pool_release(device);
     pinned_release(c->h_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;

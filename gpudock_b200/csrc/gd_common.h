@@ -64,7 +64,8 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 
 }  // namespace gd
 
-// Bytes of workspace a context keeps between calls, and of its pinned staging.
+// Bytes of workspace kept mapped between calls on a device, and of a context's
+// pinned staging.
 namespace gd {
 constexpr size_t kKeepBytes = 64 << 20;
 constexpr size_t kStageBytes = 256 << 10;
@@ -82,10 +83,8 @@ struct gd_ctx {
   // results and pose calls pass, used under stage_mu
   int *h_err = nullptr;
   unsigned char *stage = nullptr;
-  // the calls' own workspaces (poses, similarity): a pool that keeps up to
-  // kKeepBytes mapped between calls, destroyed with the context (from the
-  // device's default pool, which unmaps at every synchronisation, they took
-  // 50 .. 100 us each)
+  // the calls' own workspaces (poses, similarity): the device's pool of this
+  // library (work_pool_acquire)
   cudaMemPool_t pool = nullptr;
   std::mutex stage_mu;
   uint64_t launches = 0;
