@@ -995,8 +995,9 @@ gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int 
   R.pose_item.n_prt = d->T.n_prt;
   int grid = 0;
   if (work) {
-    GD_CUDA(pose_cells(&R, work, &grid, ctx->stream));
-    ctx->launches += 4;
+    int launches = 0;
+    GD_CUDA(pose_cells(&R, work, &grid, &launches, ctx->stream));
+    ctx->launches += launches;
   } else {
     pose_units(ctx, d->T, n_pose, &R.split, &R.packed);
     const int per = R.packed ? R.packed : 32;

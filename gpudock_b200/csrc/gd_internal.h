@@ -241,8 +241,8 @@ size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split = 1);
 size_t pose_work_bytes(const KTables &T, int n_pose);
 // Deals the poses of R (n_pose, poses) into cells, using pose_work_bytes of
 // workspace until the energy launch has ended; fills R's cell arrays and the
-// launch's grid.
-cudaError_t pose_cells(KRun *R, void *work, int *grid, cudaStream_t s);
+// launch's grid and the number of launches made.
+cudaError_t pose_cells(KRun *R, void *work, int *grid, int *launches, cudaStream_t s);
 
 // Kernel launchers (gd_kernels.cu); return the launch status.
 cudaError_t launch_dock(const KRun &R, int NA, int grid, cudaStream_t s);

@@ -9,9 +9,10 @@
 // Poses without a usable translation (not finite, or beyond kFarOut) get a
 // cell of their own, for which no point is far.
 //
-// Four short launches (about 10 us together): the box of the translations;
+// Four short launches (about 12 us together): the box of the translations;
 // every pose's cell and its rank in it; the cells' first 32-pose blocks; the
-// poses in block order.
+// poses in block order.  Up to kSmallPoses poses, one launch of one CTA does
+// all of it (about 5 us).
 #include <algorithm>
 
 #include "gd_common.h"
@@ -25,6 +26,7 @@ constexpr float kFarOut = 4.0e3f;
 // Poses per cell: a cell's last block is half empty on average, so about 5% of
 // the blocks' lanes are idle.
 constexpr int kPosesPerCell = 320;
+constexpr int kSmallPoses = 16384;
 constexpr float kMinEdge = 0.75f;  // smaller cells gain little (the ligand is larger)
 
 int max_cells(int n_pose) { return std::max(1, std::min(kMaxCells, n_pose / kPosesPerCell)); }
@@ -122,6 +124,15 @@ __device__ PoseGrid make_grid(const unsigned *box, int max_cells) {
   return g;
 }
 
+__device__ __forceinline__ int cell_of(const PoseGrid &g, const float t[3]) {
+  if (!usable(t)) return g.n_cells;
+  int c[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    c[k] = min(g.n[k] - 1, max(0, (int)((t[k] - g.lo[k]) * g.inv_edge)));
+  return (c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
+}
+
 __global__ void __launch_bounds__(kThreads)
     cell_kernel(const float *poses, int n, int max_cells, const unsigned *box, PoseGrid *grid,
                 int *count, int2 *at) {
@@ -134,14 +145,7 @@ __global__ void __launch_bounds__(kThreads)
   const int i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
   const float t[3] = {poses[(size_t)i * 6], poses[(size_t)i * 6 + 1], poses[(size_t)i * 6 + 2]};
-  int cell = g.n_cells;  // no usable translation
-  if (usable(t)) {
-    int c[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      c[k] = min(g.n[k] - 1, max(0, (int)((t[k] - g.lo[k]) * g.inv_edge)));
-    cell = (c[2] * g.n[1] + c[1]) * g.n[0] + c[0];
-  }
+  const int cell = cell_of(g, t);
   at[i] = make_int2(cell, atomicAdd(&count[cell], 1));
 }
 
@@ -188,18 +192,103 @@ __global__ void __launch_bounds__(kThreads)
   if (a.y % 32 == 0) block_cell[b] = a.x;
 }
 
+// All of the above for up to kSmallPoses poses: 16 poses a thread, the cells'
+// counts in shared memory.
+__global__ void __launch_bounds__(1024)
+    small_kernel(const float *poses, int n, int max_cells, PoseGrid *grid, int *count, int *first,
+                 int *order, int *block_cell) {
+  constexpr int kCells = kSmallPoses / kPosesPerCell + 1;
+  constexpr int kEach = kSmallPoses / 1024;
+  __shared__ unsigned s_box[6];
+  __shared__ PoseGrid g;
+  __shared__ int s_count[kCells], s_first[kCells];
+  if (threadIdx.x < 6) s_box[threadIdx.x] = 0u;
+  for (int c = threadIdx.x; c < kCells; c += 1024) s_count[c] = 0;
+  __syncthreads();
+  float t[kEach][3];
+  unsigned m[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int i = j * 1024 + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[j][k] = i < n ? poses[(size_t)i * 6 + k] : 0.f;
+    if (i < n && usable(t[j])) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        m[k] = max(m[k], ordered(-t[j][k]));
+        m[3 + k] = max(m[3 + k], ordered(t[j][k]));
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+    if ((threadIdx.x & 31) == 0 && m[k] != 0u) atomicMax(&s_box[k], m[k]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) g = make_grid(s_box, max_cells);
+  __syncthreads();
+  int cell[kEach], rank[kEach];
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    cell[j] = rank[j] = 0;
+    if (j * 1024 + (int)threadIdx.x >= n) continue;
+    cell[j] = cell_of(g, t[j]);
+    rank[j] = atomicAdd(&s_count[cell[j]], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int b = 0;
+    for (int c = 0; c <= g.n_cells; ++c) {
+      s_first[c] = b;
+      b += (s_count[c] + 31) / 32;
+    }
+    g.n_blocks = b;
+    *grid = g;
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c <= g.n_cells; c += 1024) {
+    count[c] = s_count[c];
+    first[c] = s_first[c];
+  }
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const int i = j * 1024 + threadIdx.x;
+    if (i >= n) continue;
+    const int b = s_first[cell[j]] + rank[j] / 32;
+    order[b * 32 + rank[j] % 32] = i;
+    if (rank[j] % 32 == 0) block_cell[b] = cell[j];
+  }
+}
+
 }  // namespace
 
 size_t pose_work_bytes(const KTables &T, int n_pose) {
-  // Cells pay once their launches are a small part of the call (1e12 pairs/s):
-  // about 3% at 5e8 pairs.
-  if (n_pose < 4096 || (double)n_pose * T.lna * T.pnp < 5e8) return 0;
+  // Cells pay once dealing the poses is a small part of the call (1e12
+  // pairs/s): about 5% at 1e8 pairs for one launch, 3% at 5e8 for four.  Below
+  // 2,048 poses a call's units are spread over the SMs in other ways
+  // (pose_units).
+  if (n_pose < 2048 || (double)n_pose * T.lna * T.pnp < (n_pose <= kSmallPoses ? 1e8 : 5e8))
+    return 0;
   return layout(nullptr, n_pose).total;
 }
 
-cudaError_t pose_cells(KRun *R, void *work, int *grid, cudaStream_t s) {
+cudaError_t pose_cells(KRun *R, void *work, int *grid, int *launches, cudaStream_t s) {
   const int n = R->n_pose, cells = max_cells(n);
   const Work w = layout(static_cast<unsigned char *>(work), n);
+  R->pose_grid = w.grid;
+  R->pose_order = w.order;
+  R->pose_cell = w.block_cell;
+  R->cell_first = w.first;
+  R->cell_count = w.count;
+  *grid = max_blocks(n);
+  if (n <= kSmallPoses) {
+    *launches = 1;
+    small_kernel<<<1, 1024, 0, s>>>(R->poses, n, cells, w.grid, w.count, w.first, w.order,
+                                    w.block_cell);
+    return cudaGetLastError();
+  }
+  *launches = 4;
   cudaError_t e = cudaMemsetAsync(work, 0, w.zero, s);
   if (e != cudaSuccess) return e;
   const int blocks = (n + kThreads - 1) / kThreads;
@@ -207,12 +296,6 @@ cudaError_t pose_cells(KRun *R, void *work, int *grid, cudaStream_t s) {
   cell_kernel<<<blocks, kThreads, 0, s>>>(R->poses, n, cells, w.box, w.grid, w.count, w.at);
   scan_kernel<<<1, 1024, 0, s>>>(w.grid, w.count, w.first);
   order_kernel<<<blocks, kThreads, 0, s>>>(n, w.at, w.first, w.order, w.block_cell);
-  R->pose_grid = w.grid;
-  R->pose_order = w.order;
-  R->pose_cell = w.block_cell;
-  R->cell_first = w.first;
-  R->cell_count = w.count;
-  *grid = max_blocks(n);
   return cudaGetLastError();
 }
 

@@ -27,9 +27,9 @@ def _check(cx, poses, terms, raw, pick):
     assert not bad.any(), np.nanmax(rel, axis=0)
 
 
-# 2,500 x 50: cells from 4,096 poses on; pose counts at the edges of blocks
-# and of the rule; boxes of one cell and of many
-@pytest.mark.parametrize("n", [4096, 4097, 9000, 20001])
+# 2,500 x 50: cells from 2,048 poses on, in one launch up to 16,384; pose counts
+# at the edges of blocks and of the rule; boxes of one cell and of many
+@pytest.mark.parametrize("n", [2047, 2048, 4097, 16384, 16385, 20001])
 @pytest.mark.parametrize("box", [0.0, 6.0, 40.0])
 def test_pose_cells(ctx, n, box):
     cx = synth.make_complex(synth.ComplexSpec(pnp=2500, lna=50), seed=95)
