@@ -577,66 +577,11 @@ extern "C" gd_status gd_complex_free(gd_dcomplex *d) {
 
 extern "C" size_t gd_complex_device_bytes(const gd_dcomplex *d) { return d ? d->bytes : 0; }
 
-// The device order of the points: those whose type forms an H-bond with
-// some ligand type (hdb0 > 0.1) first, each kind in two zones about the
-// pocket: the points within kNearZone, which a ligand in the pocket is mostly
-// near to (its size plus the distance from which the far form holds, about
-// 16 A), then the others by distance, so that a 32-point chunk's points are
-// mostly all near or all far.  The near zone's points are dealt over its
-// half chunks, so that each holds its share of the closest ones, whose
-// close-range terms cost most.  The chunks of both kinds, nearest first, are then dealt
-// over the tiles (and over the chunk positions of a tile), so that every
-// tile, and every tile group's chunks, hold the same mix: a split unit's CTAs
-// and a CTA's tile groups wait for the slowest.  The energy is a sum over
-// points, so the order changes nothing but the FP32 rounding inside a chunk.
-static void order_points(const gd_protein &P, const bool *hb_type, std::vector<int> *out) {
-  const int pnp = P.pnp, chunk = 32, per_tile = TILE_PTS / chunk;
-  const float kNearZone = 24.0f;
-  std::vector<float> key(pnp);  // squared distance from the pocket
-  for (int p = 0; p < pnp; ++p) {
-    const float dx = P.x[p] - P.pocket_center[0], dy = P.y[p] - P.pocket_center[1];
-    const float dz = P.z[p] - P.pocket_center[2];
-    const float d2 = dx * dx + dy * dy + dz * dz;
-    key[p] = d2 < 3.0e38f ? d2 : 3.0e38f;  // also orders NaN
-  }
-  std::vector<int> order, zone;
-  order.reserve(pnp);
-  for (int pass = 0; pass < 2; ++pass) {
-    zone.clear();
-    for (int p = 0; p < pnp; ++p)
-      if (hb_type[P.t[p]] == (pass == 0)) zone.push_back(p);
-    std::stable_sort(zone.begin(), zone.end(), [&](int a, int b) { return key[a] < key[b]; });
-    int near = 0;
-    while (near < (int)zone.size() && key[zone[near]] < kNearZone * kNearZone) ++near;
-    // in runs of two: packed lanes take several points at a time
-    const int half = chunk / 2, run = 2, nr = near / run;
-    const int nc = std::max(1, near / half);
-    for (int c = 0; c < nc; ++c)
-      for (int r = c; r < nr; r += nc)
-        order.insert(order.end(), zone.begin() + r * run, zone.begin() + (r + 1) * run);
-    order.insert(order.end(), zone.begin() + nr * run, zone.begin() + near);
-    order.insert(order.end(), zone.begin() + near, zone.end());
-  }
-  // whole chunks by their middle point; the points past them stay last
-  const int full = pnp / chunk, tiles = (full + per_tile - 1) / per_tile;
-  std::vector<int> rank(full);
-  for (int c = 0; c < full; ++c) rank[c] = c;
-  std::stable_sort(rank.begin(), rank.end(), [&](int a, int b) {
-    return key[order[a * chunk + chunk / 2]] < key[order[b * chunk + chunk / 2]];
-  });
-  out->resize(pnp);
-  int next = 0;
-  for (int q = 0; q < per_tile; ++q)
-    for (int t = 0; t < tiles; ++t) {
-      const int pos = t * per_tile + (q + t) % per_tile;
-      if (pos >= full) continue;
-      std::copy_n(order.begin() + rank[next] * chunk, chunk, out->begin() + pos * chunk);
-      ++next;
-    }
-  std::copy(order.begin() + full * chunk, order.end(), out->begin() + full * chunk);
-}
-
 // Packs the protein conformations into {x, y, z, ele} and {hpp, meta}.
+// The device order of the points: those whose type forms an H-bond with
+// some ligand type (hdb0 > 0.1) first, each kind in the caller's order.  The
+// energy is a sum over points, so the order changes nothing but the FP32
+// rounding inside a 32-point chunk.
 static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, TableUpload &U) {
   gd_dcomplex *d = U.d;
   KTables &T = d->T;
@@ -648,7 +593,11 @@ static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, TableU
     for (int i = 0; i < GD_NLT; ++i) hb_type[j] = hb_type[j] || F.hdb0[i][j] > 0.1f;
   }
   std::vector<int> &order = d->point_order;
-  order_points(P, hb_type, &order);
+  order.clear();
+  order.reserve(pnp);
+  for (int pass = 0; pass < 2; ++pass)
+    for (int p = 0; p < pnp; ++p)
+      if (hb_type[P.t[p]] == (pass == 0)) order.push_back(p);
   std::vector<float4> pa((size_t)P.n_conf * pnp_pad,
                          make_float4(PAD_POINT_COORD, PAD_POINT_COORD, PAD_POINT_COORD, 0.f));
   for (int c = 0; c < P.n_conf; ++c)

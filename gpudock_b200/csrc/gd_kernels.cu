@@ -47,9 +47,9 @@ constexpr int CHUNK = 32;  // points per FP32 partial before the FP64 flush
 // up to two atom pairs, the shorter far loop up to four (packed lanes have few
 // points per loop).  Near / far points per iteration, NH = 4: 131,072 poses x 48
 // x 2,000 in 13.0 (1 / 1), 12.8 (1 / 2), 13.4 (2 / 1), 13.9 ms (2 / 2); 65,536 x
-// 48 x 16,000 in 36.7, 34.4, 35.5, 34.1 ms.  NH = 5, headline interval: 22.4 (1
-// / 1), 23.4 (2 / 1), 26.2 ms (2 / 2; ncu's no-instruction stall 0.17, 0.37,
-// 0.87 per issue).
+// 48 x 16,000 in 36.7, 34.4, 35.5, 34.1 ms.  NH = 5 (MC steps with these loops,
+// 20-step interval of the headline): 22.4 (1 / 1), 23.4 (2 / 1), 26.2 ms (2 / 2;
+// ncu's no-instruction stall 0.17, 0.37, 0.87 per issue).
 __host__ __device__ constexpr int near_unroll(int NH) { return NH <= 2 ? 2 : 1; }
 __host__ __device__ constexpr int far_unroll(int NH, bool packed) {
   return NH <= 2 || (NH <= 4 && !packed) ? 2 : 1;
@@ -104,7 +104,8 @@ struct SlotKde {
 //   far[ag][pt]  = the distance from which every atom of the group takes the
 //                  far form with point type pt
 //   fpmf[ag][pt] = the sum of the group's pmf1 with it (the PMF term there)
-//   list[warp]   = the points of the warp's current chunk, near ones first:
+//   list[warp]   = (poses, packed lanes) the points of the warp's current
+//                  chunk, near ones first:
 //                  {offset of its record in shared memory | point type << 23
 //                  (list_entry), threshold of its close-range vote}
 //   pad          = the record of a padding point (fills up the lists)
@@ -641,6 +642,95 @@ __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (
   }
 }
 
+// One point beyond far[ag][pt] of every atom of the warp in every lane, as
+// pair_block1 evaluates it to the bit: there 2^x < 2^-25, so D1 D2 rounds to D1
+// and num1 D2 to num1, the H-bond Gaussian vanishes in its sum and no close-range
+// term applies; 17 packed FMA-pipe and 4 MUFU instructions per atom pair against
+// its 22 and 6.
+template <int NH>
+__device__ __forceinline__ void far_block1(const float2 (&nx)[NH], const float2 (&ny)[NH],
+                                           const float2 (&nz)[NH], const float4 &A0,
+                                           const float4 *pp, const PairConst &K, float2 &fvdw,
+                                           float2 &fpmf, float2 (&fek)[NH]) {
+  float2 d2[NH], r[NH], den[NH], num[NH], pm[NH];
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    const float2 dx = add2(dup2(A0.x), nx[h]);
+    const float2 dy = add2(dup2(A0.y), ny[h]);
+    const float2 dz = add2(dup2(A0.z), nz[h]);
+    d2[h] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+    r[h] = make_float2(frsqrt(d2[h].x), frsqrt(d2[h].y));
+  }
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    const float4 T0 = pp[h * 2 * PT_ROWS];      // p1a, -p2a
+    const float4 T1 = pp[h * 2 * PT_ROWS + 1];  // -pmf0, pmf1
+    const float2 d = mul2(d2[h], r[h]);
+    const float2 g = mul2(d2[h], d);
+    const float2 g3 = mul2(mul2(g, g), g);
+    den[h] = fma2(lo2(T0), fma2(K.lj1, d2[h], K.lj0), g3);
+    num[h] = fma2(hi2(T0), g, lo2(T0));
+    pm[h] = mul2(hi2(T1), den[h]);
+    fek[h] = fma2(dup2(A0.w), r[h], fek[h]);
+  }
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    const float2 inv = make_float2(frcp(den[h].x), frcp(den[h].y));
+    fvdw = fma2(num[h], inv, fvdw);
+    fpmf = fma2(pm[h], inv, fpmf);
+  }
+}
+
+// The points j0 .. j1-1 of a tile in their order, each by far_block1 (far_m) or
+// pair_block1 with `var` of its H-bond variants (none, NHB1, NHB pairs): every
+// sum adds the same values in the same order whichever points are far, so an
+// MC trajectory does not depend on where its unit's other replicas are, and is
+// bit for bit the one that pair_block1 alone gives.  The pose kernels' lists
+// (near points first, the PMF of far ones added per chunk) take 8% less time on
+// the headline, but change the last bits of the sums and with them one
+// Metropolis decision in 300,000.  One point per iteration: four bodies share
+// the instruction caches.  20-step interval of the headline: 27.0 ms without
+// the far form, 23.8 with it (the points within 16 A of some atom of the warp
+// in some lane, 37 .. 50%, still take the full form).  Bound by issue and by
+// the XU and FMA pipes together.  Returns the mask of the points that some lane
+// has a close-range term with.
+template <int NH, int NHB1, int NHB>
+__device__ __forceinline__ uint32_t chunk_ordered(const float2 (&nx)[NH], const float2 (&ny)[NH],
+                                                  const float2 (&nz)[NH], const float4 *ta,
+                                                  const float2 *tb, int j0, int j1,
+                                                  uint32_t far_m, int var, const float4 *my_ptab,
+                                                  const float4 *my_htab, const PairConst &K,
+                                                  float thr_l, float2 &fvdw, float2 &fpmf,
+                                                  float2 &fhdb, float2 (&fek)[NH]) {
+  uint32_t close = 0u;
+  float4 Ap = ta[j0];  // read one point ahead
+  int pt = (int)(__float_as_uint(tb[j0].y) & META_TYPE_MASK);
+#pragma unroll 1
+  for (int j = j0; j < j1; ++j) {
+    const int jn = min(j + 1, j1 - 1);
+    const float4 An = ta[jn];
+    const int ptn = (int)(__float_as_uint(tb[jn].y) & META_TYPE_MASK);
+    const float4 *pp = my_ptab + pt * 2, *hp = my_htab + pt;
+    if (far_m & 1u) {
+      far_block1<NH>(nx, ny, nz, Ap, pp, K, fvdw, fpmf, fek);
+    } else {
+      float mn = 3.0e38f;
+      if (var == 0)
+        pair_block1<NH, 0>(nx, ny, nz, Ap, pp, hp, K, fvdw, fpmf, fhdb, fek, mn);
+      else if (var == 1)
+        pair_block1<NH, NHB1>(nx, ny, nz, Ap, pp, hp, K, fvdw, fpmf, fhdb, fek, mn);
+      else
+        pair_block1<NH, NHB>(nx, ny, nz, Ap, pp, hp, K, fvdw, fpmf, fhdb, fek, mn);
+      const float thr = __shfl_sync(0xffffffffu, thr_l, j - j0);
+      close |= (__any_sync(0xffffffffu, mn <= thr) ? 1u : 0u) << (j - j0);
+    }
+    far_m >>= 1;
+    Ap = An;
+    pt = ptn;
+  }
+  return close;
+}
+
 // Largest value, NaN if there is one: of two values, of a warp's lanes.
 __device__ __forceinline__ float max_nan(float a, float b) {
   float y;
@@ -835,7 +925,7 @@ __device__ __forceinline__ void close_range(const float2 (&nx)[NA / 2], const fl
 // persistent schedule (KRun.pieces, REMC only), else all steps of unit
 // blockIdx.x.  PACKED: units may have few replicas (KRun.packed); a kernel of
 // its own, since the distance between a lane's list entries as a variable
-// costs the pair loop 4% (headline interval 22.0 / 22.8 ms).
+// costs the pair loop 4%.
 // No producer warp: sm_100 splits the register file between the four
 // schedulers, so a 13th warp would put four warps on one scheduler and cap
 // every thread at 128 registers; 12 warps leave room for about 168.
@@ -844,6 +934,9 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     dock_kernel(const __grid_constant__ KRun R) {
   static_assert(NA % 2 == 0, "atoms are processed in pairs");
   constexpr int NH = NA / 2;
+  // poses and packed lanes list a chunk's points, near ones first; MC units
+  // keep their order (chunk_ordered)
+  constexpr bool kLists = PACKED || MODE == KMODE_POSES;
   static_assert(HB >= 0 && HB <= NH, "H-bond pair bound");
   extern __shared__ __align__(128) unsigned char smem[];
   const int A = R.A, P = R.P, W = A * P, NS = R.n_stages;
@@ -1070,10 +1163,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const int crank0 = csize > 1 ? cluster_rank() : 0;
   // A split unit's ranks take the protein's chunks in turn (rank r the chunks
   // r, r + split, ...), and stage their own chunks side by side in tiles.
-  // Chunks have half the points then: a rank has few, and the tile groups
-  // wait for the one that got one more (plain 1,500-point complex on 8 CTAs:
-  // whole tiles in turn left four CTAs with 256 points and four with 128).
-  const int cp = csize > 1 ? CHUNK / 2 : CHUNK;  // points of a chunk
+  // Packed lanes' chunks have half the points then: a rank has few, and the
+  // tile groups wait for the one that got one more (plain 1,500-point complex
+  // on 8 CTAs: whole tiles in turn left four CTAs with 256 points and four with
+  // 128).
+  const int cp = PACKED && csize > 1 ? CHUNK / 2 : CHUNK;  // points of a chunk
   const int cpt = TILE_PTS / cp;                 // chunks of a staged tile
   const int n_own = max(0, ((T.pnp + cp - 1) / cp - crank0 + csize - 1) / csize);  // of this CTA
   const int n_tl = (n_own + cpt - 1) / cpt;      // its staged tiles
@@ -1275,9 +1369,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll
     for (int k = 0; k < NA; ++k) {
       const float4 o = at0[k];
-      const float x = q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx;
-      const float y = q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy;
-      const float z = q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz;
+      // written as FMAs: which products the compiler contracts differs between
+      // kernel variants, and the energies' last bits with it
+      const float x = fmaf(q02, o.z, fmaf(q01, o.y, q00 * o.x)) + t0 + lcx;
+      const float y = fmaf(q12, o.z, fmaf(q11, o.y, q10 * o.x)) + t1 + lcy;
+      const float z = fmaf(q22, o.z, fmaf(q21, o.y, q20 * o.x)) + t2 + lcz;
       if (k & 1) {
         nx[k >> 1].y = -x;
         ny[k >> 1].y = -y;
@@ -1344,10 +1440,11 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         // (points are ordered so that chunks rarely mix the two kinds); the
         // close-range votes are collected in a mask and served after the
         // branch-free pass, so consecutive points' chains overlap
-        // lane j looks at point j: the warp lists the points that are not far
-        // of all its atoms in all lanes, then the far ones (the far form); of
-        // the former, those that can have a close-range term come first, so
-        // that packed lanes meet them in few iterations
+        // lane j looks at point j, whether it is far of all the warp's atoms in
+        // all lanes.  MC units of more than 16 replicas keep the points' order;
+        // with lists, the warp takes the points that are not far, then the far
+        // ones, and of the former those that can have a close-range term first,
+        // so that packed lanes meet them in few iterations
         const int jl = j0 + lane;
         const bool valid = jl < j1;
         const float2 pb_l = valid ? tb[jl] : make_float2(0.f, __uint_as_float(PAD_POINT_TYPE));
@@ -1364,9 +1461,18 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
             subs > 1 ? __ballot_sync(0xffffffffu, valid && !far_l && b2_l <= thr_l) : 0u;
         // (after the order, which is the same with the MCC score on)
         if (mcc_on) thr_l = fmaxf(thr_l, T.near_mcc2);
+        const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && my_hmask[pt_l] != 0u);
+        const int var = !chunk_hdb || my_nhb <= 0 ? 0 : my_nhb <= kHB1 ? 1 : 2;
+        int it_near = 1;
+        uint32_t close;
+        if constexpr (!kLists) {
+          close = chunk_ordered<NH, kHB1, HB>(nx, ny, nz, ta, tb, j0, j1, far_m, var, my_ptab,
+                                              my_htab, K, thr_l, fvdw, fpmf, fhdb, fek);
+        } else {
         // iterations of each part: a list entry for each subset
         const int n_near = __popc(near_m), n_far = __popc(far_m);
-        const int it_near = (n_near + subs - 1) / subs, it_far = (n_far + subs - 1) / subs;
+        const int it_far = (n_far + subs - 1) / subs;
+        it_near = (n_near + subs - 1) / subs;
         const int far0 = it_near * subs;
         const uint32_t below = (1u << lane) - 1u;
         __syncwarp();  // the previous chunk's list has been read
@@ -1387,8 +1493,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
           chunk_far<NH, PACKED>(nx, ny, nz, smem, my_list + far0 + sub, it_far, subs, my_ptab, K,
                                 fvdw, fek);
         }
+        close = 0u;
         if (it_near) {
-          const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && my_hmask[pt_l] != 0u);
           // three variants per kernel: no H-bond term, kHB1 pairs (warps that
           // need no more) and HB pairs; each is a long body, so more of them
           // would cost more in instruction fetch than they save
@@ -1397,9 +1503,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
                                                                it_near, subs, my_ptab, my_htab,
                                                                K, fvdw, fpmf, fhdb, fek);
           };
-          const uint32_t close = !chunk_hdb || my_nhb <= 0 ? near_part(Int<0>{})
-                                 : my_nhb <= kHB1          ? near_part(Int<kHB1>{})
-                                                           : near_part(Int<HB>{});
+          close = var == 0   ? near_part(Int<0>{})
+                  : var == 1 ? near_part(Int<kHB1>{})
+                             : near_part(Int<HB>{});
+        }
+        }
+        if (it_near) {
           if (close) {
             // the chunk's hydrophobic sums in registers, added to the per-atom
             // sums once per chunk
@@ -1408,12 +1517,18 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
             for (int h = 0; h < NH; ++h) hacc[h] = make_float2(0.f, 0.f);
             for (uint32_t m = close; m != 0u; m &= m - 1u) {
               // this lane's point of the iteration (a padding point has no term)
-              const uint32_t e = my_list[(__ffs(m) - 1) * subs + sub].x;
-              const int j = ((int)entry_at(e) - (int)tile_at) / 16;
-              const bool real = e != pad_entry.x;
+              int j = j0 + __ffs(m) - 1;
+              bool real = true;
+              float4 pa = ta[j];
+              if constexpr (kLists) {
+                const uint32_t e = my_list[(__ffs(m) - 1) * subs + sub].x;
+                j = ((int)entry_at(e) - (int)tile_at) / 16;
+                real = e != pad_entry.x;
+                pa = entry_point(smem, e);
+              }
               const float2 pb = real ? tb[j] : make_float2(0.f, __uint_as_float(PAD_POINT_TYPE));
               const uint32_t meta = __float_as_uint(pb.y);
-              close_range<NA>(nx, ny, nz, entry_point(smem, e), pb.x, meta,
+              close_range<NA>(nx, ny, nz, pa, pb.x, meta,
                               my_ptab + (int)(meta & META_TYPE_MASK) * 2, T, s_q, s_lt, s_atom,
                               hacc, A, ag, n_my, inv_el1, fnear, fpsp, mcc_on, p0 + j - j0,
                               my_red);
@@ -1465,9 +1580,9 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     // from beyond the first instruction cache.
     double dkde = 0.0, dlhm = 0.0;
     auto placed = [&](const float4 &o) {
-      return make_float3(q00 * o.x + q01 * o.y + q02 * o.z + t0 + lcx,
-                         q10 * o.x + q11 * o.y + q12 * o.z + t1 + lcy,
-                         q20 * o.x + q21 * o.y + q22 * o.z + t2 + lcz);
+      return make_float3(fmaf(q02, o.z, fmaf(q01, o.y, q00 * o.x)) + t0 + lcx,
+                         fmaf(q12, o.z, fmaf(q11, o.y, q10 * o.x)) + t1 + lcy,
+                         fmaf(q22, o.z, fmaf(q21, o.y, q20 * o.x)) + t2 + lcz);
     };
 #pragma unroll 1
     for (int i = crank0 + csize * lw; i < lna + T.pos; i += csize * W) {
@@ -1498,8 +1613,10 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
           Mn = Mm[min(l + subs, lna - 1)];  // one atom ahead
           on = orig[min(l + subs, lna - 1)];
           if (M.w != 0.0f) {
-            const float3 x = placed(o);
-            const float dx = x.x - M.x, dy = x.y - M.y, dz = x.z - M.z;
+            const float x = fmaf(q02, o.z, fmaf(q00, o.x, q01 * o.y)) + t0 + lcx;
+            const float y = fmaf(q12, o.z, fmaf(q10, o.x, q11 * o.y)) + t1 + lcy;
+            const float z = fmaf(q22, o.z, fmaf(q20, o.x, q21 * o.y)) + t2 + lcz;
+            const float dx = x - M.x, dy = y - M.y, dz = z - M.z;
             sv += fmaf(dz, dz, fmaf(dy, dy, dx * dx));
           }
         }
