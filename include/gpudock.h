@@ -390,7 +390,7 @@ gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *dcx, int prt_conf,
  * allocator) can see even a small cudaMalloc/cudaMallocAsync fail, and a
  * caller may want no allocator call at all on its scoring path. This entry
  * point stages poses, results and the launch descriptor in one fixed
- * device array compiled into the library (about 2.2 MB per device) instead.
+ * device array compiled into the library (about 2.5 MB per device) instead.
  *
  * Limit: n_pose <= GD_NOALLOC_MAX_POSES; larger calls return GD_EINVAL
  * before anything runs (split them, or use gd_energy_poses).  An empty call
