@@ -14,7 +14,7 @@
 //             against the points near the ligand's box; the contacts go into
 //             the union of all maps, their number is kept;
 //   rank      the number of union bits below each word of the union;
-//   maps      the contacts again, now as bits numbered by their rank;
+//   maps      the contacts as bits numbered by their rank;
 //   pairs     64 x 64 tiles of (i, j), i <= j: popc(A & B) over the maps'
 //             words through shared memory, then both entries' MCC.
 // Placement and distances follow the reference's float operations in its
@@ -49,6 +49,11 @@ constexpr int kPairChunk = 32;  // words per shared-memory chunk
 
 constexpr int kCandidates = 2048;  // points looked at per round
 constexpr int kRowWords = 8192;    // largest map kept in shared memory
+// Contacts of a conformation kept from the first pass for the second (a
+// conformation with more is tested again), while the lists of all take at most
+// kListBytes.
+constexpr int kListed = 2048;
+constexpr size_t kListBytes = 32 << 20;
 
 // The largest float whose correctly rounded square root is at most p (-1:
 // none).
@@ -72,14 +77,14 @@ __global__ void bound_kernel(const float4 *tab, float *bound) {
 // Contacts of conformation blockIdx.x.  MAPS = false: into the union's bits
 // (contact l * pnp + s of atom l and point s), and their number.  MAPS = true:
 // as the conformation's map of Kp words, bits numbered by the contact's rank
-// in the union.  Bound by latency and L2 reads of the points: the atoms are
-// tested against the few points within reach of the ligand's box (600
-// conformations x 40 x 4,000: 27 us a pass; testing every pair took 227 us).
-// The second pass costs less than keeping every conformation's contacts.
+// in the union, from the list that the first pass kept, or tested again.  Bound
+// by latency and L2 reads of the points: the atoms are tested against the few
+// points within reach of the ligand's box (600 conformations x 40 x 4,000: 27 us;
+// testing every pair took 227 us).
 template <bool MAPS>
 __global__ void __launch_bounds__(kSimThreads)
     contacts_kernel(KTables T, const SimConf *confs, const float *bound, uint32_t *uni, int *pop,
-                    const int *base, uint32_t *maps, int Kp) {
+                    const int *base, uint32_t *maps, int Kp, uint32_t *listed) {
   extern __shared__ float4 s_lig[];  // placed atoms, ligand type in .w; the map's words
   uint32_t *s_row = reinterpret_cast<uint32_t *>(s_lig + T.lna);
   __shared__ float s_bound[GD_NLT * 32];
@@ -90,6 +95,28 @@ __global__ void __launch_bounds__(kSimThreads)
   const int lna = T.lna, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool row = MAPS && Kp <= kRowWords;
   uint32_t *out = MAPS ? maps + (size_t)blockIdx.x * Kp : nullptr;
+  uint32_t *ids = listed ? listed + (size_t)blockIdx.x * kListed : nullptr;
+  auto set_bit = [&](uint32_t id) {
+    const uint32_t bit = 1u << (id & 31u);
+    const int r = base[id >> 5] + __popc(uni[id >> 5] & (bit - 1u));
+    if (row)
+      atomicOr(&s_row[r >> 5], 1u << (r & 31));
+    else
+      atomicOr(&out[r >> 5], 1u << (r & 31));
+  };
+  if (MAPS && ids && pop[blockIdx.x] <= kListed) {
+    const int n = pop[blockIdx.x];
+    if (row) {
+      for (int i = threadIdx.x; i < Kp; i += kSimThreads) s_row[i] = 0u;
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < n; i += kSimThreads) set_bit(ids[i]);
+    if (row) {
+      __syncthreads();
+      for (int i = threadIdx.x; i < Kp; i += kSimThreads) out[i] = s_row[i];
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < GD_NLT * 32; i += kSimThreads) s_bound[i] = bound[i];
   if (row)
     for (int i = threadIdx.x; i < Kp; i += kSimThreads) s_row[i] = 0u;
@@ -123,7 +150,6 @@ __global__ void __launch_bounds__(kSimThreads)
     hi[k] = __uint_as_float(b & 0x80000000u ? b & 0x7fffffffu : ~b);
   }
   const float4 *P = T.pt_a + (size_t)c.prt * T.pnp_pad;
-  int my_pop = 0;
   for (int s0 = 0; s0 < T.pnp; s0 += kCandidates) {
     const int s1 = min(T.pnp, s0 + kCandidates);
     // points within reach (near_mcc2: the largest pmf0 squared, with margin)
@@ -150,26 +176,33 @@ __global__ void __launch_bounds__(kSimThreads)
       const int s = s0 + s_cand[q];
       const float4 p = P[s];
       const int pt = (int)(__float_as_uint(T.pt_b[s].y) & META_TYPE_MASK);
-      for (int l = lane; l < lna; l += 32) {
-        const float4 a = s_lig[l];
-        const float dx = __fsub_rn(a.x, p.x);
-        const float dy = __fsub_rn(a.y, p.y);
-        const float dz = __fsub_rn(a.z, p.z);
-        const float d2 =
-            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-        if (!(d2 <= s_bound[__float_as_int(a.w) * 32 + pt])) continue;
-        const size_t id = (size_t)l * T.pnp + s;
-        const uint32_t bit = 1u << (id & 31);
-        if (!MAPS) {
-          ++my_pop;
+      for (int l0 = 0; l0 < lna; l0 += 32) {
+        const int l = l0 + lane;
+        bool hit = false;
+        if (l < lna) {
+          const float4 a = s_lig[l];
+          const float dx = __fsub_rn(a.x, p.x);
+          const float dy = __fsub_rn(a.y, p.y);
+          const float dz = __fsub_rn(a.z, p.z);
+          const float d2 =
+              __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+          hit = d2 <= s_bound[__float_as_int(a.w) * 32 + pt];
+        }
+        const uint32_t id = (uint32_t)l * (uint32_t)T.pnp + (uint32_t)s;
+        if (MAPS) {
+          if (hit) set_bit(id);
+          continue;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (m == 0u) continue;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s_pop, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+        if (hit) {
+          const uint32_t bit = 1u << (id & 31u);
           // most contacts are in the union already
           if (!(__ldcg(&uni[id >> 5]) & bit)) atomicOr(&uni[id >> 5], bit);
-        } else {
-          const int r = base[id >> 5] + __popc(uni[id >> 5] & (bit - 1u));
-          if (row)
-            atomicOr(&s_row[r >> 5], 1u << (r & 31));
-          else
-            atomicOr(&out[r >> 5], 1u << (r & 31));
+          if (ids && at < kListed) ids[at] = id;
         }
       }
     }
@@ -178,9 +211,6 @@ __global__ void __launch_bounds__(kSimThreads)
     __syncthreads();
   }
   if (!MAPS) {
-    my_pop = __reduce_add_sync(0xffffffffu, my_pop);
-    if (lane == 0 && my_pop) atomicAdd(&s_pop, my_pop);
-    __syncthreads();
     if (threadIdx.x == 0) pop[blockIdx.x] = s_pop;
   } else if (row) {
     for (int i = threadIdx.x; i < Kp; i += kSimThreads) out[i] = s_row[i];
@@ -412,11 +442,14 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
     uint32_t *d_uni = nullptr, *d_maps = nullptr;
     float *d_bound = nullptr, *d_S = nullptr;
     int *d_pop = nullptr, *d_base = nullptr;
+    uint32_t *d_listed = nullptr;
     cudaError_t e = B.get(&d_conf, n);
     if (e == cudaSuccess) e = B.get(&d_uni, K);
     if (e == cudaSuccess) e = B.get(&d_bound, (size_t)GD_NLT * 32);
     if (e == cudaSuccess) e = B.get(&d_pop, n);
     if (e == cudaSuccess) e = B.get(&d_base, K + 1);
+    if (e == cudaSuccess && n * kListed * sizeof(uint32_t) <= kListBytes)
+      e = B.get(&d_listed, n * kListed);
     if (e == cudaSuccess && !S_dev) e = B.get(&d_S, n * n);
     if (S_dev) d_S = S_dev;
     if (e != cudaSuccess) return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
@@ -425,7 +458,7 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
     bound_kernel<<<(GD_NLT * 32 + 255) / 256, 256, 0, s>>>(T.tab_a, d_bound);
     GD_CUDA(cudaGetLastError());
     contacts_kernel<false><<<n_conf, kSimThreads, sizeof(float4) * T.lna, s>>>(
-        T, d_conf, d_bound, d_uni, d_pop, nullptr, nullptr, 0);
+        T, d_conf, d_bound, d_uni, d_pop, nullptr, nullptr, 0, d_listed);
     GD_CUDA(cudaGetLastError());
     rank_kernel<<<1, 1024, 0, s>>>(d_uni, (int)K, d_base);
     GD_CUDA(cudaGetLastError());
@@ -441,7 +474,7 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
       if (!row) GD_CUDA(cudaMemsetAsync(d_maps, 0, sizeof(uint32_t) * n * Kp, s));
       contacts_kernel<true><<<n_conf, kSimThreads,
                               sizeof(float4) * T.lna + (row ? sizeof(uint32_t) * Kp : 0), s>>>(
-          T, d_conf, d_bound, d_uni, d_pop, d_base, d_maps, Kp);
+          T, d_conf, d_bound, d_uni, d_pop, d_base, d_maps, Kp, d_listed);
       GD_CUDA(cudaGetLastError());
     }
     const int tiles = (n_conf + kPairTile - 1) / kPairTile;
