@@ -973,7 +973,11 @@ extern "C" gd_status gd_energy_poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int 
   GD_CUDA(cudaSetDevice(ctx->device));
   void *work = nullptr;
   const size_t bytes = pose_work_bytes(d->T, n_pose);
-  if (bytes) GD_CUDA(work_alloc(ctx, &work, bytes));
+  // without room for the cells' workspace the call runs without them
+  if (bytes && work_alloc(ctx, &work, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    work = nullptr;
+  }
   const gd_status st =
       poses_launch(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, work);
   if (work) cudaFreeAsync(work, ctx->stream);

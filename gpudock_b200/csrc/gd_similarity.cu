@@ -448,8 +448,11 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
     if (e == cudaSuccess) e = B.get(&d_bound, (size_t)GD_NLT * 32);
     if (e == cudaSuccess) e = B.get(&d_pop, n);
     if (e == cudaSuccess) e = B.get(&d_base, K + 1);
-    if (e == cudaSuccess && n * kListed * sizeof(uint32_t) <= kListBytes)
-      e = B.get(&d_listed, n * kListed);
+    if (e == cudaSuccess && n * kListed * sizeof(uint32_t) <= kListBytes &&
+        B.get(&d_listed, n * kListed) != cudaSuccess) {
+      cudaGetLastError();  // without room for the lists the contacts are tested twice
+      d_listed = nullptr;
+    }
     if (e == cudaSuccess && !S_dev) e = B.get(&d_S, n * n);
     if (S_dev) d_S = S_dev;
     if (e != cudaSuccess) return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));

@@ -347,13 +347,14 @@ gd_status gd_ctx_set_schedule_tail(gd_ctx *ctx, int tail);
 
 /* How many CTAs share each 32-replica unit of an MC launch.  With split > 1
  * the unit runs on a thread-block cluster of `split` CTAs (SMs of one GPC):
- * CTA r evaluates the protein tiles r, r + split, ..., the CTAs add their
+ * CTA r evaluates every split-th chunk of the protein, the CTAs add their
  * partial energies through distributed shared memory every MC step (in
  * rank order) and all take the same decision.  A complex's run then takes
  * about 1/split of the time when SMs are free (latency), at a few percent
  * more total work.  split = 0 (the default) chooses per complex from its
- * size and its own run: the largest power of two <= ligand-size bucket x
- * protein points / c and <= SMs / units of the run, at most 8, with
+ * size and its own run: a power of two <= ligand-size bucket x protein
+ * points / c, at most 8; a run or batch splits the complexes with the most
+ * work per CTA first, while its CTAs fit on the SMs at once.
  * c = 4,500 for runs and batches (they have the GPU to themselves: a
  * 24-atom ligand against 1,500 points runs on 8 CTAs, an ensemble or batch
  * with more units than SMs unsplit) and c = 42,500 for server requests
