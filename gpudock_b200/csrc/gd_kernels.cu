@@ -3,15 +3,16 @@
 // dock_kernel: one CTA owns up to 32 replicas (or poses) of one complex that
 // share one protein conformation; lane i of every compute warp is replica i,
 // so protein-point and type-table reads are warp-uniform shared-memory
-// broadcasts.  The compute warps form an A x P grid: warp (ag, pg) (warp
-// number pg + P ag) keeps NA ligand atoms a = ag + A k in registers and
-// sweeps the protein tiles t = pg, pg + P, ...  The protein conformation is staged in shared memory in
-// 128-point tiles by the TMA engine (cp.async.bulk + mbarrier), once per
-// launch when it fits (resident) or through an 8-stage ring that the last
-// warp to finish a stage refills (then P = 1).  Per step every warp writes
-// FP64 partial sums
-// per replica; warp 0 reduces them in a fixed order, normalises the terms
-// and takes the Metropolis decision with the counter-based RNG.
+// broadcasts (a unit of at most 16 replicas holds them several times over and
+// its lane groups share the points).  The compute warps form an A x P grid:
+// warp (ag, pg) (warp number pg + P ag) keeps NA ligand atoms a = ag + A k in
+// registers and sweeps the protein's chunks c = pg, pg + P, ...  The protein
+// conformation is staged in shared memory in 128-point tiles by the TMA engine
+// (cp.async.bulk + mbarrier), once per launch when it fits (resident) or
+// through an 8-stage ring that the last warp to finish a stage refills.  Per
+// step every warp writes FP64 partial sums per replica; the warps add them in
+// a fixed order, and warp 0 normalises the terms and takes the Metropolis
+// decision with the counter-based RNG.
 //
 // Per ligand-protein pair the fast path evaluates the terms every pair
 // contributes to (soft LJ, far-field electrostatics, contact PMF) with one
@@ -19,7 +20,8 @@
 // (hydrophobic contact d <= 9 A, near-field electrostatics d < 1/el1,
 // pocket-specific potential d <= pmf0) run only when some lane has an atom
 // within near_d2 of the point; the H-bond term runs for the type pairs that
-// define one.
+// define one.  Points beyond the type pairs' far distance (about 16 A) of all
+// atoms of a warp in all lanes take a shorter form (far_block1, chunk_far).
 //
 // Reference semantics (gpudocksm-rem-1.2/src):
 //   pair terms          calcenergy_d.cu:56-138
