@@ -262,10 +262,6 @@ __device__ __forceinline__ float contact_mcc(int tp, int fn, int fp, int tn) {
   return dividend != 0.0f ? __fdiv_rn(__int2float_rn(num), dividend) : GD_CMCC_INVALID;
 }
 
-// Entries of the matrix.  With a bit per contact of the union, in place of the
-// 32-bit words that hold one, the maps are several times shorter: 600
-// conformations 145 -> 17 us, 3,001 (upper triangle only) 9.3 -> 0.66 ms for the
-// whole call.  Bound by the ALU pipe (carry-save counting).
 // Tile pair t of the upper triangle of tiles x tiles: its row and column.
 __device__ __forceinline__ void tile_of(int t, int tiles, int *row, int *col) {
   // row r starts at r tiles - r (r - 1) / 2
@@ -279,6 +275,10 @@ __device__ __forceinline__ void tile_of(int t, int tiles, int *row, int *col) {
   *col = r + (int)(t - start(r));
 }
 
+// Entries of the matrix.  With a bit per contact of the union, in place of the
+// 32-bit words that hold one, the maps are several times shorter: 600
+// conformations 145 -> 17 us, 3,001 (upper triangle only) 9.3 -> 0.66 ms for the
+// whole call.  Bound by the ALU pipe (carry-save counting).
 __global__ void __launch_bounds__(kSimThreads)
     pairs_kernel(const uint32_t *comp, const int *pop, int n, int Kp, int total, int tiles,
                  float *S) {
