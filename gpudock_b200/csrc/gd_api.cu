@@ -19,8 +19,10 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include "gd_common.h"
+#include "gd_shared.h"
 
 using namespace gd;
 
@@ -125,91 +127,90 @@ Tile tile_for(gd_ctx *ctx, const KTables &T) {
   return default_tile(hi);
 }
 
-// Pinned blocks of the contexts.  Pinning memory takes 1 .. 3 ms up to 1 MB, so
-// the first context pins blocks for kPinnedSlots contexts at once; they are
-// unpinned with the last of them.  Contexts beyond that pin their own.
-static constexpr size_t kPinnedBlock = 256 + kStageBytes;
-static constexpr int kPinnedSlots = 4;
-static std::mutex g_pinned_mu;
-static unsigned char *g_pinned = nullptr;
-static unsigned g_pinned_used = 0;  // a bit per block
-
-static cudaError_t pinned_acquire(void **p) {
-  std::lock_guard<std::mutex> g(g_pinned_mu);
-  if (!g_pinned) {
-    const cudaError_t e = cudaHostAlloc((void **)&g_pinned, kPinnedBlock * kPinnedSlots,
-                                        cudaHostAllocPortable);
-    if (e != cudaSuccess) {
-      g_pinned = nullptr;
-      return e;
-    }
+// The runtime behind the contexts' shared blocks and pools (gd_shared.h).
+struct CudaShared {
+  using Error = cudaError_t;
+  using Pool = cudaMemPool_t;
+  static bool ok(Error e) { return e == cudaSuccess; }
+  // Serial number of the device's CUDA context, which no later one of the
+  // process has (0: this driver does not tell).
+  static uint64_t serial() {
+    static const std::pair<PFN_cuCtxGetCurrent_v4000, PFN_cuCtxGetId_v12000> fn = [] {
+      void *cur = nullptr, *id = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &cur, 4000, cudaEnableDefault, &q) !=
+          cudaSuccess)
+        cur = nullptr;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &id, 12000, cudaEnableDefault, &q) !=
+          cudaSuccess)
+        id = nullptr;
+      cudaGetLastError();
+      return std::make_pair((PFN_cuCtxGetCurrent_v4000)cur, (PFN_cuCtxGetId_v12000)id);
+    }();
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!fn.first || !fn.second || fn.first(&c) != CUDA_SUCCESS || !c ||
+        fn.second(c, &id) != CUDA_SUCCESS)
+      return 0;
+    return (uint64_t)id + 1;
   }
-  for (int k = 0; k < kPinnedSlots; ++k)
-    if (!(g_pinned_used >> k & 1u)) {
-      g_pinned_used |= 1u << k;
-      *p = g_pinned + (size_t)k * kPinnedBlock;
-      return cudaSuccess;
-    }
-  return cudaHostAlloc(p, kPinnedBlock, cudaHostAllocPortable);
-}
-
-static void pinned_release(void *p) {
-  if (!p) return;
-  std::lock_guard<std::mutex> g(g_pinned_mu);
-  unsigned char *q = static_cast<unsigned char *>(p);
-  if (!g_pinned || q < g_pinned || q >= g_pinned + kPinnedBlock * kPinnedSlots) {
-    cudaFreeHost(p);
-    return;
-  }
-  g_pinned_used &= ~(1u << ((q - g_pinned) / kPinnedBlock));
-  if (g_pinned_used == 0) {
-    cudaFreeHost(g_pinned);
-    g_pinned = nullptr;
-  }
-}
-
-// The workspaces of calls come from one memory pool per device, shared by its
-// contexts (stream-ordered, so safe between them) and destroyed with the last
-// of them.  It keeps up to kKeepBytes mapped between calls; the device's default
-// pool unmaps at every synchronisation, which cost 50 .. 100 us per allocation,
-// and a pool's first allocation takes milliseconds, so contexts do not have one
-// each.
-struct WorkPool {
-  cudaMemPool_t pool = nullptr;
-  int users = 0;
-};
-static std::mutex g_work_mu;
-static std::map<int, WorkPool> g_work;  // by device
-
-static cudaError_t work_pool_acquire(int device, cudaMemPool_t *out) {
-  std::lock_guard<std::mutex> g(g_work_mu);
-  WorkPool &w = g_work[device];
-  if (!w.pool) {
+  static Error pin(void **p, size_t bytes) { return cudaHostAlloc(p, bytes, cudaHostAllocDefault); }
+  static void unpin(void *p) { cudaFreeHost(p); }
+  // The pool is stream-ordered, so safe between contexts.  It keeps up to
+  // kKeepBytes mapped between calls; the device's default pool unmaps at every
+  // synchronisation, which cost 50 .. 100 us per allocation.
+  static Error pool_create(int device, Pool *out) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     uint64_t keep = kKeepBytes;
-    cudaError_t e = cudaMemPoolCreate(&w.pool, &props);
-    if (e == cudaSuccess)
-      e = cudaMemPoolSetAttribute(w.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      if (w.pool) cudaMemPoolDestroy(w.pool);
-      w.pool = nullptr;
-      return e;
-    }
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess)
+      cudaMemPoolDestroy(pool);
+    else
+      *out = pool;
+    return e;
   }
-  w.users += 1;
-  *out = w.pool;
+  static void pool_destroy(Pool pool) { cudaMemPoolDestroy(pool); }
+};
+
+// Never destroyed: a handle may be released while the process ends.
+static DeviceShared<CudaShared> &shared() {
+  static auto *s = new DeviceShared<CudaShared>(256 + kStageBytes);
+  return *s;
+}
+
+// The context's error word, staging and pool.
+static cudaError_t shared_attach(gd_ctx *c) {
+  DeviceShared<CudaShared>::Lease *l = nullptr;
+  cudaError_t e = cudaErrorMemoryAllocation;
+  try {
+    l = new DeviceShared<CudaShared>::Lease;
+    e = shared().acquire(c->device, l);
+  } catch (const std::bad_alloc &) {
+  }
+  if (e != cudaSuccess) {
+    delete l;
+    return e;
+  }
+  c->shared = l;
+  c->pool = l->group->pool;
+  c->h_err = static_cast<int *>(l->block);
+  c->stage = static_cast<unsigned char *>(l->block) + 256;
+  std::memset(l->block, 0, 256);
   return cudaSuccess;
 }
 
-static void work_pool_release(int device) {
-  std::lock_guard<std::mutex> g(g_work_mu);
-  WorkPool &w = g_work[device];
-  if (--w.users > 0) return;
-  cudaMemPoolDestroy(w.pool);
-  w = WorkPool{};
+static void shared_detach(gd_ctx *c) {
+  auto *l = static_cast<DeviceShared<CudaShared>::Lease *>(c->shared);
+  if (!l) return;
+  shared().release(l);
+  delete l;
+  c->shared = nullptr;
 }
 
 void ctx_retain(gd_ctx *c) {
@@ -256,8 +257,7 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
-  work_pool_release(c->device);
-  pinned_release(c->h_err);
+  shared_detach(c);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -490,27 +490,17 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
     }
     c->own_stream = true;
   }
-  e = pinned_acquire((void **)&c->h_err);
+  e = shared_attach(c);
   if (e != cudaSuccess) {
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
-    return fail(GD_ENOMEM, "pinned host memory: %s", cudaGetErrorString(e));
+    return fail(GD_ENOMEM, "pinned host memory and memory pool: %s", cudaGetErrorString(e));
   }
-  std::memset(c->h_err, 0, 256);
-  e = work_pool_acquire(device, &c->pool);
-  if (e != cudaSuccess) {
-    pinned_release(c->h_err);
-    if (c->own_stream) cudaStreamDestroy(c->stream);
-    delete c;
-    return fail(GD_ENOMEM, "memory pool: %s", cudaGetErrorString(e));
-  }
-  c->stage = reinterpret_cast<unsigned char *>(c->h_err) + 256;
   // the fixed scratch of gd_energy_poses_noalloc is committed now, not on
   // that entry point's first call
   const gd_status st = noalloc_attach(c);
   if (st != GD_OK) {
-    work_pool_release(device);
-    pinned_release(c->h_err);
+    shared_detach(c);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return st;

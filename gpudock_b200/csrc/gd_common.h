@@ -84,8 +84,9 @@ struct gd_ctx {
   int *h_err = nullptr;
   unsigned char *stage = nullptr;
   // the calls' own workspaces (poses, similarity): the device's pool of this
-  // library (work_pool_acquire)
+  // library (gd_shared.h, where `shared` is this context's lease)
   cudaMemPool_t pool = nullptr;
+  void *shared = nullptr;
   std::mutex stage_mu;
   uint64_t launches = 0;
   int n_sm = 148;
