@@ -14,6 +14,7 @@
 // poses in block order.  Up to kSmallPoses poses, one launch of one CTA does
 // all of it (about 5 us).
 #include <algorithm>
+#include <climits>
 
 #include "gd_common.h"
 
@@ -27,6 +28,11 @@ constexpr float kFarOut = 4.0e3f;
 // the blocks' lanes are idle.
 constexpr int kPosesPerCell = 320;
 constexpr int kSmallPoses = 16384;
+// The most poses that are dealt: below it every index here is an int (a pose's
+// place in block order, and a grid-stride loop's step past the last pose).
+constexpr int kMostPoses = 1 << 30;
+static_assert((long long)kMostPoses + 32LL * (kMaxCells + 1) + 148LL * 4 * kThreads < INT_MAX,
+              "pose indexes");
 constexpr float kMinEdge = 0.75f;  // smaller cells gain little (the ligand is larger)
 
 int max_cells(int n_pose) { return std::max(1, std::min(kMaxCells, n_pose / kPosesPerCell)); }
@@ -268,7 +274,8 @@ size_t pose_work_bytes(const KTables &T, int n_pose) {
   // pairs/s): about 5% at 1e8 pairs for one launch, 3% at 5e8 for four.  Below
   // 2,048 poses a call's units are spread over the SMs in other ways
   // (pose_units).
-  if (n_pose < 2048 || (double)n_pose * T.lna * T.pnp < (n_pose <= kSmallPoses ? 1e8 : 5e8))
+  if (n_pose < 2048 || n_pose > kMostPoses ||
+      (double)n_pose * T.lna * T.pnp < (n_pose <= kSmallPoses ? 1e8 : 5e8))
     return 0;
   return layout(nullptr, n_pose).total;
 }
