@@ -745,10 +745,17 @@ __device__ __forceinline__ float warp_max(float x) {
   return y;
 }
 
+// Coordinates that the far form takes: finite, and so that d^9 between a point
+// and an atom does not overflow, since from there on the two forms differ.
+constexpr float kUsable = 5.0e3f;
+__device__ __forceinline__ bool usable_at(float x, float y, float z) {  // false for NaN
+  return fabsf(x) < kUsable && fabsf(y) < kUsable && fabsf(z) < kUsable;
+}
+
 // Where a warp's placed atoms are, over all lanes: the box of their
 // coordinates, its centre, and the largest distance of an atom from that.
-// Atoms without a usable position (not finite, or so far out that d^9
-// overflows) leave an unbounded region, which no point is far from.
+// Atoms without a usable position leave an unbounded region, which no point is
+// far from.
 struct Region {
   float3 lo, hi, mid;
   float rad;
@@ -788,11 +795,8 @@ __device__ __forceinline__ Region warp_region(const float2 (&nx)[NA / 2],
     r2 = fmaxf(r2, fmaxf(2 * h < n_my ? d2.x : 0.f, 2 * h + 1 < n_my ? d2.y : 0.f));
   }
   g.rad = sqrtf(warp_max(r2));
-  bool usable = true;  // false for NaN
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-    usable = usable && (lo[i] > hi[i] || (fabsf(lo[i]) < 5.0e3f && fabsf(hi[i]) < 5.0e3f));
-  if (!usable) {
+  const bool none = lo[0] > hi[0];
+  if (!none && !(usable_at(lo[0], lo[1], lo[2]) && usable_at(hi[0], hi[1], hi[2]))) {
     g.lo = make_float3(-big, -big, -big);
     g.hi = make_float3(big, big, big);
     g.rad = big;
@@ -816,10 +820,11 @@ __device__ __forceinline__ Region pose_region(const KRun &R, int unit, float cx,
   if (cell >= P.n_cells) return g;
   const int x = cell % P.n[0], y = cell / P.n[0] % P.n[1], z = cell / P.n[0] / P.n[1];
   const float m = P.margin;
-  g.lo = make_float3(cx + P.lo[0] + x * P.edge - m, cy + P.lo[1] + y * P.edge - m,
-                     cz + P.lo[2] + z * P.edge - m);
-  g.hi = make_float3(g.lo.x + P.edge + 2.f * m, g.lo.y + P.edge + 2.f * m,
-                     g.lo.z + P.edge + 2.f * m);
+  const float3 lo = make_float3(cx + P.lo[0] + x * P.edge - m, cy + P.lo[1] + y * P.edge - m,
+                                cz + P.lo[2] + z * P.edge - m);
+  const float3 hi = make_float3(lo.x + P.edge + 2.f * m, lo.y + P.edge + 2.f * m,
+                                lo.z + P.edge + 2.f * m);
+  if (usable_at(lo.x, lo.y, lo.z) && usable_at(hi.x, hi.y, hi.z)) g.lo = lo, g.hi = hi;
   return g;
 }
 
@@ -1399,10 +1404,10 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll
       for (int k = 0; k < NA; ++k)
         if (k < n_my)
-          reach = fmaxf(reach, fmaf(at0[k].z, at0[k].z, fmaf(at0[k].y, at0[k].y,
-                                                             at0[k].x * at0[k].x)));
+          reach = max_nan(reach, fmaf(at0[k].z, at0[k].z, fmaf(at0[k].y, at0[k].y,
+                                                               at0[k].x * at0[k].x)));
       reach = sqrtf(reach) * 1.0001f + 1e-3f;
-      if (!(reach < 5.0e3f)) reach = 3.0e38f;  // also NaN: nothing is far
+      if (!(reach < 0.2f * kUsable)) reach = 3.0e38f;  // also NaN: nothing is far
     }
     double far_pmf = 0.0;  // PMF of this lane's far points (every lane's replica)
 
@@ -1456,7 +1461,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
         const float4 p_l = ta[valid ? jl : j0];
         const float b2_l = box_dist2(G, p_l);
-        const bool far_l = valid && is_far(G, p_l, b2_l, my_far[pt_l] + reach);
+        const bool far_l = valid && usable_at(p_l.x, p_l.y, p_l.z) &&
+                           is_far(G, p_l, b2_l, my_far[pt_l] + reach);
         const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
         const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
         const uint32_t close_m =

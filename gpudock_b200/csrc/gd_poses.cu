@@ -6,8 +6,8 @@
 // Which points take the far form follows from the cell alone, never from the
 // other poses of the CTA, and the cells from the box of the call's
 // translations: a pose's energy does not depend on the order of the poses.
-// Poses without a usable translation (not finite, or beyond kFarOut) get a
-// cell of their own, for which no point is far.
+// Poses without a usable place (a value that is not finite, or a translation
+// beyond kFarOut) get a cell of their own, for which no point is far.
 //
 // Four short launches (about 12 us together): the box of the translations;
 // every pose's cell and its rank in it; the cells' first 32-pose blocks; the
@@ -83,10 +83,19 @@ __device__ __forceinline__ bool usable(const float t[3]) {
   return fabsf(t[0]) < kFarOut && fabsf(t[1]) < kFarOut && fabsf(t[2]) < kFarOut;
 }
 
+// The translation of a pose; not usable when an angle is not finite: its atoms
+// have no positions then.
+__device__ __forceinline__ void load_translation(const float *poses, int i, float t[3]) {
+  const float *m = poses + (size_t)i * 6;
+  t[0] = m[0], t[1] = m[1], t[2] = m[2];
+  if (!(isfinite(m[3]) && isfinite(m[4]) && isfinite(m[5]))) t[0] = INFINITY;
+}
+
 __global__ void __launch_bounds__(kThreads) box_kernel(const float *poses, int n, unsigned *box) {
   unsigned m[6] = {0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    const float t[3] = {poses[(size_t)i * 6], poses[(size_t)i * 6 + 1], poses[(size_t)i * 6 + 2]};
+    float t[3];
+    load_translation(poses, i, t);
     if (!usable(t)) continue;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -150,7 +159,8 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();
   const int i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
-  const float t[3] = {poses[(size_t)i * 6], poses[(size_t)i * 6 + 1], poses[(size_t)i * 6 + 2]};
+  float t[3];
+  load_translation(poses, i, t);
   const int cell = cell_of(g, t);
   at[i] = make_int2(cell, atomicAdd(&count[cell], 1));
 }
@@ -216,8 +226,7 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
   for (int j = 0; j < kEach; ++j) {
     const int i = j * 1024 + threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) t[j][k] = i < n ? poses[(size_t)i * 6 + k] : 0.f;
+    if (i < n) load_translation(poses, i, t[j]);
     if (i < n && usable(t[j])) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
