@@ -623,8 +623,10 @@ static gd_status upload_protein(const gd_protein &P, const gd_enepara &F, TableU
 // a point type j (infinity: never), each bound solved from the term itself:
 // - contact PMF pmf1 / (1 + e), e = exp((6 - d/2)(d - pmf0)): from where
 //   e <= exp(-18) < 2^-25, 1 + e rounds to 1 in FP32 and the term is pmf1;
-// - H-bond hdb1 exp(-h^2/2), h = (d - hdb0) hdb1: below 2^-40 of its peak
-//   from h = 7.46 on (the FP32 sum of the near terms no longer sees it);
+// - H-bond hdb1 exp(-h^2/2), h = (d - hdb0) hdb1: exactly zero in FP32 from
+//   h = 13.3 on (the argument of 2^x is below -127, and the kernel's 2^x gives 0
+//   below -126).  A bound at a small value would not do: a chunk whose other
+//   points have no H-bond term starts its sum at 0, and sees any value;
 // - near-field electrostatics (el1 d < 1), hydrophobic contact (9 A) and the
 //   contact tests (d <= pmf0) are over.
 static float far_distance(const gd_enepara &F, int i, int j, float max_pmf0) {
@@ -634,7 +636,7 @@ static float far_distance(const gd_enepara &F, int i, int j, float max_pmf0) {
   D = std::max(D, F.el1 > 0.f ? 1.0 / (double)F.el1 : inf);
   D = std::max(D, 0.5 * (12.0 + p0 + std::sqrt((12.0 - p0) * (12.0 - p0) + 144.0)));
   if (F.hdb0[i][j] > 0.1f)
-    D = std::max(D, F.hdb1[i][j] > 0.f ? (double)F.hdb0[i][j] + 7.46 / (double)F.hdb1[i][j] : inf);
+    D = std::max(D, F.hdb1[i][j] > 0.f ? (double)F.hdb0[i][j] + 13.3 / (double)F.hdb1[i][j] : inf);
   D = D * 1.0005 + 0.01;  // rounding of the distances compared with it
   return std::isfinite(p0) && D < 1e6 ? (float)D : std::numeric_limits<float>::infinity();
 }

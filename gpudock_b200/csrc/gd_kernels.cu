@@ -646,8 +646,7 @@ __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (
 
 // One point beyond far[ag][pt] of every atom of the warp in every lane, as
 // pair_block1 evaluates it to the bit: there 2^x < 2^-25, so D1 D2 rounds to D1
-// and num1 D2 to num1, the H-bond Gaussian vanishes in its sum and no close-range
-// term applies; 17 packed FMA-pipe and 4 MUFU instructions per atom pair against
+// and num1 D2 to num1, the H-bond Gaussian is 0 and no close-range term applies; 17 packed FMA-pipe and 4 MUFU instructions per atom pair against
 // its 22 and 6.
 template <int NH>
 __device__ __forceinline__ void far_block1(const float2 (&nx)[NH], const float2 (&ny)[NH],
