@@ -540,8 +540,6 @@ struct TableUpload {
 template <typename T>
 static gd_status upload(TableUpload &U, const std::vector<T> &h, const T **out) {
   const size_t n = std::max<size_t>(h.size(), 1) * sizeof(T);
-  if (injected_alloc_failure(U.d->ctx))
-    return fail(GD_ENOMEM, "cudaMallocAsync of %zu bytes: out of memory (injected)", n);
   const size_t o = (U.host.size() + 255) & ~size_t(255);
   U.host.resize(o + n);
   if (!h.empty()) std::memcpy(U.host.data() + o, h.data(), h.size() * sizeof(T));
@@ -551,12 +549,21 @@ static gd_status upload(TableUpload &U, const std::vector<T> &h, const T **out) 
 }
 
 static gd_status upload_finish(TableUpload &U) {
-  cudaStream_t s = U.d->ctx->stream;
+  gd_ctx *c = U.d->ctx;
+  const auto injected = [&] {
+    return fail(GD_ENOMEM, "cudaMallocAsync of %zu bytes: out of memory (injected)",
+                U.host.size());
+  };
   unsigned char *p = nullptr;
-  GD_CUDA(cudaMallocAsync((void **)&p, U.host.size(), s));
+  if (injected_alloc_failure(c)) return injected();
+  GD_CUDA(cudaMallocAsync((void **)&p, U.host.size(), c->stream));
   U.d->allocs.push_back(p);
-  GD_CUDA(cudaMemcpyAsync(p, U.host.data(), U.host.size(), cudaMemcpyHostToDevice, s));
-  for (const auto &x : U.at) *x.first = p + x.second;
+  for (const auto &x : U.at) {
+    // each table counts as an allocation: a failure with the memory taken
+    if (injected_alloc_failure(c)) return injected();
+    *x.first = p + x.second;
+  }
+  GD_CUDA(cudaMemcpyAsync(p, U.host.data(), U.host.size(), cudaMemcpyHostToDevice, c->stream));
   return GD_OK;
 }
 

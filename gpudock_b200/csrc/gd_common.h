@@ -129,10 +129,6 @@ void ctx_release(gd_ctx *c);
 void dcx_retain(gd_dcomplex *d);
 void dcx_release(gd_dcomplex *d);
 gd_status ctx_check(gd_ctx *c);
-// Stream-ordered workspace of a call (freed with cudaFreeAsync).
-inline cudaError_t work_alloc(gd_ctx *c, void **p, size_t bytes) {
-  return cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-}
 // Status for a nonzero kernel error word (KRun.err).
 gd_status kernel_error(int code);
 // Loads the module that holds the fixed pose-scratch array of
@@ -146,6 +142,11 @@ inline bool injected_alloc_failure(gd_ctx *c) {
   while (n > 0 && !c->alloc_fail_in.compare_exchange_weak(n, n - 1)) {
   }
   return n == 1;
+}
+// Stream-ordered workspace of a call (freed with cudaFreeAsync).
+inline cudaError_t work_alloc(gd_ctx *c, void **p, size_t bytes) {
+  if (injected_alloc_failure(c)) return cudaErrorMemoryAllocation;
+  return cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
 }
 // Ligand-size bucket: sizes are rounded up to a multiple of 8 atoms; launch
 // shapes are chosen (and autotuned) per bucket and cover its largest size.
