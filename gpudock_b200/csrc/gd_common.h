@@ -172,6 +172,12 @@ int split_for(gd_ctx *ctx, const KTables &T, int run_units, double min_cost);
 // 32-replica units of a complex's replicas (n_prt x n_lig x n_tmp): whole
 // exchange groups per unit when n_tmp divides 32.
 int units_of(int n_prt, int n_lig, int n_tmp);
+// What an idle server lane launches next: the initialisation of its new
+// requests (true), or MC steps of those it has.  Never two initialisations in
+// a row while it has some: under steady arrivals they would take no step.
+inline bool lane_inits_next(bool has_fresh, bool has_members, bool last_was_init) {
+  return has_fresh && !(has_members && last_was_init);
+}
 // Whether some of those units has at most 16 replicas (KRun.packed).
 bool has_packed_units(int n_prt, int n_lig, int n_tmp);
 

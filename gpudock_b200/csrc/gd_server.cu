@@ -511,8 +511,9 @@ void finish(gd_server *S, Req *r, ReqState st, gd_status err) {
 // The scheduler thread.  Each round it admits queued requests while the HBM
 // budget and the slot count allow, collects the lanes whose launch has ended
 // (advancing their requests, finishing the completed ones), and relaunches
-// every idle lane with its current members plus the newly admitted requests
-// of its shape (initialised first, on the same stream).
+// every idle lane: newly admitted requests of its shape are initialised by a
+// launch of their own and are members from then on, and MC launches advance all
+// members; the two take turns while both have something to do.
 void scheduler(gd_server *S) {
   cudaSetDevice(S->ctx->device);
   auto t_busy = Clock::now();
@@ -628,7 +629,7 @@ void scheduler(gd_server *S) {
       // new requests are initialised by a launch of their own, which the next
       // MC launch does not have to wait for in the stream
       std::vector<Req *> now;
-      if (!L.fresh.empty()) {
+      if (lane_inits_next(!L.fresh.empty(), !L.members.empty(), L.init)) {
         now.swap(L.fresh);
         for (Req *r : now) L.members.push_back(r);
         st = launch_lane(S, L, now, KMODE_INIT);
