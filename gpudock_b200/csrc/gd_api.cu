@@ -108,12 +108,10 @@ int units_of(int n_prt, int n_lig, int n_tmp) {
   return n_prt * ((n_lig * n_tmp + 31) / 32);
 }
 
-bool has_packed_units(int n_prt, int n_lig, int n_tmp) {
+bool all_packed_units(int n_lig, int n_tmp) {
   // every unit but the last of a protein conformation is full
-  const int G = 32 % n_tmp == 0 ? 32 / n_tmp : 0;
-  const int full = G ? G * n_tmp : 32, all = n_lig * n_tmp;
-  const int last = all % full ? all % full : full;
-  return packed_reps(last) < 32 || (all >= full && packed_reps(full) < 32);
+  const int full = 32 % n_tmp == 0 ? 32 / n_tmp * n_tmp : 32;
+  return packed_reps(std::min(full, n_lig * n_tmp)) < 32;
 }
 
 Tile tile_for(gd_ctx *ctx, const KTables &T) {

@@ -178,8 +178,10 @@ int units_of(int n_prt, int n_lig, int n_tmp);
 inline bool lane_inits_next(bool has_fresh, bool has_members, bool last_was_init) {
   return has_fresh && !(has_members && last_was_init);
 }
-// Whether some of those units has at most 16 replicas (KRun.packed).
-bool has_packed_units(int n_prt, int n_lig, int n_tmp);
+// Whether each of those units has at most 16 replicas (KRun.packed).  One full
+// unit keeps the ordered kernel for all of them: the packed one forms its sums
+// in another order, and the run ends with its full units either way.
+bool all_packed_units(int n_lig, int n_tmp);
 
 // Launches of different shapes (one per launch plan) are independent; each
 // kernel holds one CTA per SM, so a plan with fewer CTAs than SMs leaves the

@@ -42,7 +42,7 @@ struct Plan {
   int n_stages = 0, resident = 0, group_major = 0, fused = 0, grid = 0;
   int hb_pairs = 0;  // largest hb_pairs_of over its items
   int split = 1;     // CTAs (a cluster) per unit (split_for)
-  int packed = 0;    // some unit has at most 16 replicas (KRun.packed)
+  int packed = 0;    // every unit has at most 16 replicas (KRun.packed)
   int *d_cta_item = nullptr, *d_cta_rep0 = nullptr, *d_cta_nrep = nullptr;
   // persistent schedules (KRun.pieces) of this plan's units, by launch length
   std::vector<double> unit_cost;  // [grid] cost of one MC step of each unit
@@ -310,7 +310,7 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
     const int nt = I.n_tmp, nl = I.n_lig_conf;
     const bool gm = (32 % nt) == 0;
     const bool exch = (I.flags & GD_MC_EXCHANGE) != 0;
-    const int packed = has_packed_units(I.n_prt, nl, nt) ? 1 : 0;
+    const int packed = all_packed_units(nl, nt) ? 1 : 0;
     const Key key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, split, packed};
     Plan &pl = plans[key];
     pl.tile = t;

@@ -164,8 +164,8 @@ struct KRun {
                          // CTAs (<= 8) share each unit, CTA rank r taking the
                          // protein tiles r, r + split, ... (grid = units x split);
                          // 0 or 1: one CTA per unit
-  int packed;            // REMC / INIT: nonzero when some unit of the launch has at
-                         // most 16 replicas (packed_reps < 32); POSES: poses
+  int packed;            // REMC / INIT: nonzero when every unit of the launch has
+                         // at most 16 replicas (packed_reps < 32); POSES: poses
                          // per unit (8 or 16), or 0 for 32
   int hb_pairs;          // most atom pairs with an H-bond term in any warp of
                          // any item (hb_pairs_of); selects the kernel variant

@@ -929,7 +929,7 @@ __device__ __forceinline__ void close_range(const float2 (&nx)[NA / 2], const fl
 // HB: atom pairs per warp that evaluate the H-bond term (at least what the
 // launch's items need, KRun.hb_pairs).  PIECES: the CTA runs the pieces of a
 // persistent schedule (KRun.pieces, REMC only), else all steps of unit
-// blockIdx.x.  PACKED: units may have few replicas (KRun.packed); a kernel of
+// blockIdx.x.  PACKED: every unit has few replicas (KRun.packed); a kernel of
 // its own, since the distance between a lane's list entries as a variable
 // costs the pair loop 4%.
 // No producer warp: sm_100 splits the register file between the four

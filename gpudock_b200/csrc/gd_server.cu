@@ -98,7 +98,7 @@ struct Lane {
   Tile tile;
   int ns = 0, res = 0, gm = 0, spe = 0;
   int split = 1;                    // CTAs (a cluster) per request unit
-  int packed = 0;                   // some unit has at most 16 replicas (KRun.packed)
+  int packed = 0;                   // every unit has at most 16 replicas (KRun.packed)
   cudaStream_t stream = nullptr;
   // the lane's kernel error word and its count of ended launches, in pinned
   // host memory that the kernels write directly, and the launch's CTA counter
@@ -235,7 +235,7 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
   pick_stages(T, t, &ns, &res, split);
   const bool gm = (32 % r->mc.n_tmp) == 0;
   const int spe = r->mc.steps_per_exchange;
-  const int packed = has_packed_units(T.n_prt, T.n_lig, r->mc.n_tmp) ? 1 : 0;
+  const int packed = all_packed_units(T.n_lig, r->mc.n_tmp) ? 1 : 0;
   // the shape's least loaded lane; a new one while that lane holds requests
   // and the shape has fewer than kSubLanes
   Lane *best = nullptr;
