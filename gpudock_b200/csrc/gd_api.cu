@@ -71,11 +71,12 @@ Tile default_tile(int lna) {
   return best;
 }
 
-void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, int split) {
+void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, int split,
+                 bool lists) {
   const int n_tiles = (T.pnp + TILE_PTS - 1) / TILE_PTS;
   const int own = (n_tiles + split - 1) / split;  // tiles of a split's busiest CTA
   const size_t limit = 227 * 1024;
-  if (own <= MAX_RESIDENT_TILES && dock_smem_bytes(t.A, t.P, t.NA, own, split) <= limit) {
+  if (own <= MAX_RESIDENT_TILES && dock_smem_bytes(t.A, t.P, t.NA, own, split, lists) <= limit) {
     *n_stages = own;
     *resident = 1;
   } else {
@@ -677,6 +678,9 @@ static gd_status upload_ligand(const gd_complex *cx, TableUpload &U) {
   std::vector<int> koff(GD_NLT + 1, 0);
   for (int k = 0; k < cx->kde.pnk; ++k) koff[cx->kde.t[k] + 1] += 1;
   for (int i = 0; i < GD_NLT; ++i) koff[i + 1] += koff[i];
+  std::vector<KdeRange> kof(GD_NLT);
+  for (int i = 0; i < GD_NLT; ++i)
+    kof[i] = {koff[i], koff[i + 1], 1.0 / (double)std::max(1, koff[i + 1] - koff[i])};
   std::vector<float4> kd((size_t)cx->kde.pnk);
   {
     std::vector<int> fill(koff.begin(), koff.end() - 1);
@@ -720,7 +724,7 @@ static gd_status upload_ligand(const gd_complex *cx, TableUpload &U) {
     GD_TRY(upload(U, mask, &T.psp_mask));
   }
   GD_TRY(upload(U, kd, &T.kde));
-  GD_TRY(upload(U, koff, &T.kde_off));
+  GD_TRY(upload(U, kof, &T.kde_of));
   GD_TRY(upload(U, mc, &T.mcs));
   GD_TRY(upload(U, mw, &T.mcs_w));
 
@@ -949,7 +953,7 @@ gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int 
     const int per = R.packed ? R.packed : 32;
     grid = (n_pose + per - 1) / per * R.split;
   }
-  pick_stages(d->T, tile, &R.n_stages, &R.resident, std::max(1, R.split));
+  pick_stages(d->T, tile, &R.n_stages, &R.resident, std::max(1, R.split), true);
   GD_CUDA(launch_dock(R, tile.NA, grid, ctx->stream));
   ctx->launches += 1;
   return GD_OK;

@@ -60,7 +60,9 @@ Tile default_tile(int lna);
 int round_na(int na);  // smallest compiled NA >= na (0 if none)
 // Resident staging when the tiles of one CTA (of a split's busiest CTA) fit
 // in shared memory, else the streaming ring.
-void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, int split = 1);
+// lists: as in dock_smem_bytes
+void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, int split,
+                 bool lists);
 
 }  // namespace gd
 

@@ -306,11 +306,11 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
     Tile t = tile_for(ctx, I.T);
     const int split = splits[i];
     int ns, res;
-    pick_stages(I.T, t, &ns, &res, split);
     const int nt = I.n_tmp, nl = I.n_lig_conf;
+    const int packed = all_packed_units(nl, nt) ? 1 : 0;
+    pick_stages(I.T, t, &ns, &res, split, packed != 0);
     const bool gm = (32 % nt) == 0;
     const bool exch = (I.flags & GD_MC_EXCHANGE) != 0;
-    const int packed = all_packed_units(nl, nt) ? 1 : 0;
     const Key key{t.A, t.P, t.NA, ns, res, gm ? 1 : 0, split, packed};
     Plan &pl = plans[key];
     pl.tile = t;

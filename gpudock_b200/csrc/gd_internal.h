@@ -52,6 +52,12 @@ __host__ __device__ inline int packed_reps(int n) {
 
 enum KMode : int { KMODE_POSES = 0, KMODE_REMC = 1, KMODE_INIT = 2 };
 
+// KDE points of a ligand type: first, end and 1 / their number.
+struct KdeRange {
+  int begin, end;
+  double inv_n;
+};
+
 // Tables of one complex (device pointers + scalars).
 struct KTables {
   const float4 *pt_a;   // [n_prt][pnp_pad] {x, y, z, ele}
@@ -69,7 +75,7 @@ struct KTables {
   const uint32_t *psp_mask;  // [(psp_ncol + 31) / 32] bit r: some atom type of
                              // this ligand has a nonzero psp[type][r]
   const float4 *kde;    // [pnk] sorted by type {x, y, z, 0}
-  const int *kde_off;   // [NLT + 1]
+  const KdeRange *kde_of; // [NLT] a ligand type's points
   const float4 *mcs;    // [pos][lna] {x, y, z, valid}
   const double2 *mcs_w; // [pos] {tcc, 1 / number of valid atoms}
   const uint32_t *mcc_ref;  // [lna][mcc_words] reference contact map (bits)
@@ -234,7 +240,8 @@ struct KGroup {
   int item, p, l, pad;
 };
 
-size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split = 1);
+// lists: the kernel lists a chunk's points (poses and packed units)
+size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split, bool lists);
 
 // Device workspace that a pose call wants for dealing its poses into cells, 0
 // for a call too small to gain from them (gd_poses.cu).

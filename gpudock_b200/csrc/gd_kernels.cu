@@ -87,12 +87,6 @@ struct LaneState {
 static_assert(sizeof(LaneState) == 152, "LaneState layout");
 static_assert(sizeof(KItem) % 8 == 0, "KItem must keep the barriers 8-byte aligned");
 
-// KDE points of a slot's ligand type: first, end and 1 / their number.
-struct SlotKde {
-  int begin, end;
-  double inv_n;
-};
-
 // Shared-memory carve-up of one CTA.  The pair tables hold, for every
 // (atom group, atom pair h, point type), the parameters of the warp's two
 // atoms of pair h side by side, so one 16-byte load yields the operand pairs
@@ -101,19 +95,25 @@ struct SlotKde {
 //   ptab[.][1] = {-pmf0 a, -pmf0 b, pmf1 a, pmf1 b}
 //   htab[.]    = {-hdb0 a, -hdb0 b, w a, w b}  (w = hdb1 where the H-bond
 //                                               term is defined, else 0)
-// hmask[ag][pt] has bit h set when pair h of group ag has an H-bond term with
-// point type pt.  Slot s = ag + A k holds ligand atom order[s].
-//   far[ag][pt]  = the distance from which every atom of the group takes the
-//                  far form with point type pt
+// far[ag][pt]: the distance from which every atom of the group takes the far
+// form with point type pt, rounded up to a multiple of 32 units in the last
+// place; its low bits are the group's H-bond mask, bit h set when pair h has an
+// H-bond term with point type pt.  Slot s = ag + A k holds ligand atom order[s].
+// Kernels that list a chunk's points (lists: poses, packed units) also have:
 //   fpmf[ag][pt] = the sum of the group's pmf1 with it (the PMF term there)
-//   list[warp]   = (poses, packed lanes) the points of the warp's current
-//                  chunk, near ones first:
+//   list[warp]   = the points of the warp's current chunk, near ones first:
 //                  {offset of its record in shared memory | point type << 23
 //                  (list_entry), threshold of its close-range vote}
 //   pad          = the record of a padding point (fills up the lists)
+//   slot_k       = the KDE points of each slot's ligand type
+// The ordered kernel, which holds its protein for a whole launch where it
+// fits, goes without: 40 atoms and up to 6,144 points stay resident (5,760 with
+// them).
+constexpr uint32_t kHbMask = 31u;  // a bit per atom pair
+static_assert(MAX_NA / 2 <= 5, "H-bond mask");
 struct SmemLayout {
-  size_t ptab, htab, hmask, far, fpmf, list, pad, slot_q, slot_t, slot_a, slot_k, tiles, red, hpc, lane, item, bars,
-      ctl, xch, xch_step, total;
+  size_t ptab, htab, far, fpmf, list, pad, slot_q, slot_t, slot_a, slot_k, tiles, red, hpc, lane,
+      item, bars, ctl, xch, xch_step, total;
 };
 
 // Piece bookkeeping of a CTA, in shared memory so that none of it holds a
@@ -139,7 +139,8 @@ static_assert(sizeof(PieceCtl) <= 64, "PieceCtl fits its slot");
 // each CTA then also holds two (step parity) exchange buffers of its
 // per-replica partial sums: NRED FP64 terms and one FP32 hydrophobic sum per
 // atom slot, 32 lanes each.
-__host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, int split = 1) {
+__host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, int split,
+                                                  bool lists) {
   SmemLayout L;
   const size_t NH = NA / 2, MAXA = (size_t)A * NA, W = (size_t)A * P;
   size_t o = 0;
@@ -149,26 +150,23 @@ __host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, 
   o += (size_t)A * NH * PT_ROWS * 32;
   L.htab = o;
   o += (size_t)A * NH * PT_ROWS * 16;
-  L.hmask = o;
-  o += (size_t)A * PT_ROWS * 4;
   L.far = o;
   o += (size_t)A * PT_ROWS * 4;
   L.fpmf = o;
-  o += (size_t)A * PT_ROWS * 8;
+  if (lists) o += (size_t)A * PT_ROWS * 8;
   L.list = o;
-  o += W * LIST_LEN * sizeof(uint2);
-  o = (o + 15) & ~size_t(15);
+  if (lists) o += W * LIST_LEN * sizeof(uint2);
   L.pad = o;
-  o += 16;
+  if (lists) o += 16;
   L.slot_q = o;
   o += MAXA * 4;
   L.slot_t = o;
   o += MAXA * 4;
   L.slot_a = o;
   o += MAXA * 4;
-  o = (o + 15) & ~size_t(15);
+  if (lists) o = (o + 15) & ~size_t(15);
   L.slot_k = o;
-  o += MAXA * sizeof(SlotKde);
+  if (lists) o += MAXA * sizeof(KdeRange);
   o = (o + 127) & ~size_t(127);
   L.tiles = o;
   o += (size_t)NS * STAGE_BYTES;
@@ -193,8 +191,8 @@ __host__ __device__ inline SmemLayout smem_layout(int A, int P, int NA, int NS, 
 }
 
 #if GD_DOCK_PART == 0
-size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split) {
-  return smem_layout(A, P, NA, n_stages, split).total;
+size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split, bool lists) {
+  return smem_layout(A, P, NA, n_stages, split, lists).total;
 }
 #endif
 
@@ -950,16 +948,15 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   // split launch: clusters of csize CTAs, rank crank, share one unit; CTA
   // crank takes the protein tiles crank, crank + csize, ...
   const int csize = (!PIECES && R.split > 1) ? R.split : 1;
-  const SmemLayout SL = smem_layout(A, P, NA, NS, csize);
+  const SmemLayout SL = smem_layout(A, P, NA, NS, csize, kLists);
   float4 *s_ptab = reinterpret_cast<float4 *>(smem + SL.ptab);
   float4 *s_htab = reinterpret_cast<float4 *>(smem + SL.htab);
-  uint32_t *s_hmask = reinterpret_cast<uint32_t *>(smem + SL.hmask);
-  float *s_far = reinterpret_cast<float *>(smem + SL.far);
+  uint32_t *s_far = reinterpret_cast<uint32_t *>(smem + SL.far);
   double *s_fpmf = reinterpret_cast<double *>(smem + SL.fpmf);
   float *s_q = reinterpret_cast<float *>(smem + SL.slot_q);
   int *s_lt = reinterpret_cast<int *>(smem + SL.slot_t);
   int *s_atom = reinterpret_cast<int *>(smem + SL.slot_a);
-  SlotKde *s_kde = reinterpret_cast<SlotKde *>(smem + SL.slot_k);
+  KdeRange *s_kde = reinterpret_cast<KdeRange *>(smem + SL.slot_k);
   unsigned char *s_tiles = smem + SL.tiles;
   double *s_red = reinterpret_cast<double *>(smem + SL.red);
   float *s_hpc = reinterpret_cast<float *>(smem + SL.hpc);
@@ -1071,14 +1068,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
       s_atom[s] = a;
       s_lt[s] = a >= 0 ? TG.lig_t[a] : GD_NLT;
       s_q[s] = a >= 0 ? TG.lig_q[a] : 0.f;
-      SlotKde sk{0, 0, 0.0};
-      if (a >= 0) {
-        const int lt = TG.lig_t[a];
-        sk.begin = TG.kde_off[lt];
-        sk.end = TG.kde_off[lt + 1];
-        sk.inv_n = 1.0 / (double)max(1, sk.end - sk.begin);
-      }
-      s_kde[s] = sk;
+      if (kLists) s_kde[s] = a >= 0 ? TG.kde_of[TG.lig_t[a]] : KdeRange{0, 0, 0.0};
     }
     __syncthreads();
     // The pair tables from the slots' types (a padding atom's row is all zero;
@@ -1108,7 +1098,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll
         for (int k = 0; k < NA; ++k) fd = fmaxf(fd, TG.tab_far[s_lt[ag + A * k] * GD_NPT + pt]);
       }
-      s_far[i] = fd;
+      s_far[i] = (__float_as_uint(fd) + kHbMask) & ~kHbMask;
     }
     __syncthreads();
     // which pairs have an H-bond term, and the group's PMF sum
@@ -1123,8 +1113,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         if (H.x != 0.f || H.y != 0.f) m |= 1u << h;
         fp += (double)P1.z + (double)P1.w;
       }
-      s_hmask[i] = m;
-      s_fpmf[i] = fp;
+      s_far[i] |= m;
+      if (kLists) s_fpmf[i] = fp;
     }
     __syncthreads();  // every thread has read s_ctl->item
     if (threadIdx.x == 0) s_ctl->item = item;
@@ -1293,23 +1283,24 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   K.cb = dup2(6.0f * LOG2E);
   const float4 *my_ptab = s_ptab + (size_t)ag * NH * PT_ROWS * 2;
   const float4 *my_htab = s_htab + (size_t)ag * NH * PT_ROWS;
-  const uint32_t *my_hmask = s_hmask + (size_t)ag * PT_ROWS;
-  const float *my_far = s_far + (size_t)ag * PT_ROWS;
+  const uint32_t *my_far = s_far + (size_t)ag * PT_ROWS;
   const double *my_fpmf = s_fpmf + (size_t)ag * PT_ROWS;
   uint2 *my_list = reinterpret_cast<uint2 *>(smem + SL.list) + (size_t)warp * LIST_LEN;
   // padding points: the record, and the list entry (its vote never fires);
   // entries past a chunk's points are read ahead, so they start as valid ones
   const uint2 pad_entry =
       make_uint2(list_entry((uint32_t)SL.pad, PAD_POINT_TYPE), __float_as_uint(-1.0f));
-  if (threadIdx.x == 0)
-    *reinterpret_cast<float4 *>(smem + SL.pad) =
-        make_float4(PAD_POINT_COORD, PAD_POINT_COORD, PAD_POINT_COORD, 0.f);
-  for (int i = lane; i < LIST_LEN; i += 32) my_list[i] = pad_entry;
+  if constexpr (kLists) {
+    if (threadIdx.x == 0)
+      *reinterpret_cast<float4 *>(smem + SL.pad) =
+          make_float4(PAD_POINT_COORD, PAD_POINT_COORD, PAD_POINT_COORD, 0.f);
+    for (int i = lane; i < LIST_LEN; i += 32) my_list[i] = pad_entry;
+  }
   const bool mcc_on = MODE != KMODE_POSES && (I.flags & GD_MC_MCC) != 0u;
   // atom pairs of this warp with an H-bond term for some point type: the
   // first my_nhb pairs (capable atoms come first in the slot order)
   const int my_nhb =
-      32 - __clz(__reduce_or_sync(0xffffffffu, lane < PT_ROWS ? my_hmask[lane] : 0u));
+      32 - __clz(__reduce_or_sync(0xffffffffu, lane < PT_ROWS ? my_far[lane] & kHbMask : 0u));
   // the host's bound must cover this warp; report it if not (code 3)
   if (my_nhb > HB && lane == 0) report(R.err, 3);
   // warps whose atoms need fewer H-bond pairs than the launch's HB take a
@@ -1460,15 +1451,16 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
         const float4 p_l = ta[valid ? jl : j0];
         const float b2_l = box_dist2(G, p_l);
+        const uint32_t far_w = my_far[pt_l];
         const bool far_l = valid && usable_at(p_l.x, p_l.y, p_l.z) &&
-                           is_far(G, p_l, b2_l, my_far[pt_l] + reach);
+                           is_far(G, p_l, b2_l, __uint_as_float(far_w & ~kHbMask) + reach);
         const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
         const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
         const uint32_t close_m =
             subs > 1 ? __ballot_sync(0xffffffffu, valid && !far_l && b2_l <= thr_l) : 0u;
         // (after the order, which is the same with the MCC score on)
         if (mcc_on) thr_l = fmaxf(thr_l, T.near_mcc2);
-        const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && my_hmask[pt_l] != 0u);
+        const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && (far_w & kHbMask) != 0u);
         const int var = !chunk_hdb || my_nhb <= 0 ? 0 : my_nhb <= kHB1 ? 1 : 2;
         int it_near = 1;
         uint32_t close;
@@ -1594,7 +1586,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 #pragma unroll 1
     for (int i = crank0 + csize * lw; i < lna + T.pos; i += csize * W) {
       if (i < lna) {
-        const SlotKde sk = s_kde[i];
+        const KdeRange sk = kLists ? s_kde[i] : T.kde_of[s_lt[i]];
         if (sk.end > sk.begin) {
           const float3 x = placed(orig[s_atom[i]]);
           float kv = 0.f;
@@ -1887,7 +1879,7 @@ __global__ void fma_peak_kernel(float *out, int iters) {
 template <int MODE, int NA, int HB, bool PIECES, bool PACKED>
 static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *occ) {
   const int split = (!PIECES && R.split > 1) ? R.split : 1;
-  const size_t smem = dock_smem_bytes(R.A, R.P, NA, R.n_stages, split);
+  const size_t smem = dock_smem_bytes(R.A, R.P, NA, R.n_stages, split, PACKED || MODE == KMODE_POSES);
   const int threads = R.A * R.P * 32;
   cudaError_t e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, PACKED>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

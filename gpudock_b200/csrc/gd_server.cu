@@ -182,7 +182,7 @@ size_t request_bytes(const gd_complex *cx, const gd_mc_params *mc, int n_rep) {
   size_t b = (size_t)TAB_ROWS * GD_NPT * 28;
   b += (size_t)cx->lig.n_conf * cx->lig.lna * 16 + (size_t)cx->lig.lna * 8;
   b += (size_t)GD_NLT * cx->psp.n_col * 4;
-  b += (size_t)cx->kde.pnk * 16 + (GD_NLT + 1) * 4;
+  b += (size_t)cx->kde.pnk * 16 + GD_NLT * sizeof(KdeRange);
   b += (size_t)cx->mcs.pos * cx->lig.lna * 16 + (size_t)cx->mcs.pos * 16;
   b += (size_t)n_rep * (6 + GD_NTERM + 3) * 4 + 3 * MAX_TMP * 4;
   // MCC reference map: one bit per (atom, padded point)
@@ -232,10 +232,10 @@ gd_status lane_for(gd_server *S, const Req *r, Lane **out) {
   const int split =
       split_for(S->ctx, T, units_of(T.n_prt, T.n_lig, r->mc.n_tmp), kServeSplitCost);
   int ns, res;
-  pick_stages(T, t, &ns, &res, split);
+  const int packed = all_packed_units(T.n_lig, r->mc.n_tmp) ? 1 : 0;
+  pick_stages(T, t, &ns, &res, split, packed != 0);
   const bool gm = (32 % r->mc.n_tmp) == 0;
   const int spe = r->mc.steps_per_exchange;
-  const int packed = all_packed_units(T.n_lig, r->mc.n_tmp) ? 1 : 0;
   // the shape's least loaded lane; a new one while that lane holds requests
   // and the shape has fewer than kSubLanes
   Lane *best = nullptr;
