@@ -369,7 +369,7 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
     }
 
     if (MODE == KMODE_POSES) {
-      if (active) {
+      if (primary && active) {
 #pragma unroll
         for (int i = 0; i < GD_NTERM; ++i) R.terms[(size_t)rep * GD_NTERM + i] = e[i];
         if (R.raw) {
