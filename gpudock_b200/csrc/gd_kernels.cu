@@ -742,9 +742,11 @@ __device__ __forceinline__ float warp_max(float x) {
   return y;
 }
 
-// Coordinates that the far form takes: finite, and so that d^9 between a point
-// and an atom does not overflow, since from there on the two forms differ.
-constexpr float kUsable = 5.0e3f;
+// The far form is for finite coordinates, and such that d^9 between a point and
+// an atom does not overflow (from there on the two forms differ): atoms within
+// kUsable of the origin in each coordinate and points within kFarMost of the
+// region's middle are at most 1.8e4 A apart.
+constexpr float kUsable = 5.0e3f, kFarMost = 8.0e3f;
 __device__ __forceinline__ bool usable_at(float x, float y, float z) {  // false for NaN
   return fabsf(x) < kUsable && fabsf(y) < kUsable && fabsf(z) < kUsable;
 }
@@ -833,11 +835,13 @@ __device__ __forceinline__ float box_dist2(const Region &g, const float4 &p) {
   return fmaf(bz, bz, fmaf(by, by, bx * bx));
 }
 // Whether the point, at box_dist2 = b2, is at least D away from the region:
-// outside the box grown by D, or outside the ball grown by D.
+// outside the box grown by D, or outside the ball grown by D.  Never for a point
+// without a usable position.
 __device__ __forceinline__ bool is_far(const Region &g, const float4 &p, float b2, float D) {
   const float cx = g.mid.x - p.x, cy = g.mid.y - p.y, cz = g.mid.z - p.z;
   const float e = D + g.rad;
-  return b2 > D * D || fmaf(cz, cz, fmaf(cy, cy, cx * cx)) > e * e;
+  const float c2 = fmaf(cz, cz, fmaf(cy, cy, cx * cx));
+  return c2 < kFarMost * kFarMost && (b2 > D * D || c2 > e * e);  // false for NaN
 }
 
 // Close-range terms of one protein point (calcenergy_d.cu:80-138): the
@@ -1452,8 +1456,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         const float4 p_l = ta[valid ? jl : j0];
         const float b2_l = box_dist2(G, p_l);
         const uint32_t far_w = my_far[pt_l];
-        const bool far_l = valid && usable_at(p_l.x, p_l.y, p_l.z) &&
-                           is_far(G, p_l, b2_l, __uint_as_float(far_w & ~kHbMask) + reach);
+        const bool far_l = valid && is_far(G, p_l, b2_l, __uint_as_float(far_w & ~kHbMask) + reach);
         const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
         const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
         const uint32_t close_m =
