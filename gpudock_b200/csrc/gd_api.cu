@@ -97,7 +97,7 @@ int split_rule(gd_ctx *ctx, const KTables &T, int run_units, double min_cost) {
   const double cost = (double)lna_bucket(T.lna) * T.pnp;
   const int free = ctx->n_sm / std::max(1, run_units);
   int k = 1;
-  while (k < 8 && cost >= min_cost * 2.0 * k && 2 * k <= free) k *= 2;
+  while (k < MAX_SPLIT && cost >= min_cost * 2.0 * k && 2 * k <= free) k *= 2;
   return k;
 }
 

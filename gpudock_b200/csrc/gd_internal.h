@@ -21,7 +21,7 @@ constexpr int MAX_RESIDENT_TILES = 56; // 7168 points kept in smem for a launch
 constexpr int MAX_WARPS = GD_MAX_WARPS; // warps per CTA (all compute)
 constexpr int MAX_NA = 10;             // ligand atoms per warp (template bound)
 constexpr int MAX_LNA = 128;           // ligand atoms per complex
-constexpr int MAX_SPLIT = 16;          // CTAs that can share a unit (a cluster)
+constexpr int MAX_SPLIT = 8;           // CTAs that can share a unit (a cluster)
 constexpr int NRED = 10;               // partial sums per replica per warp
 constexpr int MAX_TMP = 64;            // temperatures per exchange group
 constexpr int TAB_ROWS = GD_NLT + 1;   // + one all-zero row for padding atoms

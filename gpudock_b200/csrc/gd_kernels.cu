@@ -462,7 +462,7 @@ __device__ __noinline__ void finish_step(const KRun &R, const KItem &I, LaneStat
   }
 
 struct PairConst {
-  float2 one, lj1, lj0, ca, cb;
+  float2 lj1, lj0, ca, cb;
 };
 
 // One protein point (A0) against this lane's NA atoms, two atoms per packed
@@ -1280,7 +1280,6 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   }
   const float inv_el1 = T.inv_el1;
   PairConst K;
-  K.one = dup2(1.0f);
   K.lj1 = dup2(T.lj0lj1);
   K.lj0 = dup2(T.lj0);
   K.ca = dup2(-0.5f * LOG2E);
@@ -1896,11 +1895,6 @@ static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *o
   }
   // clusters of `split` CTAs (grid = units x split), on SMs of one GPC
   if (split > MAX_SPLIT || grid % split) return cudaErrorInvalidValue;
-  if (split > 8) {  // beyond the portable size
-    e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, PACKED>,
-                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
