@@ -145,10 +145,13 @@ inline bool injected_alloc_failure(gd_ctx *c) {
   }
   return n == 1;
 }
-// Stream-ordered workspace of a call (freed with cudaFreeAsync).
+// Stream-ordered workspace of a call (freed with cudaFreeAsync).  One that the
+// work pool would not keep comes from the device's default pool, where uploads
+// and runs can have its memory next.
 inline cudaError_t work_alloc(gd_ctx *c, void **p, size_t bytes) {
   if (injected_alloc_failure(c)) return cudaErrorMemoryAllocation;
-  return cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  return bytes > kKeepBytes ? cudaMallocAsync(p, bytes, c->stream)
+                            : cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
 }
 // Ligand-size bucket: sizes are rounded up to a multiple of 8 atoms; launch
 // shapes are chosen (and autotuned) per bucket and cover its largest size.

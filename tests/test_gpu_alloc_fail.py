@@ -93,3 +93,20 @@ def test_similarity_workspace(ctx):
         _used_up(ctx, cx)
     assert np.array_equal(d.similarity_matrix(confs), want)
     d.close()
+
+
+def test_large_workspace_is_of_the_default_pool(ctx):
+    """A matrix beyond what the work pool keeps: its memory is the default
+    pool's, for uploads and runs to take next, and given back."""
+    cx = synth.make_complex(synth.ComplexSpec(pnp=300, lna=8), seed=105)
+    n = 4200
+    confs = np.zeros((n, 8), np.float32)
+    confs[:, 2:] = np.random.default_rng(4).normal(0.0, 1.0, (n, 6))
+    d = lib.DeviceComplex(ctx, cx)
+    used = _pool_used()
+    _high(reset=True)
+    got = d.similarity_matrix(confs)
+    assert _high() >= used + got.nbytes and _pool_used() == used
+    pick = np.arange(0, n, 97)
+    assert np.array_equal(got[np.ix_(pick, pick)], d.similarity_matrix(confs[pick]))
+    d.close()
