@@ -24,7 +24,7 @@ LIB = os.path.join(LIBDIR, "libgpudock.so")
 SOURCES = ["gd_kernels.cu", "gd_api.cu", "gd_ensemble.cu", "gd_server.cu", "gd_noalloc.cu",
            "gd_poses.cu", "gd_similarity.cu", "gd_load.cpp"]
 # the kernel variants of gd_kernels.cu are compiled in parts, in parallel
-PARTS = {"gd_kernels.cu": [f"-DGD_DOCK_PART={k}" for k in range(6)]}
+PARTS = {"gd_kernels.cu": [f"-DGD_DOCK_PART={k}" for k in range(8)]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

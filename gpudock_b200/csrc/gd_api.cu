@@ -647,6 +647,36 @@ static float far_distance(const gd_enepara &F, int i, int j, float max_pmf0) {
   return std::isfinite(p0) && D < 1e6 ? (float)D : std::numeric_limits<float>::infinity();
 }
 
+// gd_dcomplex.far_share, of protein conformation pc.
+static double far_share_of(const gd_complex *cx, int pc) {
+  const gd_ligand &L = cx->lig;
+  const gd_protein &P = cx->prt;
+  const gd_enepara &F = *cx->ff;
+  float max_pmf0 = 0.f, reach2 = 0.f;
+  for (int i = 0; i < GD_NLT; ++i)
+    for (int j = 0; j < GD_NPT; ++j) max_pmf0 = std::max(max_pmf0, F.pmf0[i][j]);
+  bool present[GD_NLT] = {};
+  for (int a = 0; a < L.lna; ++a) {
+    present[L.t[a]] = true;
+    reach2 = std::max(reach2, L.x[a] * L.x[a] + L.y[a] * L.y[a] + L.z[a] * L.z[a]);
+  }
+  float far2[GD_NPT];
+  for (int j = 0; j < GD_NPT; ++j) {
+    float d = 0.f;
+    for (int i = 0; i < GD_NLT; ++i)
+      if (present[i]) d = std::max(d, far_distance(F, i, j, max_pmf0));
+    d += std::sqrt(reach2);
+    far2[j] = d * d;
+  }
+  int n = 0;
+  for (int p = 0; p < P.pnp; ++p) {
+    const size_t i = (size_t)pc * P.pnp + p;
+    const float dx = P.x[i] - L.center[0], dy = P.y[i] - L.center[1], dz = P.z[i] - L.center[2];
+    n += dx * dx + dy * dy + dz * dz > far2[P.t[p]];
+  }
+  return (double)n / P.pnp;
+}
+
 // Ligand, pocket template and force-field tables of a complex.
 static gd_status upload_ligand(const gd_complex *cx, TableUpload &U) {
   gd_dcomplex *d = U.d;
@@ -881,6 +911,7 @@ static gd_status complex_upload_common(gd_ctx *ctx, const gd_complex *cx,
     }
     if (st == GD_OK) st = upload_ligand(cx, U);
     if (st == GD_OK) st = upload_mcc_ref(cx, share ? prt_conf0 : 0, U);
+    d->far_share = far_share_of(cx, share ? prt_conf0 : 0);
     if (st == GD_OK) st = upload_finish(U);
     if (st == GD_OK) {
       cudaError_t e = cudaStreamSynchronize(ctx->stream);
@@ -953,7 +984,8 @@ gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int 
     const int per = R.packed ? R.packed : 32;
     grid = (n_pose + per - 1) / per * R.split;
   }
-  pick_stages(d->T, tile, &R.n_stages, &R.resident, std::max(1, R.split), true);
+  pick_stages(d->T, tile, &R.n_stages, &R.resident, std::max(1, R.split),
+              R.packed != 0 || R.pose_grid != nullptr);
   GD_CUDA(launch_dock(R, tile.NA, grid, ctx->stream));
   ctx->launches += 1;
   return GD_OK;

@@ -120,6 +120,8 @@ struct gd_dcomplex {
   size_t bytes = 0;
   std::atomic<int> refs{1};
   gd_dcomplex *protein_owner = nullptr;  // when the protein arrays are shared
+  double far_share = 0.0;  // share of the protein's points that are far of the
+                           // ligand at its start place, however it is turned
   // device position -> caller's point index: points whose type can form an
   // H-bond come first, so a 32-point chunk rarely mixes the two kinds
   std::vector<int> point_order;
@@ -183,6 +185,12 @@ int units_of(int n_prt, int n_lig, int n_tmp);
 inline bool lane_inits_next(bool has_fresh, bool has_members, bool last_was_init) {
   return has_fresh && !(has_members && last_was_init);
 }
+// MC launches whose complexes have a smaller share of far points (far_share)
+// take them all in the full form (KFORM_NEAR, the same bits).  20 steps of 160
+// units, near form against near / far: share 0.01 (96 atoms x 700 points) 7.59
+// against 8.14 ms, 0.08 (24 x 700) 2.38 and 2.52, 0.17 (96 x 1,500) 13.9 and 14.4;
+// 0.29 (48 x 1,500) 7.18 and 7.10, 0.43 (24 x 1,500) 3.83 and 3.61.
+constexpr double kFarShareMc = 0.25;
 // Whether each of those units has at most 16 replicas (KRun.packed).  One full
 // unit keeps the ordered kernel for all of them: the packed one forms its sums
 // in another order, and the run ends with its full units either way.

@@ -42,6 +42,7 @@ struct Plan {
   int n_stages = 0, resident = 0, group_major = 0, fused = 0, grid = 0;
   int hb_pairs = 0;  // largest hb_pairs_of over its items
   int split = 1;     // CTAs (a cluster) per unit (split_for)
+  double far = 0.0;  // far_share of its units, weighted by their cost
   int packed = 0;    // every unit has at most 16 replicas (KRun.packed)
   int *d_cta_item = nullptr, *d_cta_rep0 = nullptr, *d_cta_nrep = nullptr;
   // persistent schedules (KRun.pieces) of this plan's units, by launch length
@@ -351,6 +352,7 @@ gd_status ens_build(Ens &E, gd_ctx *ctx, int n, const gd_dcomplex *const *dcx,
       c0.push_back(std::get<2>(c));
       cn.push_back(std::get<3>(c));
       pl.cost += std::get<0>(c);
+      pl.far += std::get<0>(c) * dcx[std::get<1>(c)]->far_share;
       pl.unit_cost.push_back(std::get<0>(c));
     }
     pl.grid = (int)ci.size();
@@ -398,6 +400,7 @@ KRun run_desc(const Ens &E, const Plan &pl, int mode) {
   R.hb_pairs = pl.hb_pairs;
   R.split = pl.split;
   R.packed = pl.packed;
+  R.near_only = pl.far < kFarShareMc * pl.cost;
   return R;
 }
 

@@ -58,6 +58,13 @@ struct KdeRange {
   double inv_n;
 };
 
+// How a launch takes a chunk's points (gd_kernels.cu): all of them in the full
+// form, in their order (NEAR); in their order, each near or far (ORDERED); near
+// ones first, from a list (LISTS); lists shared by groups of lanes (PACKED).
+// Poses: NEAR, LISTS (in cells), PACKED.  MC steps: NEAR, ORDERED (the same
+// bits), PACKED.  Start energies: ORDERED, PACKED.
+enum KForm : int { KFORM_NEAR, KFORM_ORDERED, KFORM_LISTS, KFORM_PACKED };
+
 // Tables of one complex (device pointers + scalars).
 struct KTables {
   const float4 *pt_a;   // [n_prt][pnp_pad] {x, y, z, ele}
@@ -173,6 +180,7 @@ struct KRun {
   int packed;            // REMC / INIT: nonzero when every unit of the launch has
                          // at most 16 replicas (packed_reps < 32); POSES: poses
                          // per unit (8 or 16), or 0 for 32
+  int near_only;         // REMC: few points are far of the ligands (kFarShareMc)
   int hb_pairs;          // most atom pairs with an H-bond term in any warp of
                          // any item (hb_pairs_of); selects the kernel variant
   // Persistent schedule (REMC; nullptr: CTA b runs every step of unit b,

@@ -66,6 +66,10 @@ constexpr float FAR = 1.0e3f;
 constexpr int PT_ROWS = 32;
 static_assert(PAD_POINT_TYPE >= GD_NPT && PAD_POINT_TYPE < PT_ROWS, "padding type row");
 
+__host__ __device__ constexpr bool form_lists(int form) {
+  return form == KFORM_LISTS || form == KFORM_PACKED;
+}
+
 // A chunk's list: its points, both parts filled up to a multiple of the
 // subsets, and what the loops read ahead of their last entry.
 constexpr int LIST_LEN = CHUNK + 4 * MAX_SUBS;
@@ -730,6 +734,36 @@ __device__ __forceinline__ uint32_t chunk_ordered(const float2 (&nx)[NH], const 
   return close;
 }
 
+// The points j0 .. j1-1 of a tile in their order, all by pair_block1, two per
+// iteration: where few points are far, the far body and the choice of one cost
+// more than they save.  700 points x 96 atoms x 160 units: 7.65 ms per 20 steps
+// against chunk_ordered's 8.14; 2,100 .. 20,000 poses: 4 .. 6% less than from lists.
+template <int NH, int NHB>
+__device__ __forceinline__ uint32_t chunk_near(const float2 (&nx)[NH], const float2 (&ny)[NH],
+                                               const float2 (&nz)[NH], const float4 *ta,
+                                               const float2 *tb, int j0, int j1,
+                                               const float4 *my_ptab, const float4 *my_htab,
+                                               const PairConst &K, float thr_l, float2 &fvdw,
+                                               float2 &fpmf, float2 &fhdb, float2 (&fek)[NH]) {
+  uint32_t close = 0u;
+  float4 Ap = ta[j0];  // read one point ahead
+  int pt = (int)(__float_as_uint(tb[j0].y) & META_TYPE_MASK);
+#pragma unroll 2
+  for (int j = j0; j < j1; ++j) {
+    const int jn = min(j + 1, j1 - 1);
+    const float4 An = ta[jn];
+    const int ptn = (int)(__float_as_uint(tb[jn].y) & META_TYPE_MASK);
+    float mn = 3.0e38f;
+    pair_block1<NH, NHB>(nx, ny, nz, Ap, my_ptab + pt * 2, my_htab + pt, K, fvdw, fpmf, fhdb, fek,
+                         mn);
+    const float thr = __shfl_sync(0xffffffffu, thr_l, j - j0);
+    close |= (__any_sync(0xffffffffu, mn <= thr) ? 1u : 0u) << (j - j0);
+    Ap = An;
+    pt = ptn;
+  }
+  return close;
+}
+
 // Largest value, NaN if there is one: of two values, of a warp's lanes.
 __device__ __forceinline__ float max_nan(float a, float b) {
   float y;
@@ -931,20 +965,19 @@ __device__ __forceinline__ void close_range(const float2 (&nx)[NA / 2], const fl
 // HB: atom pairs per warp that evaluate the H-bond term (at least what the
 // launch's items need, KRun.hb_pairs).  PIECES: the CTA runs the pieces of a
 // persistent schedule (KRun.pieces, REMC only), else all steps of unit
-// blockIdx.x.  PACKED: every unit has few replicas (KRun.packed); a kernel of
-// its own, since the distance between a lane's list entries as a variable
-// costs the pair loop 4%.
+// blockIdx.x.  FORM: how it takes a chunk's points (KForm).  Kernels of their
+// own: as a branch in one kernel the bodies would not fit the instruction caches,
+// and PACKED's distance between a lane's list entries as a variable costs the
+// pair loop 4%.
 // No producer warp: sm_100 splits the register file between the four
 // schedulers, so a 13th warp would put four warps on one scheduler and cap
 // every thread at 128 registers; 12 warps leave room for about 168.
-template <int MODE, int NA, int HB, bool PIECES, bool PACKED>
+template <int MODE, int NA, int HB, bool PIECES, int FORM>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     dock_kernel(const __grid_constant__ KRun R) {
   static_assert(NA % 2 == 0, "atoms are processed in pairs");
   constexpr int NH = NA / 2;
-  // poses and packed lanes list a chunk's points, near ones first; MC units
-  // keep their order (chunk_ordered)
-  constexpr bool kLists = PACKED || MODE == KMODE_POSES;
+  constexpr bool PACKED = FORM == KFORM_PACKED, kLists = form_lists(FORM);
   static_assert(HB >= 0 && HB <= NH, "H-bond pair bound");
   extern __shared__ __align__(128) unsigned char smem[];
   const int A = R.A, P = R.P, W = A * P, NS = R.n_stages;
@@ -1390,7 +1423,9 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     // by the atoms' largest distance from the ligand's centre (any rotation)
     Region G;
     float reach = 0.f;
-    if (MODE != KMODE_POSES) {
+    if constexpr (FORM == KFORM_NEAR) {
+      // every point is near
+    } else if (MODE != KMODE_POSES) {
       G = warp_region<NA>(nx, ny, nz, rl < n_act ? n_my : 0);
     } else {
       G = pose_region(R, unit, lcx, lcy, lcz);
@@ -1441,10 +1476,9 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         // close-range votes are collected in a mask and served after the
         // branch-free pass, so consecutive points' chains overlap
         // lane j looks at point j, whether it is far of all the warp's atoms in
-        // all lanes.  MC units of more than 16 replicas keep the points' order;
-        // with lists, the warp takes the points that are not far, then the far
-        // ones, and of the former those that can have a close-range term first,
-        // so that packed lanes meet them in few iterations
+        // all lanes.  With lists, the warp takes the points that are not far, then
+        // the far ones, and of the former those that can have a close-range term
+        // first, so that packed lanes meet them in few iterations
         const int jl = j0 + lane;
         const bool valid = jl < j1;
         const float2 pb_l = valid ? tb[jl] : make_float2(0.f, __uint_as_float(PAD_POINT_TYPE));
@@ -1452,21 +1486,32 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         const int pt_l = (int)(meta_l & META_TYPE_MASK);
         float thr_l = T.near4[((meta_l & META_HPC_BIT) ? 1 : 0) |
                               ((((meta_l >> META_CLASS_SHIFT) & 3u) == 2u) ? 2 : 0)];
-        const float4 p_l = ta[valid ? jl : j0];
-        const float b2_l = box_dist2(G, p_l);
         const uint32_t far_w = my_far[pt_l];
-        const bool far_l = valid && is_far(G, p_l, b2_l, __uint_as_float(far_w & ~kHbMask) + reach);
-        const uint32_t far_m = __ballot_sync(0xffffffffu, far_l);
-        const uint32_t near_m = __ballot_sync(0xffffffffu, valid && !far_l);
-        const uint32_t close_m =
-            subs > 1 ? __ballot_sync(0xffffffffu, valid && !far_l && b2_l <= thr_l) : 0u;
+        bool far_l = false;
+        uint32_t far_m = 0u, near_m = 0u, close_m = 0u;
+        if constexpr (FORM != KFORM_NEAR) {
+          const float4 p_l = ta[valid ? jl : j0];
+          const float b2_l = box_dist2(G, p_l);
+          far_l = valid && is_far(G, p_l, b2_l, __uint_as_float(far_w & ~kHbMask) + reach);
+          far_m = __ballot_sync(0xffffffffu, far_l);
+          near_m = __ballot_sync(0xffffffffu, valid && !far_l);
+          if (subs > 1) close_m = __ballot_sync(0xffffffffu, valid && !far_l && b2_l <= thr_l);
+        }
         // (after the order, which is the same with the MCC score on)
         if (mcc_on) thr_l = fmaxf(thr_l, T.near_mcc2);
         const bool chunk_hdb = __any_sync(0xffffffffu, !far_l && (far_w & kHbMask) != 0u);
         const int var = !chunk_hdb || my_nhb <= 0 ? 0 : my_nhb <= kHB1 ? 1 : 2;
         int it_near = 1;
         uint32_t close;
-        if constexpr (!kLists) {
+        if constexpr (FORM == KFORM_NEAR) {
+          auto near_part = [&](auto hb) {
+            return chunk_near<NH, decltype(hb)::value>(nx, ny, nz, ta, tb, j0, j1, my_ptab,
+                                                       my_htab, K, thr_l, fvdw, fpmf, fhdb, fek);
+          };
+          close = var == 0   ? near_part(Int<0>{})
+                  : var == 1 ? near_part(Int<kHB1>{})
+                             : near_part(Int<HB>{});
+        } else if constexpr (FORM == KFORM_ORDERED) {
           close = chunk_ordered<NH, kHB1, HB>(nx, ny, nz, ta, tb, j0, j1, far_m, var, my_ptab,
                                               my_htab, K, thr_l, fvdw, fpmf, fhdb, fek);
         } else {
@@ -1878,19 +1923,19 @@ __global__ void fma_peak_kernel(float *out, int iters) {
 #endif  // GD_DOCK_PART == 0
 
 // ---------------------------------------------------------------------------
-template <int MODE, int NA, int HB, bool PIECES, bool PACKED>
+template <int MODE, int NA, int HB, bool PIECES, int FORM>
 static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *occ) {
   const int split = (!PIECES && R.split > 1) ? R.split : 1;
-  const size_t smem = dock_smem_bytes(R.A, R.P, NA, R.n_stages, split, PACKED || MODE == KMODE_POSES);
+  const size_t smem = dock_smem_bytes(R.A, R.P, NA, R.n_stages, split, form_lists(FORM));
   const int threads = R.A * R.P * 32;
-  cudaError_t e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, PACKED>,
+  cudaError_t e = cudaFuncSetAttribute(dock_kernel<MODE, NA, HB, PIECES, FORM>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (occ)  // occupancy query instead of a launch
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dock_kernel<MODE, NA, HB, PIECES, PACKED>,
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dock_kernel<MODE, NA, HB, PIECES, FORM>,
                                                          threads, smem);
   if (split == 1) {
-    dock_kernel<MODE, NA, HB, PIECES, PACKED><<<grid, threads, smem, s>>>(R);
+    dock_kernel<MODE, NA, HB, PIECES, FORM><<<grid, threads, smem, s>>>(R);
     return cudaGetLastError();
   }
   // clusters of `split` CTAs (grid = units x split), on SMs of one GPC
@@ -1907,57 +1952,62 @@ static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *o
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, dock_kernel<MODE, NA, HB, PIECES, PACKED>, R);
+  return cudaLaunchKernelEx(&cfg, dock_kernel<MODE, NA, HB, PIECES, FORM>, R);
 }
 
 // Three H-bond bounds per NA: at most two or three pairs (ligands where up
 // to about a third or half of the atoms have the term, the common cases), or
 // every pair, which is the packed kernel's only one.
-template <int MODE, int NA, bool PIECES, bool PACKED>
+template <int MODE, int NA, bool PIECES, int FORM>
 static cudaError_t launch_na(const KRun &R, int grid, cudaStream_t s, int *occ) {
   constexpr int NH = NA / 2;
   constexpr int HB2 = NH < 2 ? NH : 2;
   constexpr int HB3 = NH < 3 ? NH : 3;
-  if constexpr (!PACKED) {
-    if (R.hb_pairs <= HB2) return launch_kernel<MODE, NA, HB2, PIECES, false>(R, grid, s, occ);
-    if (R.hb_pairs <= HB3) return launch_kernel<MODE, NA, HB3, PIECES, false>(R, grid, s, occ);
+  if constexpr (FORM != KFORM_PACKED) {
+    if (R.hb_pairs <= HB2) return launch_kernel<MODE, NA, HB2, PIECES, FORM>(R, grid, s, occ);
+    if (R.hb_pairs <= HB3) return launch_kernel<MODE, NA, HB3, PIECES, FORM>(R, grid, s, occ);
   }
-  return launch_kernel<MODE, NA, NH, PIECES, PACKED>(R, grid, s, occ);
+  return launch_kernel<MODE, NA, NH, PIECES, FORM>(R, grid, s, occ);
 }
 
 // The kernel variants are compiled in several objects of this source
-// (GD_DOCK_PART 1 .. 5; part 0 holds everything else).
-template <int MODE, bool PIECES, bool PACKED>
+// (GD_DOCK_PART 1 .. 7; part 0 holds everything else).
+template <int MODE, bool PIECES, int FORM>
 cudaError_t launch_part(const KRun &R, int NA, int grid, cudaStream_t s, int *occ);
 
 #if GD_DOCK_PART > 0
-template <int MODE, bool PIECES, bool PACKED>
+template <int MODE, bool PIECES, int FORM>
 cudaError_t launch_part(const KRun &R, int NA, int grid, cudaStream_t s, int *occ) {
   switch (NA) {
-    case 2: return launch_na<MODE, 2, PIECES, PACKED>(R, grid, s, occ);
-    case 4: return launch_na<MODE, 4, PIECES, PACKED>(R, grid, s, occ);
-    case 6: return launch_na<MODE, 6, PIECES, PACKED>(R, grid, s, occ);
-    case 8: return launch_na<MODE, 8, PIECES, PACKED>(R, grid, s, occ);
-    case 10: return launch_na<MODE, 10, PIECES, PACKED>(R, grid, s, occ);
+    case 2: return launch_na<MODE, 2, PIECES, FORM>(R, grid, s, occ);
+    case 4: return launch_na<MODE, 4, PIECES, FORM>(R, grid, s, occ);
+    case 6: return launch_na<MODE, 6, PIECES, FORM>(R, grid, s, occ);
+    case 8: return launch_na<MODE, 8, PIECES, FORM>(R, grid, s, occ);
+    case 10: return launch_na<MODE, 10, PIECES, FORM>(R, grid, s, occ);
     default: return cudaErrorInvalidValue;
   }
 }
-#define GD_DOCK_VARIANT(MODE, PIECES, PACKED)                                                  \
-  template cudaError_t launch_part<MODE, PIECES, PACKED>(const KRun &, int, int, cudaStream_t, \
-                                                         int *)
+#define GD_DOCK_VARIANT(MODE, PIECES, FORM)                                                  \
+  template cudaError_t launch_part<MODE, PIECES, FORM>(const KRun &, int, int, cudaStream_t, \
+                                                       int *)
 #if GD_DOCK_PART == 1
-GD_DOCK_VARIANT(KMODE_POSES, false, false);
-GD_DOCK_VARIANT(KMODE_POSES, false, true);
+GD_DOCK_VARIANT(KMODE_POSES, false, KFORM_LISTS);
+GD_DOCK_VARIANT(KMODE_POSES, false, KFORM_PACKED);
 #elif GD_DOCK_PART == 2
-GD_DOCK_VARIANT(KMODE_REMC, false, false);
+GD_DOCK_VARIANT(KMODE_REMC, false, KFORM_ORDERED);
 #elif GD_DOCK_PART == 3
-GD_DOCK_VARIANT(KMODE_REMC, true, false);
+GD_DOCK_VARIANT(KMODE_REMC, true, KFORM_ORDERED);
 #elif GD_DOCK_PART == 4
-GD_DOCK_VARIANT(KMODE_REMC, false, true);
-GD_DOCK_VARIANT(KMODE_REMC, true, true);
+GD_DOCK_VARIANT(KMODE_REMC, false, KFORM_PACKED);
+GD_DOCK_VARIANT(KMODE_REMC, true, KFORM_PACKED);
+#elif GD_DOCK_PART == 5
+GD_DOCK_VARIANT(KMODE_INIT, false, KFORM_ORDERED);
+GD_DOCK_VARIANT(KMODE_INIT, false, KFORM_PACKED);
+#elif GD_DOCK_PART == 6
+GD_DOCK_VARIANT(KMODE_POSES, false, KFORM_NEAR);
+GD_DOCK_VARIANT(KMODE_REMC, false, KFORM_NEAR);
 #else
-GD_DOCK_VARIANT(KMODE_INIT, false, false);
-GD_DOCK_VARIANT(KMODE_INIT, false, true);
+GD_DOCK_VARIANT(KMODE_REMC, true, KFORM_NEAR);
 #endif
 
 #else
@@ -1966,17 +2016,20 @@ static cudaError_t dock_dispatch(const KRun &R, int NA, int grid, cudaStream_t s
   const bool packed = R.packed != 0;
   switch (R.mode) {
     case KMODE_POSES:
-      return packed ? launch_part<KMODE_POSES, false, true>(R, NA, grid, s, occ)
-                    : launch_part<KMODE_POSES, false, false>(R, NA, grid, s, occ);
+      return packed        ? launch_part<KMODE_POSES, false, KFORM_PACKED>(R, NA, grid, s, occ)
+             : R.pose_grid ? launch_part<KMODE_POSES, false, KFORM_LISTS>(R, NA, grid, s, occ)
+                           : launch_part<KMODE_POSES, false, KFORM_NEAR>(R, NA, grid, s, occ);
     case KMODE_REMC:
       if (R.pieces)
-        return packed ? launch_part<KMODE_REMC, true, true>(R, NA, grid, s, occ)
-                      : launch_part<KMODE_REMC, true, false>(R, NA, grid, s, occ);
-      return packed ? launch_part<KMODE_REMC, false, true>(R, NA, grid, s, occ)
-                    : launch_part<KMODE_REMC, false, false>(R, NA, grid, s, occ);
+        return packed        ? launch_part<KMODE_REMC, true, KFORM_PACKED>(R, NA, grid, s, occ)
+               : R.near_only ? launch_part<KMODE_REMC, true, KFORM_NEAR>(R, NA, grid, s, occ)
+                             : launch_part<KMODE_REMC, true, KFORM_ORDERED>(R, NA, grid, s, occ);
+      return packed        ? launch_part<KMODE_REMC, false, KFORM_PACKED>(R, NA, grid, s, occ)
+             : R.near_only ? launch_part<KMODE_REMC, false, KFORM_NEAR>(R, NA, grid, s, occ)
+                           : launch_part<KMODE_REMC, false, KFORM_ORDERED>(R, NA, grid, s, occ);
     default:
-      return packed ? launch_part<KMODE_INIT, false, true>(R, NA, grid, s, occ)
-                    : launch_part<KMODE_INIT, false, false>(R, NA, grid, s, occ);
+      return packed ? launch_part<KMODE_INIT, false, KFORM_PACKED>(R, NA, grid, s, occ)
+                    : launch_part<KMODE_INIT, false, KFORM_ORDERED>(R, NA, grid, s, occ);
   }
 }
 

@@ -414,7 +414,14 @@ gd_status launch_lane(gd_server *S, Lane &L, const std::vector<Req *> &rs, int m
   R.busy_ns = S->d_busy_ns;
   R.split = L.split;
   R.packed = L.packed;
-  for (const Req *r : rs) R.hb_pairs = std::max(R.hb_pairs, hb_pairs_of(r->item.T, L.tile.A));
+  double cost = 0.0, far = 0.0;
+  for (const Req *r : rs) {
+    R.hb_pairs = std::max(R.hb_pairs, hb_pairs_of(r->item.T, L.tile.A));
+    const double c = r->cost * r->n_rep * r->item.n_run;
+    cost += c;
+    far += c * r->dcx->far_share;
+  }
+  R.near_only = far < kFarShareMc * cost;
   GD_CUDA(launch_dock(R, L.tile.NA, (int)n_cta * L.split, s));
   S->ctx->launches += 1;
   S->n_launch += 1;
