@@ -1005,7 +1005,7 @@ extern "C" gd_status gd_energy_poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int 
   if (!poses || !terms) return fail(GD_EINVAL, "poses/terms NULL");
   GD_CUDA(cudaSetDevice(ctx->device));
   void *work = nullptr;
-  const size_t bytes = pose_work_bytes(d->T, n_pose);
+  const size_t bytes = pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose);
   // without room for the cells' workspace the call runs without them
   if (bytes && work_alloc(ctx, &work, bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -1032,7 +1032,7 @@ extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_
   const size_t total = up(pose_b) + up(term_b) + raw_b;
   // a small call passes through the context's pinned memory, which the kernel
   // reads and writes directly: no allocation and no copy in the stream
-  if (total <= kStageBytes && pose_work_bytes(d->T, n_pose) == 0) {
+  if (total <= kStageBytes && pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose) == 0) {
     std::unique_lock<std::mutex> lk(ctx->stage_mu, std::try_to_lock);
     if (lk.owns_lock()) {
       unsigned char *p = ctx->stage;

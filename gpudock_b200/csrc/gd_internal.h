@@ -251,9 +251,11 @@ struct KGroup {
 // lists: the kernel lists a chunk's points (poses and packed units)
 size_t dock_smem_bytes(int A, int P, int NA, int n_stages, int split, bool lists);
 
-// Device workspace that a pose call wants for dealing its poses into cells, 0
-// for a call too small to gain from them (gd_poses.cu).
-size_t pose_work_bytes(const KTables &T, int n_pose);
+// Whether a pose call is faster with its poses dealt into cells, and the device
+// workspace that it wants for that, else 0 (gd_poses.cu).  far_share: as in
+// gd_dcomplex.
+bool pose_cells_pay(const KTables &T, double far_share, int n_sm, int n_pose);
+size_t pose_work_bytes(const KTables &T, double far_share, int n_sm, int n_pose);
 // Deals the poses of R (n_pose, poses) into cells, using pose_work_bytes of
 // workspace until the energy launch has ended; fills R's cell arrays and the
 // launch's grid and the number of launches made.

@@ -74,7 +74,7 @@ extern "C" gd_status gd_energy_poses_noalloc(gd_ctx *ctx, const gd_dcomplex *d, 
   float *d_poses = reinterpret_cast<float *>(base);
   float *d_terms = reinterpret_cast<float *>(base + kPoseBytes);
   double *d_raw = reinterpret_cast<double *>(base + kPoseBytes + kTermBytes);
-  const size_t work = gd::pose_work_bytes(d->T, n_pose);
+  const size_t work = gd::pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose);
   if (work > kWorkBytes) return gd::fail(GD_EINVAL, "internal: pose workspace of %zu bytes", work);
   const size_t pose_b = sizeof(float) * 6 * (size_t)n_pose;
   GD_CUDA(cudaMemcpyAsync(d_poses, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream));

@@ -9,12 +9,13 @@
 // Poses without a usable place (a value that is not finite, or a translation
 // beyond kFarOut) get a cell of their own, for which no point is far.
 //
-// Four short launches (about 12 us together): the box of the translations;
-// every pose's cell and its rank in it; the cells' first 32-pose blocks; the
-// poses in block order.  Up to kSmallPoses poses, one launch of one CTA does
-// all of it (about 5 us).
+// Four short launches (33 us together for 65,536 poses, caches cold): the box of
+// the translations; every pose's cell and its rank in it; the cells' first
+// 32-pose blocks; the poses in block order.  Up to kSmallPoses poses, one launch
+// of one CTA does all of it (11 us for 4,096 poses, 27 us for 16,384).
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "gd_common.h"
 
@@ -278,15 +279,33 @@ __global__ void __launch_bounds__(1024)
 
 }  // namespace
 
-size_t pose_work_bytes(const KTables &T, int n_pose) {
-  // Cells pay once dealing the poses is a small part of the call (1e12
-  // pairs/s): about 5% at 1e8 pairs for one launch, 3% at 5e8 for four.  Below
-  // 2,048 poses a call's units are spread over the SMs in other ways
-  // (pose_units).
-  if (n_pose < 2048 || n_pose > kMostPoses ||
-      (double)n_pose * T.lna * T.pnp < (n_pose <= kSmallPoses ? 1e8 : 5e8))
-    return 0;
-  return layout(nullptr, n_pose).total;
+bool pose_cells_pay(const KTables &T, double far_share, int n_sm, int n_pose) {
+  if (n_pose > kMostPoses) return false;
+  // While the poses leave half of the SMs idle they are spread over them in
+  // other ways (pose_units): 2,048 poses x 48 x 1,100 in 338 us with cells, 181
+  // on clusters of two.
+  const int units = (n_pose + 31) / 32;
+  if (2 * units <= n_sm) return false;
+  // Else the waves of blocks, times a block's time (6 pairs per ns and SM), with
+  // the cells' half-filled last blocks and the deal on one side.  Were all points
+  // far they would take 0.4 of a block's time off it on average, less where a wave
+  // lasts as long as its slowest block, and the lists add 0.05; poses away from
+  // the start place have more far points than far_share says.  Measured, cells
+  // against without: 4,700 x 96 x 700 (a second wave) 856 and 442 us; 4,096 x 24 x
+  // 1,500 216 and 212; 16,384 of them 783 and 819; 20,000 x 96 x 700 (1% of the
+  // points far) 2,226 and 2,112; 131,072 x 48 x 2,000 12.6 and 14.3 ms; 30,011 x
+  // 48 x 8,000 9.0 and 12.2 ms.
+  const double cells = max_cells(n_pose);
+  const double blocks = units + 0.5 * cells + std::sqrt(cells);
+  const double w0 = std::ceil((double)units / n_sm), w1 = std::ceil(blocks / n_sm);
+  const double block_us = 32.0 * T.lna * T.pnp / 6000.0;
+  const double deal_us = n_pose <= kSmallPoses ? 6.0 + n_pose / 800.0 : 20.0 + n_pose / 4000.0;
+  const double block = 1.05 - 0.4 * far_share * (1.0 - 0.4 / w1);
+  return w1 * block_us * block + deal_us < w0 * block_us;
+}
+
+size_t pose_work_bytes(const KTables &T, double far_share, int n_sm, int n_pose) {
+  return pose_cells_pay(T, far_share, n_sm, n_pose) ? layout(nullptr, n_pose).total : 0;
 }
 
 cudaError_t pose_cells(KRun *R, void *work, int *grid, int *launches, cudaStream_t s) {

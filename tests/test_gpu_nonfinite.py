@@ -31,7 +31,7 @@ def _same(got, want):
     np.testing.assert_allclose(got, want, rtol=2e-5, atol=1e-6)
 
 
-@pytest.mark.parametrize("n", [2100, 17000])  # cells in one launch, in four
+@pytest.mark.parametrize("n", [2100, 4200, 17000])  # split; cells in one launch, in four
 @pytest.mark.parametrize("far", [0.0, 60.0, 300.0])
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
 def test_angles(ctx, n, far, bad):
@@ -62,7 +62,7 @@ def test_coordinates(ctx, what, bad, far):
         cx.prt_xyz[:, _hbond_point(cx), 0] = bad
     cx._struct = None
     d = lib.DeviceComplex(ctx, cx)
-    poses = np.zeros((2100, 6), np.float32)
+    poses = np.zeros((4200, 6), np.float32)
     want, want_raw = d.energy_poses(poses[:3])
     assert np.isnan(want_raw[0, [0, 2, 4]]).all()  # (1/d is 0 at an infinite distance)
     terms, raw = d.energy_poses(poses)
