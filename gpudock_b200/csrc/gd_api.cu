@@ -126,10 +126,9 @@ Tile tile_for(gd_ctx *ctx, const KTables &T) {
   return default_tile(hi);
 }
 
-// The runtime behind the contexts' shared blocks and pools (gd_shared.h).
+// The runtime behind the contexts' shared pinned blocks (gd_shared.h).
 struct CudaShared {
   using Error = cudaError_t;
-  using Pool = cudaMemPool_t;
   static bool ok(Error e) { return e == cudaSuccess; }
   // Serial number of the device's CUDA context, which no later one of the
   // process has (0: this driver does not tell).
@@ -155,26 +154,6 @@ struct CudaShared {
   }
   static Error pin(void **p, size_t bytes) { return cudaHostAlloc(p, bytes, cudaHostAllocDefault); }
   static void unpin(void *p) { cudaFreeHost(p); }
-  // The pool is stream-ordered, so safe between contexts.  It keeps up to
-  // kKeepBytes mapped between calls; the device's default pool unmaps at every
-  // synchronisation, which cost 50 .. 100 us per allocation.
-  static Error pool_create(int device, Pool *out) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    uint64_t keep = kKeepBytes;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    if (e != cudaSuccess) return e;
-    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess)
-      cudaMemPoolDestroy(pool);
-    else
-      *out = pool;
-    return e;
-  }
-  static void pool_destroy(Pool pool) { cudaMemPoolDestroy(pool); }
 };
 
 // Never destroyed: a handle may be released while the process ends.
@@ -183,7 +162,7 @@ static DeviceShared<CudaShared> &shared() {
   return *s;
 }
 
-// The context's error word, staging and pool.
+// The context's error word and staging.
 static cudaError_t shared_attach(gd_ctx *c) {
   DeviceShared<CudaShared>::Lease *l = nullptr;
   cudaError_t e = cudaErrorMemoryAllocation;
@@ -197,7 +176,6 @@ static cudaError_t shared_attach(gd_ctx *c) {
     return e;
   }
   c->shared = l;
-  c->pool = l->group->pool;
   c->h_err = static_cast<int *>(l->block);
   c->stage = static_cast<unsigned char *>(l->block) + 256;
   std::memset(l->block, 0, 256);
@@ -210,6 +188,68 @@ static void shared_detach(gd_ctx *c) {
   shared().release(l);
   delete l;
   c->shared = nullptr;
+}
+
+// The context's memory for this call, if no other call has it and the stream is
+// not under capture.
+void Workspace::take() {
+  asked_ = true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(c_->stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (cap != cudaStreamCaptureStatusNone) return;
+  {
+    std::lock_guard<std::mutex> g(c_->work_mu);
+    if (c_->work_busy) return;
+    c_->work_busy = kept_ = true;
+  }
+  if (expect_ > c_->work_bytes) resize(expect_);
+}
+
+Workspace::~Workspace() {
+  for (int k = 0; k < n_own_; ++k) cudaFreeAsync(own_[k], c_->stream);
+  if (!kept_) return;
+  if (want_ > c_->work_bytes) resize(want_);  // for the next such call
+  std::lock_guard<std::mutex> g(c_->work_mu);
+  c_->work_busy = false;
+}
+
+// Sets the context's kept memory to at least `bytes`, unless that is too much.
+void Workspace::resize(size_t bytes) {
+  constexpr size_t kStep = 1 << 20;
+  bytes = (bytes + kStep - 1) / kStep * kStep;
+  if (bytes > kKeepBytes) return;
+  if (c_->work) cudaFreeAsync(c_->work, c_->stream);
+  c_->work = nullptr;
+  c_->work_bytes = 0;
+  if (cudaMallocAsync((void **)&c_->work, bytes, c_->stream) != cudaSuccess) {
+    cudaGetLastError();
+    c_->work = nullptr;
+    return;
+  }
+  c_->work_bytes = bytes;
+}
+
+cudaError_t Workspace::get(void **p, size_t bytes) {
+  *p = nullptr;
+  if (injected_alloc_failure(c_)) return cudaErrorMemoryAllocation;
+  if (!asked_) take();
+  bytes = padded(std::max<size_t>(bytes, 1));
+  want_ += bytes;
+  if (kept_ && used_ + bytes <= c_->work_bytes) {
+    *p = c_->work + used_;
+    used_ += bytes;
+    return cudaSuccess;
+  }
+  if (n_own_ == kOwn) return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMallocAsync(p, bytes, c_->stream);
+  if (e == cudaSuccess)
+    own_[n_own_++] = *p;
+  else
+    *p = nullptr;
+  return e;
 }
 
 void ctx_retain(gd_ctx *c) {
@@ -256,6 +296,7 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
+  if (c->work) cudaFreeAsync(c->work, c->stream);
   shared_detach(c);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -493,7 +534,7 @@ extern "C" gd_status gd_ctx_create(int device, void *stream, gd_ctx **out) {
   if (e != cudaSuccess) {
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
-    return fail(GD_ENOMEM, "pinned host memory and memory pool: %s", cudaGetErrorString(e));
+    return fail(GD_ENOMEM, "pinned host memory: %s", cudaGetErrorString(e));
   }
   // the fixed scratch of gd_energy_poses_noalloc is committed now, not on
   // that entry point's first call
@@ -991,30 +1032,41 @@ gd_status gd::poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int 
   return GD_OK;
 }
 
+static gd_status check_confs(const gd_dcomplex *d, int prt_conf, int lig_conf) {
+  if (prt_conf < 0 || prt_conf >= d->T.n_prt)
+    return fail(GD_EINVAL, "prt_conf %d outside [0, %d)", prt_conf, d->T.n_prt);
+  if (lig_conf < 0 || lig_conf >= d->T.n_lig)
+    return fail(GD_EINVAL, "lig_conf %d outside [0, %d)", lig_conf, d->T.n_lig);
+  return GD_OK;
+}
+
+static size_t cell_bytes(const gd_ctx *ctx, const gd_dcomplex *d, int n_pose) {
+  return pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose);
+}
+
+// A checked pose call on device pointers, with the call's workspace.
+static gd_status poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int lig_conf,
+                           int n_pose, const float *poses, float *terms, double *raw,
+                           Workspace &W) {
+  void *work = nullptr;
+  const size_t bytes = cell_bytes(ctx, d, n_pose);
+  // without room for the cells' workspace the call runs without them
+  if (bytes && W.get(&work, bytes) != cudaSuccess) cudaGetLastError();
+  return poses_launch(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, work);
+}
+
 extern "C" gd_status gd_energy_poses_dev(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf,
                                          int lig_conf, int n_pose, const float *poses,
                                          float *terms, double *raw) {
   NvtxRange nvtx("gd_energy_poses_dev");
   if (!ctx || !d) return fail(GD_EINVAL, "gd_energy_poses_dev: NULL handle");
   if (n_pose < 0) return fail(GD_EINVAL, "n_pose=%d", n_pose);
-  if (prt_conf < 0 || prt_conf >= d->T.n_prt)
-    return fail(GD_EINVAL, "prt_conf %d outside [0, %d)", prt_conf, d->T.n_prt);
-  if (lig_conf < 0 || lig_conf >= d->T.n_lig)
-    return fail(GD_EINVAL, "lig_conf %d outside [0, %d)", lig_conf, d->T.n_lig);
+  GD_TRY(check_confs(d, prt_conf, lig_conf));
   if (n_pose == 0) return GD_OK;
   if (!poses || !terms) return fail(GD_EINVAL, "poses/terms NULL");
   GD_CUDA(cudaSetDevice(ctx->device));
-  void *work = nullptr;
-  const size_t bytes = pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose);
-  // without room for the cells' workspace the call runs without them
-  if (bytes && work_alloc(ctx, &work, bytes) != cudaSuccess) {
-    cudaGetLastError();
-    work = nullptr;
-  }
-  const gd_status st =
-      poses_launch(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, work);
-  if (work) cudaFreeAsync(work, ctx->stream);
-  return st;
+  Workspace W(ctx, cell_bytes(ctx, d, n_pose));
+  return poses_dev(ctx, d, prt_conf, lig_conf, n_pose, poses, terms, raw, W);
 }
 
 extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf,
@@ -1032,7 +1084,7 @@ extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_
   const size_t total = up(pose_b) + up(term_b) + raw_b;
   // a small call passes through the context's pinned memory, which the kernel
   // reads and writes directly: no allocation and no copy in the stream
-  if (total <= kStageBytes && pose_work_bytes(d->T, d->far_share, ctx->n_sm, n_pose) == 0) {
+  if (total <= kStageBytes && cell_bytes(ctx, d, n_pose) == 0) {
     std::unique_lock<std::mutex> lk(ctx->stage_mu, std::try_to_lock);
     if (lk.owns_lock()) {
       unsigned char *p = ctx->stage;
@@ -1048,25 +1100,29 @@ extern "C" gd_status gd_energy_poses(gd_ctx *ctx, const gd_dcomplex *d, int prt_
       return GD_OK;
     }
   }
-  unsigned char *p = nullptr;
+  GD_TRY(check_confs(d, prt_conf, lig_conf));
   gd_status st = GD_OK;
-  cudaError_t e = work_alloc(ctx, (void **)&p, total);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(p, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) {
-    st = fail(GD_ENOMEM, "pose buffers: %s", cudaGetErrorString(e));
-  } else {
-    float *dt = reinterpret_cast<float *>(p + up(pose_b));
-    double *dr = raw ? reinterpret_cast<double *>(p + up(pose_b) + up(term_b)) : nullptr;
-    st = gd_energy_poses_dev(ctx, d, prt_conf, lig_conf, n_pose, reinterpret_cast<float *>(p), dt,
-                             dr);
-    if (st == GD_OK) {
-      e = cudaMemcpyAsync(terms, dt, term_b, cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess && raw)
-        e = cudaMemcpyAsync(raw, dr, raw_b, cudaMemcpyDeviceToHost, ctx->stream);
-      if (e != cudaSuccess) st = fail(GD_ECUDA, "copy back: %s", cudaGetErrorString(e));
+  {
+    // (a workspace that is not kept is given back before the call's last wait)
+    Workspace W(ctx, Workspace::padded(total) + cell_bytes(ctx, d, n_pose));
+    unsigned char *p = nullptr;
+    cudaError_t e = W.get((void **)&p, total);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(p, poses, pose_b, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) {
+      st = fail(GD_ENOMEM, "pose buffers: %s", cudaGetErrorString(e));
+    } else {
+      float *dt = reinterpret_cast<float *>(p + up(pose_b));
+      double *dr = raw ? reinterpret_cast<double *>(p + up(pose_b) + up(term_b)) : nullptr;
+      st = poses_dev(ctx, d, prt_conf, lig_conf, n_pose, reinterpret_cast<float *>(p), dt, dr, W);
+      if (st == GD_OK) {
+        e = cudaMemcpyAsync(terms, dt, term_b, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess && raw)
+          e = cudaMemcpyAsync(raw, dr, raw_b, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e != cudaSuccess) st = fail(GD_ECUDA, "copy back: %s", cudaGetErrorString(e));
+      }
     }
   }
-  if (p) cudaFreeAsync(p, ctx->stream);
   if (st != GD_OK) {
     cudaStreamSynchronize(ctx->stream);
     return st;

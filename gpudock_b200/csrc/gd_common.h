@@ -66,8 +66,8 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 
 }  // namespace gd
 
-// Bytes of workspace kept mapped between calls on a device, and of a context's
-// pinned staging.
+// Most bytes of workspace that a context keeps between calls, and the bytes of
+// its pinned staging.
 namespace gd {
 constexpr size_t kKeepBytes = 64 << 20;
 constexpr size_t kStageBytes = 256 << 10;
@@ -85,11 +85,14 @@ struct gd_ctx {
   // results and pose calls pass, used under stage_mu
   int *h_err = nullptr;
   unsigned char *stage = nullptr;
-  // the calls' own workspaces (poses, similarity): the device's pool of this
-  // library (gd_shared.h, where `shared` is this context's lease)
-  cudaMemPool_t pool = nullptr;
-  void *shared = nullptr;
+  void *shared = nullptr;  // its lease of them (gd_shared.h)
   std::mutex stage_mu;
+  // device memory kept for the calls' workspaces (Workspace), of one call at a
+  // time
+  std::mutex work_mu;
+  bool work_busy = false;
+  unsigned char *work = nullptr;
+  size_t work_bytes = 0;
   uint64_t launches = 0;
   int n_sm = 148;
   int sched_mode = 0;      // GD_SCHED_*
@@ -147,14 +150,36 @@ inline bool injected_alloc_failure(gd_ctx *c) {
   }
   return n == 1;
 }
-// Stream-ordered workspace of a call (freed with cudaFreeAsync).  One that the
-// work pool would not keep comes from the device's default pool, where uploads
-// and runs can have its memory next.
-inline cudaError_t work_alloc(gd_ctx *c, void **p, size_t bytes) {
-  if (injected_alloc_failure(c)) return cudaErrorMemoryAllocation;
-  return bytes > kKeepBytes ? cudaMallocAsync(p, bytes, c->stream)
-                            : cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-}
+// The device memory of one call, all of whose work is on the context's stream
+// (poses, similarity).  It comes from the memory that the context keeps, which
+// the next call's work follows in stream order, so that a repeated call makes no
+// allocation (each took 50 .. 100 us from the device's default pool, which unmaps
+// at every synchronisation; from a pool shared by the device's contexts a call
+// took longer with every context that had used it: 0.10 ms with one, 0.55 with
+// 24).  Another call under way on the context, a call under capture, whose graph
+// may run beside later calls, and what is beyond kKeepBytes take memory of their
+// own from the default pool.
+class Workspace {
+ public:
+  // expect: what the call is likely to need in all
+  Workspace(gd_ctx *c, size_t expect) : c_(c), expect_(expect) {}
+  ~Workspace();
+  Workspace(const Workspace &) = delete;
+  Workspace &operator=(const Workspace &) = delete;
+  static size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+  cudaError_t get(void **p, size_t bytes);
+
+ private:
+  void take();
+  void resize(size_t bytes);
+  gd_ctx *c_;
+  const size_t expect_;
+  bool asked_ = false, kept_ = false;  // kept_: this call has the context's memory
+  size_t used_ = 0, want_ = 0;
+  static constexpr int kOwn = 12;
+  void *own_[kOwn];
+  int n_own_ = 0;
+};
 // Ligand-size bucket: sizes are rounded up to a multiple of 8 atoms; launch
 // shapes are chosen (and autotuned) per bucket and cover its largest size.
 int lna_bucket(int lna);

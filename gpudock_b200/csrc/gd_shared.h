@@ -1,20 +1,18 @@
-// gd_shared.h -- what the contexts of a device share: pinned host blocks and
-// the memory pool of the calls' workspaces.
+// gd_shared.h -- what the contexts of a device share: blocks of pinned memory.
 //
-// Pinning memory takes 1 .. 3 ms up to 1 MB and a pool's first allocation
-// several more, so the contexts of a device have them together, from the first
-// of them to the last.  Both belong to the device's CUDA context and end with
-// it (cudaDeviceReset), whether or not the handles that use them were destroyed
-// first.  So they are kept by device and by the serial number of its CUDA
-// context: a context created after a reset leaves the old group to the handles
-// that still name it and starts a new one, and nothing of a group whose CUDA
-// context is gone is handed out, written or given back to the runtime.  Where
-// the serial number is not to be had (0), every context has a group of its own.
+// Pinning memory takes 1 .. 3 ms up to 1 MB, so a device's contexts share blocks
+// of it, from the first of them to the last.  A block belongs to the device's
+// CUDA context and ends with it (cudaDeviceReset), whether or not the handles
+// that use it were destroyed first.  So blocks are kept by device and by the
+// serial number of its CUDA context: a context created after a reset leaves the
+// old block to the handles that still name it and starts a new one, and nothing
+// of a block whose CUDA context is gone is handed out, written or given back to
+// the runtime.  Where the serial number is not to be had (0), every context has
+// a block of its own.
 //
-// Rt is the runtime (tests put one of their own in its place): the types
-// Error and Pool, ok(Error), serial(), pin(void **, size_t), unpin(void *),
-// pool_create(int device, Pool *), pool_destroy(Pool), all of them about the
-// current device.
+// Rt is the runtime (tests put one of their own in its place): the type Error,
+// ok(Error), serial(), pin(void **, size_t) and unpin(void *), all of them about
+// the current device.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -36,7 +34,6 @@ class DeviceShared {
     int users = 0;
     unsigned char *pinned = nullptr;
     unsigned used = 0;  // a bit per slot of `pinned`
-    typename Rt::Pool pool{};
   };
   // One context's part.
   struct Lease {
@@ -64,11 +61,6 @@ class DeviceShared {
       fresh->serial = serial;
       e = rt_.pin((void **)&fresh->pinned, block_bytes_ * kSlots);
       if (!rt_.ok(e)) return e;
-      e = rt_.pool_create(device, &fresh->pool);
-      if (!rt_.ok(e)) {
-        rt_.unpin(fresh->pinned);
-        return e;
-      }
     }
     Group *g = fresh ? fresh.get() : current;
     Lease l;
@@ -101,10 +93,7 @@ class DeviceShared {
       rt_.unpin(l->block);
     *l = Lease{};
     if (--g->users > 0) return;
-    if (alive) {
-      rt_.unpin(g->pinned);
-      rt_.pool_destroy(g->pool);
-    }
+    if (alive) rt_.unpin(g->pinned);
     Group *&current = current_[g->device];
     if (current == g) current = nullptr;
     delete g;

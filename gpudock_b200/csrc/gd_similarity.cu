@@ -368,22 +368,10 @@ __global__ void __launch_bounds__(kSimThreads)
   }
 }
 
-// Device buffers of one call, freed on every path.
-struct SimBuffers {
-  gd_ctx *ctx;
-  std::vector<void *> ptrs;
-  ~SimBuffers() {
-    for (void *p : ptrs) cudaFreeAsync(p, ctx->stream);
-  }
-  template <typename T>
-  cudaError_t get(T **p, size_t count) {
-    void *v = nullptr;
-    const cudaError_t e = work_alloc(ctx, &v, std::max<size_t>(count, 1) * sizeof(T));
-    if (e == cudaSuccess) ptrs.push_back(v);
-    *p = (T *)v;
-    return e;
-  }
-};
+template <typename T>
+cudaError_t get(Workspace &W, T **p, size_t count) {
+  return W.get((void **)p, count * sizeof(T));
+}
 
 }  // namespace
 }  // namespace gd
@@ -437,23 +425,26 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
   const size_t n = (size_t)n_conf;
   gd_status st = GD_OK;
   {
-    SimBuffers B{ctx, {}};
+    const size_t listed = n * kListed * sizeof(uint32_t) <= kListBytes ? n * kListed : 0;
+    // (the maps' words follow from the contacts: 1 in 16 pairs of the union at most
+    // is what a trajectory near one pocket has)
+    Workspace W(ctx, 4096 + sizeof(SimConf) * n + 8 * K + 4 * (n + listed + n * (K / 16)) +
+                         (S_dev ? 0 : sizeof(float) * n * n));
     SimConf *d_conf = nullptr;
     uint32_t *d_uni = nullptr, *d_maps = nullptr;
     float *d_bound = nullptr, *d_S = nullptr;
     int *d_pop = nullptr, *d_base = nullptr;
     uint32_t *d_listed = nullptr;
-    cudaError_t e = B.get(&d_conf, n);
-    if (e == cudaSuccess) e = B.get(&d_uni, K);
-    if (e == cudaSuccess) e = B.get(&d_bound, (size_t)GD_NLT * 32);
-    if (e == cudaSuccess) e = B.get(&d_pop, n);
-    if (e == cudaSuccess) e = B.get(&d_base, K + 1);
-    if (e == cudaSuccess && n * kListed * sizeof(uint32_t) <= kListBytes &&
-        B.get(&d_listed, n * kListed) != cudaSuccess) {
+    cudaError_t e = get(W, &d_conf, n);
+    if (e == cudaSuccess) e = get(W, &d_uni, K);
+    if (e == cudaSuccess) e = get(W, &d_bound, (size_t)GD_NLT * 32);
+    if (e == cudaSuccess) e = get(W, &d_pop, n);
+    if (e == cudaSuccess) e = get(W, &d_base, K + 1);
+    if (e == cudaSuccess && listed && get(W, &d_listed, listed) != cudaSuccess) {
       cudaGetLastError();  // without room for the lists the contacts are tested twice
       d_listed = nullptr;
     }
-    if (e == cudaSuccess && !S_dev) e = B.get(&d_S, n * n);
+    if (e == cudaSuccess && !S_dev) e = get(W, &d_S, n * n);
     if (S_dev) d_S = S_dev;
     if (e != cudaSuccess) return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
     GD_CUDA(cudaMemcpyAsync(d_conf, hc.data(), sizeof(SimConf) * n, cudaMemcpyHostToDevice, s));
@@ -470,7 +461,7 @@ static gd_status similarity_run(gd_ctx *ctx, const gd_dcomplex *d, int n_conf,
     GD_CUDA(cudaStreamSynchronize(s));
     const int Kp = (n_bits + 32 * kPairChunk - 1) / (32 * kPairChunk) * kPairChunk;
     if (Kp) {
-      e = B.get(&d_maps, n * (size_t)Kp);
+      e = get(W, &d_maps, n * (size_t)Kp);
       if (e != cudaSuccess)
         return fail(GD_ENOMEM, "similarity buffers: %s", cudaGetErrorString(e));
       const bool row = Kp <= kRowWords;

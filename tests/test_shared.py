@@ -11,22 +11,18 @@ FAKE = r"""
 #include <set>
 #include "gd_shared.h"
 struct State {
-  int device = 0, pins = 0, pools = 0, fail_in = 0, next_pool = 1;
+  int device = 0, pins = 0, fail_in = 0;
   std::map<int, uint64_t> serial{{0, 7}, {1, 8}};
   std::map<void *, uint64_t> pinned;   // live blocks, by the serial they belong to
-  std::map<int, uint64_t> pool;
   bool wrong = false;                  // something dead was given back
   void reset(int d, uint64_t s) {      // everything of the old CUDA context goes
     for (auto it = pinned.begin(); it != pinned.end();)
       if (it->second == serial[d]) { std::free(it->first); it = pinned.erase(it); } else ++it;
-    for (auto it = pool.begin(); it != pool.end();)
-      if (it->second == serial[d]) it = pool.erase(it); else ++it;
     serial[d] = s;
   }
 };
 struct Fake {
   using Error = int;
-  using Pool = int;
   State *s;
   static bool ok(int e) { return e == 0; }
   uint64_t serial() { return s->serial[s->device]; }
@@ -44,14 +40,6 @@ struct Fake {
     std::free(p);
     s->pinned.erase(it);
   }
-  int pool_create(int, int *out) {
-    if (fails()) return 2;
-    s->pool[s->next_pool] = serial();
-    s->pools++;
-    *out = s->next_pool++;
-    return 0;
-  }
-  void pool_destroy(int p) { if (!s->pool.erase(p)) s->wrong = true; }
 };
 using Shared = gd::DeviceShared<Fake>;
 using Lease = Shared::Lease;
@@ -67,13 +55,13 @@ bool live(State &s, const Lease &l, size_t n) {
 
 CASES = {
     # six contexts, released out of order and taken again: blocks are distinct,
-    # one pool, and everything goes with the last of them
+    # everything goes with the last of them
     "mixed_order": r"""
   State s;
   Shared S(512, Fake{&s});
   Lease l[6];
   for (auto &x : l) CHECK(S.acquire(0, &x) == 0);
-  CHECK(s.pools == 1 && s.pins == 3);  // a block of four, two of their own
+  CHECK(s.pins == 3);  // a block of four, two of their own
   std::set<void *> seen;
   for (auto &x : l) { seen.insert(x.block); CHECK(live(s, x, 512)); }
   CHECK(seen.size() == 6);
@@ -87,9 +75,8 @@ CASES = {
   CHECK(S.acquire(0, &l[1]) == 0 && s.pins == 3);
   CHECK(again.block == b1 || l[1].block == b1);
   for (Lease *x : {&l[3], &again, &l[5], &l[1]}) S.release(x);
-  CHECK(s.pool.size() == 1);
   S.release(&l[2]);
-  CHECK(s.pool.empty() && s.pinned.empty() && !s.wrong);
+  CHECK(s.pinned.empty() && !s.wrong);
   S.release(&l[2]);  // a lease is given back once
 """,
     # the block of device 1's context is not device 0's to take away
@@ -103,29 +90,29 @@ CASES = {
   s.device = 0;
   S.release(&a);
   s.reset(0, 9);
-  CHECK(live(s, b, 512) && s.pool.count(b.group->pool));
+  CHECK(live(s, b, 512));
   s.device = 1;
   S.release(&b);
-  CHECK(s.pool.empty() && s.pinned.empty() && !s.wrong);
+  CHECK(s.pinned.empty() && !s.wrong);
 """,
-    # a reset under live contexts: the next context gets a block and a pool that
-    # exist, and releasing the old ones later gives nothing dead back
+    # a reset under live contexts: the next context gets a block that
+    # exists, and releasing the old ones later gives nothing dead back
     "reset": r"""
   State s;
   Shared S(512, Fake{&s});
   Lease old[6], now[2];
   for (auto &x : old) CHECK(S.acquire(0, &x) == 0);
   s.reset(0, 9);
-  CHECK(S.acquire(0, &now[0]) == 0 && live(s, now[0], 512) && s.pool.count(now[0].group->pool));
+  CHECK(S.acquire(0, &now[0]) == 0 && live(s, now[0], 512));
   S.release(&old[5]);
   S.release(&old[0]);
   CHECK(S.acquire(0, &now[1]) == 0 && live(s, now[1], 512));
   CHECK(now[0].block != now[1].block && now[0].group == now[1].group);
   for (int k : {1, 2, 3, 4}) S.release(&old[k]);
-  CHECK(live(s, now[0], 512) && s.pool.size() == 1 && !s.wrong);
+  CHECK(live(s, now[0], 512) && !s.wrong);
   S.release(&now[0]);
   S.release(&now[1]);
-  CHECK(s.pool.empty() && s.pinned.empty() && !s.wrong);
+  CHECK(s.pinned.empty() && !s.wrong);
 """,
     # no serial number: nothing is shared
     "unknown": r"""
@@ -133,26 +120,24 @@ CASES = {
   s.serial[0] = 0;
   Shared S(512, Fake{&s});
   Lease a, b;
-  CHECK(S.acquire(0, &a) == 0 && S.acquire(0, &b) == 0 && a.group != b.group && s.pools == 2);
+  CHECK(S.acquire(0, &a) == 0 && S.acquire(0, &b) == 0 && a.group != b.group && s.pins == 2);
   S.release(&a);
   CHECK(live(s, b, 512));
   S.release(&b);
-  CHECK(s.pool.empty() && s.pinned.empty() && !s.wrong);
+  CHECK(s.pinned.empty() && !s.wrong);
 """,
-    # the block, the pool or a fifth context's own block cannot be had
+    # the block or a fifth context's own cannot be had
     "failures": r"""
   State s;
   Shared S(512, Fake{&s});
   Lease l[5];
-  for (int k : {1, 2}) {
-    s.fail_in = k;
-    CHECK(S.acquire(0, &l[0]) != 0 && s.pool.empty() && s.pinned.empty());
-  }
+  s.fail_in = 1;
+  CHECK(S.acquire(0, &l[0]) != 0 && s.pinned.empty());
   for (int k = 0; k < 4; ++k) CHECK(S.acquire(0, &l[k]) == 0);
   s.fail_in = 1;
-  CHECK(S.acquire(0, &l[4]) != 0 && s.pool.size() == 1 && s.pinned.size() == 1);
+  CHECK(S.acquire(0, &l[4]) != 0 && s.pinned.size() == 1);
   for (int k = 0; k < 4; ++k) S.release(&l[k]);
-  CHECK(s.pool.empty() && s.pinned.empty() && !s.wrong);
+  CHECK(s.pinned.empty() && !s.wrong);
 """,
 }
 
