@@ -288,19 +288,19 @@ bool pose_cells_pay(const KTables &T, double far_share, int n_sm, int n_pose) {
   if (2 * units <= n_sm) return false;
   // Else the waves of blocks, times a block's time (6 pairs per ns and SM), with
   // the cells' half-filled last blocks and the deal on one side.  Were all points
-  // far they would take 0.4 of a block's time off it on average, less where a wave
-  // lasts as long as its slowest block, and the lists add 0.05; poses away from
-  // the start place have more far points than far_share says.  Measured, cells
-  // against without: 4,700 x 96 x 700 (a second wave) 856 and 442 us; 4,096 x 24 x
-  // 1,500 216 and 212; 16,384 of them 783 and 819; 20,000 x 96 x 700 (1% of the
-  // points far) 2,226 and 2,112; 131,072 x 48 x 2,000 12.6 and 14.3 ms; 30,011 x
-  // 48 x 8,000 9.0 and 12.2 ms.
+  // far they would take 0.4 of a block's time off it, and the lists add 0.05; poses
+  // away from the start place have more far points than far_share says.  Measured,
+  // cells against without: 4,700 x 96 x 700 (a second wave) 856 and 442 us; 2,900 x
+  // 48 x 1,000 (6% of the points far) 327 and 310; 4,096 x 24 x 1,500 (34%) 165 and
+  // 178 among other calls, whose blocks start as the shorter ones end, 216 and 212
+  // one after another; 16,384 of them 783 and 819; 131,072 x 48 x 2,000 12.6 and
+  // 14.3 ms; 30,011 x 48 x 8,000 9.0 and 12.2 ms.
   const double cells = max_cells(n_pose);
   const double blocks = units + 0.5 * cells + std::sqrt(cells);
   const double w0 = std::ceil((double)units / n_sm), w1 = std::ceil(blocks / n_sm);
   const double block_us = 32.0 * T.lna * T.pnp / 6000.0;
   const double deal_us = n_pose <= kSmallPoses ? 6.0 + n_pose / 800.0 : 20.0 + n_pose / 4000.0;
-  const double block = 1.05 - 0.4 * far_share * (1.0 - 0.4 / w1);
+  const double block = 1.05 - 0.4 * far_share;
   return w1 * block_us * block + deal_us < w0 * block_us;
 }
 

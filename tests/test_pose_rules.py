@@ -39,6 +39,8 @@ def test_cells_only_where_they_pay(tmp_path):
   // many waves: from about a third of the points on
   CHECK(cells(131072, 48, 2000, 0.36) && !cells(131072, 48, 2000, 0.2));
   CHECK(cells(30011, 48, 8000, 0.79) && cells(12345, 96, 6000, 0.7) && cells(16384, 24, 1500, 0.34));
+  // one wave of blocks
+  CHECK(cells(4096, 24, 1500, 0.34) && !cells(4096, 24, 1500, 0.1) && !cells(2900, 48, 1000, 0.06));
   // a few points: the deal takes longer than it saves
   CHECK(!cells(20000, 8, 100, 0.9));
   // wherever the SMs are many or few, no cells on half of them
