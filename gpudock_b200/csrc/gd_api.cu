@@ -126,9 +126,11 @@ Tile tile_for(gd_ctx *ctx, const KTables &T) {
   return default_tile(hi);
 }
 
-// The runtime behind the contexts' shared pinned blocks (gd_shared.h).
+// The runtime behind what a device's contexts share (gd_shared.h).
 struct CudaShared {
   using Error = cudaError_t;
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
   static bool ok(Error e) { return e == cudaSuccess; }
   // Serial number of the device's CUDA context, which no later one of the
   // process has (0: this driver does not tell).
@@ -154,20 +156,36 @@ struct CudaShared {
   }
   static Error pin(void **p, size_t bytes) { return cudaHostAlloc(p, bytes, cudaHostAllocDefault); }
   static void unpin(void *p) { cudaFreeHost(p); }
+  static Error alloc(void **p, size_t bytes, Stream s) {
+    const cudaError_t e = cudaMallocAsync(p, bytes, s);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+  }
+  static void free(void *p, Stream s) { cudaFreeAsync(p, s); }
+  static Error event(Event *e) { return cudaEventCreateWithFlags(e, cudaEventDisableTiming); }
+  static Error record(Event e, Stream s) { return cudaEventRecord(e, s); }
+  static bool done(Event e) {
+    const cudaError_t q = cudaEventQuery(e);
+    if (q != cudaSuccess && q != cudaErrorNotReady) cudaGetLastError();
+    return q == cudaSuccess;
+  }
+  static void drop(Event e) { cudaEventDestroy(e); }
 };
 
 // Never destroyed: a handle may be released while the process ends.
-static DeviceShared<CudaShared> &shared() {
-  static auto *s = new DeviceShared<CudaShared>(256 + kStageBytes);
+using Shared = DeviceShared<CudaShared>;
+static Shared &shared() {
+  static auto *s = new Shared(256 + kStageBytes, kKeepBytes);
   return *s;
 }
+static Shared::Group *group_of(gd_ctx *c) { return static_cast<Shared::Lease *>(c->shared)->group; }
 
 // The context's error word and staging.
 static cudaError_t shared_attach(gd_ctx *c) {
-  DeviceShared<CudaShared>::Lease *l = nullptr;
+  Shared::Lease *l = nullptr;
   cudaError_t e = cudaErrorMemoryAllocation;
   try {
-    l = new DeviceShared<CudaShared>::Lease;
+    l = new Shared::Lease;
     e = shared().acquire(c->device, l);
   } catch (const std::bad_alloc &) {
   }
@@ -183,16 +201,15 @@ static cudaError_t shared_attach(gd_ctx *c) {
 }
 
 static void shared_detach(gd_ctx *c) {
-  auto *l = static_cast<DeviceShared<CudaShared>::Lease *>(c->shared);
+  auto *l = static_cast<Shared::Lease *>(c->shared);
   if (!l) return;
-  shared().release(l);
+  shared().release(l, c, c->stream);
   delete l;
   c->shared = nullptr;
 }
 
-// The context's memory for this call, if no other call has it and the stream is
-// not under capture.
-void Workspace::take() {
+// A slab for this call, unless the stream is under capture.
+void Workspace::take(size_t bytes) {
   asked_ = true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
   if (cudaStreamIsCapturing(c_->stream, &cap) != cudaSuccess) {
@@ -200,46 +217,27 @@ void Workspace::take() {
     return;
   }
   if (cap != cudaStreamCaptureStatusNone) return;
-  {
-    std::lock_guard<std::mutex> g(c_->work_mu);
-    if (c_->work_busy) return;
-    c_->work_busy = kept_ = true;
-  }
-  if (expect_ > c_->work_bytes) resize(expect_);
+  Shared::Slab *b = shared().lend(group_of(c_), c_, c_->stream, bytes);
+  if (!b) return;
+  slab_ = b;
+  base_ = b->p;
+  room_ = b->bytes;
 }
 
 Workspace::~Workspace() {
   for (int k = 0; k < n_own_; ++k) cudaFreeAsync(own_[k], c_->stream);
-  if (!kept_) return;
-  if (want_ > c_->work_bytes) resize(want_);  // for the next such call
-  std::lock_guard<std::mutex> g(c_->work_mu);
-  c_->work_busy = false;
-}
-
-// Sets the context's kept memory to at least `bytes`, unless that is too much.
-void Workspace::resize(size_t bytes) {
-  constexpr size_t kStep = 1 << 20;
-  bytes = (bytes + kStep - 1) / kStep * kStep;
-  if (bytes > kKeepBytes) return;
-  if (c_->work) cudaFreeAsync(c_->work, c_->stream);
-  c_->work = nullptr;
-  c_->work_bytes = 0;
-  if (cudaMallocAsync((void **)&c_->work, bytes, c_->stream) != cudaSuccess) {
-    cudaGetLastError();
-    c_->work = nullptr;
-    return;
-  }
-  c_->work_bytes = bytes;
+  if (slab_)
+    shared().give_back(group_of(c_), static_cast<Shared::Slab *>(slab_), c_, c_->stream, want_);
 }
 
 cudaError_t Workspace::get(void **p, size_t bytes) {
   *p = nullptr;
   if (injected_alloc_failure(c_)) return cudaErrorMemoryAllocation;
-  if (!asked_) take();
   bytes = padded(std::max<size_t>(bytes, 1));
+  if (!asked_) take(std::max(expect_, bytes));
   want_ += bytes;
-  if (kept_ && used_ + bytes <= c_->work_bytes) {
-    *p = c_->work + used_;
+  if (used_ + bytes <= room_) {
+    *p = base_ + used_;
     used_ += bytes;
     return cudaSuccess;
   }
@@ -296,7 +294,6 @@ void ctx_release(gd_ctx *c) {
   }
   for (cudaEvent_t e : c->side_done) cudaEventDestroy(e);
   if (c->forked) cudaEventDestroy(c->forked);
-  if (c->work) cudaFreeAsync(c->work, c->stream);
   shared_detach(c);
   if (c->own_stream) cudaStreamDestroy(c->stream);
   delete c;

@@ -66,8 +66,8 @@ void pick_stages(const KTables &T, const Tile &t, int *n_stages, int *resident, 
 
 }  // namespace gd
 
-// Most bytes of workspace that a context keeps between calls, and the bytes of
-// its pinned staging.
+// Most bytes of workspace kept between calls on a device, and the bytes of a
+// context's pinned staging.
 namespace gd {
 constexpr size_t kKeepBytes = 64 << 20;
 constexpr size_t kStageBytes = 256 << 10;
@@ -87,12 +87,6 @@ struct gd_ctx {
   unsigned char *stage = nullptr;
   void *shared = nullptr;  // its lease of them (gd_shared.h)
   std::mutex stage_mu;
-  // device memory kept for the calls' workspaces (Workspace), of one call at a
-  // time
-  std::mutex work_mu;
-  bool work_busy = false;
-  unsigned char *work = nullptr;
-  size_t work_bytes = 0;
   uint64_t launches = 0;
   int n_sm = 148;
   int sched_mode = 0;      // GD_SCHED_*
@@ -151,14 +145,13 @@ inline bool injected_alloc_failure(gd_ctx *c) {
   return n == 1;
 }
 // The device memory of one call, all of whose work is on the context's stream
-// (poses, similarity).  It comes from the memory that the context keeps, which
-// the next call's work follows in stream order, so that a repeated call makes no
-// allocation (each took 50 .. 100 us from the device's default pool, which unmaps
-// at every synchronisation; from a pool shared by the device's contexts a call
-// took longer with every context that had used it: 0.10 ms with one, 0.55 with
-// 24).  Another call under way on the context, a call under capture, whose graph
-// may run beside later calls, and what is beyond kKeepBytes take memory of their
-// own from the default pool.
+// (poses, similarity): a slab that the device's contexts keep (gd_shared.h), so
+// that a repeated call makes no allocation.  (Each took 50 .. 100 us from the
+// device's default pool, which unmaps at every synchronisation; from a pool
+// shared by the device's contexts a call took longer with every context that had
+// used it: 0.10 ms with one, 0.55 with 24.)  A call under capture, whose graph may
+// run beside later calls, one that finds no slab and what is beyond kKeepBytes
+// take memory of their own from the default pool.
 class Workspace {
  public:
   // expect: what the call is likely to need in all
@@ -170,12 +163,13 @@ class Workspace {
   cudaError_t get(void **p, size_t bytes);
 
  private:
-  void take();
-  void resize(size_t bytes);
+  void take(size_t bytes);
   gd_ctx *c_;
   const size_t expect_;
-  bool asked_ = false, kept_ = false;  // kept_: this call has the context's memory
-  size_t used_ = 0, want_ = 0;
+  bool asked_ = false;
+  void *slab_ = nullptr;  // (DeviceShared::Slab)
+  unsigned char *base_ = nullptr;
+  size_t room_ = 0, used_ = 0, want_ = 0;
   static constexpr int kOwn = 12;
   void *own_[kOwn];
   int n_own_ = 0;

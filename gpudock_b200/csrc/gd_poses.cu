@@ -286,21 +286,30 @@ bool pose_cells_pay(const KTables &T, double far_share, int n_sm, int n_pose) {
   // on clusters of two.
   const int units = (n_pose + 31) / 32;
   if (2 * units <= n_sm) return false;
-  // Else the waves of blocks, times a block's time (6 pairs per ns and SM), with
-  // the cells' half-filled last blocks and the deal on one side.  Were all points
-  // far they would take 0.4 of a block's time off it, and the lists add 0.05; poses
-  // away from the start place have more far points than far_share says.  Measured,
-  // cells against without: 4,700 x 96 x 700 (a second wave) 856 and 442 us; 2,900 x
-  // 48 x 1,000 (6% of the points far) 327 and 310; 4,096 x 24 x 1,500 (34%) 165 and
-  // 178 among other calls, whose blocks start as the shorter ones end, 216 and 212
-  // one after another; 16,384 of them 783 and 819; 131,072 x 48 x 2,000 12.6 and
-  // 14.3 ms; 30,011 x 48 x 8,000 9.0 and 12.2 ms.
-  const double cells = max_cells(n_pose);
-  const double blocks = units + 0.5 * cells + std::sqrt(cells);
-  const double w0 = std::ceil((double)units / n_sm), w1 = std::ceil(blocks / n_sm);
+  // Else the waves of blocks (from four on the SMs take them as they come), times
+  // a block's time (6 pairs per ns and SM), with the cells' half-filled last blocks
+  // and the deal on one side.  A block's time was fitted to calls whose poses lie
+  // 1 to 4 A about the start place, where most have more far points than the share
+  // there says; in few waves, which last as long as their slowest blocks, less is
+  // gained.  Measured, cells against without (box in A, share): 4,700 x 96 x 700 (a
+  // second wave) 856 and 442 us; 2,900 x 48 x 1,000 (4, 0.06) 327 and 310; 4,096 x
+  // 24 x 1,500 (4, 0.34) 165 and 178 among other calls, whose blocks start as the
+  // shorter ones end, 215 and 212 one after another; 60,000 x 48 x 900 (6, 0.02)
+  // 3.83 and 3.68 ms; 40,000 x 40 x 700 (2, 0.08) 1.56 and 1.51; 50,000 x 60 x 1,300
+  // (6, 0.07) 5.67 and 6.01; 100,000 x 20 x 800 (8, 0.12) 2.86 and 3.16; 131,072 x 48
+  // x 2,000 (8, 0.21) 13.8 and 14.9, (8, 0.36) 12.6 and 14.2; 30,011 x 48 x 8,000 (8,
+  // 0.79) 9.0 and 12.2.
+  const double cells = max_cells(n_pose), f = far_share;
+  const double units_with = units + 0.5 * cells;
   const double block_us = 32.0 * T.lna * T.pnp / 6000.0;
   const double deal_us = n_pose <= kSmallPoses ? 6.0 + n_pose / 800.0 : 20.0 + n_pose / 4000.0;
-  const double block = 1.05 - 0.4 * far_share;
+  double w0 = (double)units / n_sm, w1 = units_with / n_sm;
+  double block = 1.02 - 0.95 * f + 0.65 * f * f;
+  if (w0 < 4.0) {
+    w0 = std::ceil(w0);
+    w1 = std::ceil((units_with + std::sqrt(cells)) / n_sm);
+    block = 1.05 - 0.45 * f;
+  }
   return w1 * block_us * block + deal_us < w0 * block_us;
 }
 

@@ -36,8 +36,9 @@ def test_cells_only_where_they_pay(tmp_path):
   CHECK(cells(8600, 96, 6000, 0.7) && !cells(9400, 96, 6000, 0.7));
   // nothing far: at no size
   for (int n = 2048; n < 2000000; n += n / 7) CHECK(!cells(n, 96, 700, 0.01));
-  // many waves: from about a third of the points on
-  CHECK(cells(131072, 48, 2000, 0.36) && !cells(131072, 48, 2000, 0.2));
+  // many waves
+  CHECK(cells(131072, 48, 2000, 0.36) && cells(131072, 48, 2000, 0.21));
+  CHECK(cells(100000, 20, 800, 0.12) && !cells(60000, 48, 900, 0.02));
   CHECK(cells(30011, 48, 8000, 0.79) && cells(12345, 96, 6000, 0.7) && cells(16384, 24, 1500, 0.34));
   // one wave of blocks
   CHECK(cells(4096, 24, 1500, 0.34) && !cells(4096, 24, 1500, 0.1) && !cells(2900, 48, 1000, 0.06));
