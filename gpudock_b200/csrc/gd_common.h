@@ -183,12 +183,15 @@ Tile tile_for(gd_ctx *ctx, const KTables &T);
 gd_status poses_launch(gd_ctx *ctx, const gd_dcomplex *d, int prt_conf, int lig_conf, int n_pose,
                        const float *poses, float *terms, double *raw, void *work);
 // CTAs (a thread-block cluster) that share each 32-replica unit of a complex
-// in MC launches: a function of the complex (ligand-size bucket x protein
-// points) and of the units of its own run, never of what else runs, so
-// results are the same in any mix.  The largest power of two <= cost /
-// min_cost and <= SMs / units, at most 8.  Runs (gd_remc, gd_batch) have the
-// GPU to themselves and split down to kRunSplitCost pairs per CTA; a server
-// request is a run of its own among others and splits only from
+// in MC launches.  The order of the FP64 sums, and so a run's last bits, depend on
+// it.  split_rule: a function of the complex (ligand-size bucket x protein points)
+// and of run_units, the units that want SMs with it; for a server request those
+// of its own run, never of what else runs, so a request's results do not depend on
+// the server's load.  In a run or batch, run_splits (gd_ensemble.cu) deals the
+// SMs over all its complexes, the costliest first: a complex's split there follows
+// from the sizes of the others too.
+// min_cost: pairs per CTA that a split must leave.  Runs and batches have the GPU
+// to themselves: kRunSplitCost.  Server requests share it with one another:
 // kServeSplitCost, so that splitting under load costs little throughput.
 constexpr double kRunSplitCost = 4500.0;
 constexpr double kServeSplitCost = 42500.0;

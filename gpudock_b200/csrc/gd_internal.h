@@ -173,10 +173,10 @@ struct KRun {
   int step0, n_steps;
   const int *step_ptr;
   int item_step;
-  int split;             // REMC / INIT without a schedule: clusters of `split`
-                         // CTAs (<= 8) share each unit, CTA rank r taking the
-                         // protein tiles r, r + split, ... (grid = units x split);
-                         // 0 or 1: one CTA per unit
+  int split;             // without a schedule: clusters of `split` CTAs (<= 8)
+                         // share each unit, CTA rank r taking the protein's
+                         // chunks r, r + split, ... (grid = units x split); 0 or
+                         // 1: one CTA per unit
   int packed;            // REMC / INIT: nonzero when every unit of the launch has
                          // at most 16 replicas (packed_reps < 32); POSES: poses
                          // per unit (8 or 16), or 0 for 32

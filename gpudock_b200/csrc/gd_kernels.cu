@@ -556,8 +556,8 @@ __device__ __forceinline__ float4 entry_point(const unsigned char *smem, uint32_
 
 // n points of a list (n >= 1) for each of the `subs` point subsets of the
 // lanes (PACKED; else one): list points at this lane's first entry, its next
-// ones follow at distance subs.  Returns the mask of the iterations in which some lane has a
-// close-range term.
+// ones follow at distance subs.  Returns the mask of the iterations in which some
+// lane has a close-range term.
 template <int NH, int NHB, bool PACKED>
 __device__ __forceinline__ uint32_t chunk_fast(const float2 (&nx)[NH], const float2 (&ny)[NH],
                                                const float2 (&nz)[NH],
@@ -648,8 +648,8 @@ __device__ __forceinline__ void chunk_far(const float2 (&nx)[NH], const float2 (
 
 // One point beyond far[ag][pt] of every atom of the warp in every lane, as
 // pair_block1 evaluates it to the bit: there 2^x < 2^-25, so D1 D2 rounds to D1
-// and num1 D2 to num1, the H-bond Gaussian is 0 and no close-range term applies; 17 packed FMA-pipe and 4 MUFU instructions per atom pair against
-// its 22 and 6.
+// and num1 D2 to num1, the H-bond Gaussian is 0 and no close-range term applies;
+// 17 packed FMA-pipe and 4 MUFU instructions per atom pair against its 22 and 6.
 template <int NH>
 __device__ __forceinline__ void far_block1(const float2 (&nx)[NH], const float2 (&ny)[NH],
                                            const float2 (&nz)[NH], const float4 &A0,
@@ -693,7 +693,7 @@ __device__ __forceinline__ void far_block1(const float2 (&nx)[NH], const float2 
 // the headline, but change the last bits of the sums and with them one
 // Metropolis decision in 300,000.  One point per iteration: four bodies share
 // the instruction caches.  20-step interval of the headline: 27.0 ms without
-// the far form, 23.8 with it (the points within 16 A of some atom of the warp
+// the far form, 24.2 with it (the points within 16 A of some atom of the warp
 // in some lane, 37 .. 50%, still take the full form).  Bound by issue and by
 // the XU and FMA pipes together.  Returns the mask of the points that some lane
 // has a close-range term with.
@@ -983,7 +983,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   const int A = R.A, P = R.P, W = A * P, NS = R.n_stages;
   const int MAXA = A * NA;
   // split launch: clusters of csize CTAs, rank crank, share one unit; CTA
-  // crank takes the protein tiles crank, crank + csize, ...
+  // crank takes the protein's chunks crank, crank + csize, ...
   const int csize = (!PIECES && R.split > 1) ? R.split : 1;
   const SmemLayout SL = smem_layout(A, P, NA, NS, csize, kLists);
   float4 *s_ptab = reinterpret_cast<float4 *>(smem + SL.ptab);
@@ -1527,7 +1527,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
           if (!far_l)
             at = (close_m >> lane) & 1u ? __popc(close_m & below)
                                         : __popc(close_m) + __popc(near_m & ~close_m & below);
-          my_list[at] = make_uint2(list_entry(tile_at + (uint32_t)jl * 16u, pt_l), __float_as_uint(thr_l));
+          my_list[at] = make_uint2(list_entry(tile_at + (uint32_t)jl * 16u, pt_l),
+                                   __float_as_uint(thr_l));
         }
         if (subs > 1) {  // padding points fill both parts
           if (n_near + lane < far0) my_list[n_near + lane] = pad_entry;
@@ -1714,7 +1715,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
         if (i < NRED) {
           double v[MAX_SPLIT];
 #pragma unroll
-          for (int r = 0; r < MAX_SPLIT; ++r) v[r] = r < csize ? cluster_map(xs, r)[i * 32 + rl] : 0.0;
+          for (int r = 0; r < MAX_SPLIT; ++r)
+            v[r] = r < csize ? cluster_map(xs, r)[i * 32 + rl] : 0.0;
           double acc = 0.0;
 #pragma unroll
           for (int r = 0; r < MAX_SPLIT; ++r) acc += v[r];
@@ -1932,8 +1934,8 @@ static cudaError_t launch_kernel(const KRun &R, int grid, cudaStream_t s, int *o
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (occ)  // occupancy query instead of a launch
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, dock_kernel<MODE, NA, HB, PIECES, FORM>,
-                                                         threads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        occ, dock_kernel<MODE, NA, HB, PIECES, FORM>, threads, smem);
   if (split == 1) {
     dock_kernel<MODE, NA, HB, PIECES, FORM><<<grid, threads, smem, s>>>(R);
     return cudaGetLastError();

@@ -51,7 +51,9 @@ constexpr int kCandidates = 2048;  // points looked at per round
 constexpr int kRowWords = 8192;    // largest map kept in shared memory
 // Contacts of a conformation kept from the first pass for the second (a
 // conformation with more is tested again), while the lists of all take at most
-// kListBytes.
+// kListBytes: up to 4,096 conformations; a call with more tests every contact
+// twice (3,001 conformations: the second pass 10 us with lists, 143 us as the
+// first).
 constexpr int kListed = 2048;
 constexpr size_t kListBytes = 32 << 20;
 
@@ -79,8 +81,8 @@ __global__ void bound_kernel(const float4 *tab, float *bound) {
 // as the conformation's map of Kp words, bits numbered by the contact's rank
 // in the union, from the list that the first pass kept, or tested again.  Bound
 // by latency and L2 reads of the points: the atoms are tested against the few
-// points within reach of the ligand's box (600 conformations x 40 x 4,000: 27 us;
-// testing every pair took 227 us).
+// points within reach of the ligand's box (600 conformations x 40 x 4,000, caches
+// cold: 42 us; testing every pair took 230 us).
 template <bool MAPS>
 __global__ void __launch_bounds__(kSimThreads)
     contacts_kernel(KTables T, const SimConf *confs, const float *bound, uint32_t *uni, int *pop,
@@ -276,9 +278,9 @@ __device__ __forceinline__ void tile_of(int t, int tiles, int *row, int *col) {
 }
 
 // Entries of the matrix.  With a bit per contact of the union, in place of the
-// 32-bit words that hold one, the maps are several times shorter: 600
-// conformations 145 -> 17 us, 3,001 (upper triangle only) 9.3 -> 0.66 ms for the
-// whole call.  Bound by the ALU pipe (carry-save counting).
+// 32-bit words that hold one, the maps are several times shorter, and only the
+// upper triangle's tiles are counted: 600 conformations 261 -> 24 us, 3,001 3,890
+// -> 156 us.  Bound by the ALU pipe (carry-save counting).
 __global__ void __launch_bounds__(kSimThreads)
     pairs_kernel(const uint32_t *comp, const int *pop, int n, int Kp, int total, int tiles,
                  float *S) {

@@ -362,8 +362,9 @@ gd_status gd_ctx_set_schedule_tail(gd_ctx *ctx, int tail);
  * little throughput: 120 atoms against 10,000 points on 8 CTAs, 30 atoms
  * against 4,000 on 2); 1, 2, 4 or 8 fix it for every complex.  A run's
  * results depend on its split (the partial sums are added in another
- * order) but never on what runs beside it.  Applies to runs, batches and
- * server lanes created after the call. */
+ * order) but never on what runs beside it; in a batch the split of a
+ * complex follows from the sizes of the batch's other complexes too.
+ * Applies to runs, batches and server lanes created after the call. */
 gd_status gd_ctx_set_split(gd_ctx *ctx, int split);
 
 /* ------------------------------------------------------------------------ */
