@@ -29,7 +29,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <utility>
 
 namespace gd {
 
@@ -132,7 +131,17 @@ class DeviceShared {
     bytes = (bytes + kStep - 1) / kStep * kStep;
     if (bytes > keep_) return nullptr;
     std::lock_guard<std::mutex> lk(mu_);
-    Slab *fit = nullptr, *small = nullptr, *none = nullptr;
+    Slab *fit = nullptr;
+    // the user's own first: no event is queried then (another thread of the
+    // process may have a stream under capture, which a query can end)
+    for (Slab &b : g->slabs)
+      if (b.p && !b.lent && b.user == user && b.bytes >= bytes && (!fit || b.bytes < fit->bytes))
+        fit = &b;
+    if (fit) {
+      fit->lent = true;
+      return fit;
+    }
+    Slab *small = nullptr, *none = nullptr;
     size_t total = 0;
     for (Slab &b : g->slabs) {
       total += b.bytes;
@@ -140,7 +149,7 @@ class DeviceShared {
       if (!b.p || !free_for(b, user)) continue;
       if (b.bytes < bytes) {
         if (!small || b.bytes < small->bytes) small = &b;
-      } else if (!fit || rank(b, user) < rank(*fit, user)) {
+      } else if (!fit || b.bytes < fit->bytes) {
         fit = &b;
       }
     }
@@ -177,10 +186,6 @@ class DeviceShared {
  private:
   bool free_for(const Slab &b, const void *user) {
     return !b.lent && (b.user == user || rt_.done(b.done));
-  }
-  // the user's own first, then the smallest
-  static std::pair<int, size_t> rank(const Slab &b, const void *user) {
-    return {b.user == user ? 0 : 1, b.bytes};
   }
   bool make(Slab &b, size_t bytes, Stream s) {
     b = Slab{};

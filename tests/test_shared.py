@@ -17,7 +17,7 @@ struct State {
   std::map<void *, uint64_t> pinned;   // live blocks, by the serial they belong to
   std::map<void *, uint64_t> mem;      // device allocations
   std::map<int, bool> ended;           // events: whether the work before them has ended
-  int allocs = 0, next_event = 1;
+  int allocs = 0, queries = 0, next_event = 1;
   bool wrong = false;                  // something dead was given back
   void reset(int d, uint64_t s) {      // everything of the old CUDA context goes
     for (auto it = pinned.begin(); it != pinned.end();)
@@ -57,7 +57,7 @@ struct Fake {
   }
   int event(int *e) { *e = s->next_event++; s->ended[*e] = true; return 0; }
   int record(int e, int) { s->ended[e] = false; return 0; }
-  bool done(int e) { return s->ended[e]; }
+  bool done(int e) { s->queries++; return s->ended[e]; }
   void drop(int e) { if (!s->ended.erase(e)) s->wrong = true; }
   void unpin(void *p) {
     auto it = s->pinned.find(p);
@@ -179,7 +179,9 @@ CASES = {
   CHECK(a2 && a2 != a && s.allocs == 2);
   S.give_back(g, a, &A, 1, MB);
   S.give_back(g, a2, &A, 1, MB);
+  const int q = s.queries;
   CHECK(S.lend(g, &A, 1, 2 * MB) == a && s.allocs == 2);  // its own stream orders them
+  CHECK(s.queries == q);
   S.give_back(g, a, &A, 1, 2 * MB);
   auto *b = S.lend(g, &B, 2, 2 * MB);  // A's work has not ended
   CHECK(b && b != a && b != a2 && s.allocs == 3);
